@@ -275,7 +275,7 @@ size_t place(DeviceBuffers* b, const Capacity& c, char* base) {
   CLUE_PLACE(seed_event, int32_t, N);
   CLUE_PLACE(scan_desc, unsigned long long, c.scan_blocks);
   CLUE_PLACE(counters, int32_t, 16);
-  CLUE_PLACE(large_tiles, int32_t, N / 256 + 1);
+  CLUE_PLACE(large_tiles, int32_t, N / (kEventLargeTilePoints + 1) + 1);
   CLUE_PLACE(oversize, int32_t, N / 4096 + 1);
   CLUE_PLACE(status, uint32_t, 1);
   CLUE_PLACE(stats, unsigned long long, 8);
@@ -649,6 +649,8 @@ clue_status run_device(clue_workspace* ws, const clue_params* params, const clue
       return fail(CLUE_ERR_INVALID_ARGUMENT, err);
   }
   const RunShape& sh = piece ? *piece->shape : ws->tables.shape;
+  // the kernels of such a run take its tables as arguments: nothing to upload
+  const bool event = !piece && event_path(sh);
   DeviceBuffers b = ws->b;
   if (piece) {
     b.grids = piece->grids;
@@ -664,9 +666,9 @@ clue_status run_device(clue_workspace* ws, const clue_params* params, const clue
                              pts->tags != nullptr, staged)) != CLUE_OK)
       return s;
     b = ws->b;
-    if ((s = stage_tables(ws, t)) != CLUE_OK)
+    if (!event && (s = stage_tables(ws, t)) != CLUE_OK)
       return s;
-    if (ws->graph_exec) {  // the cached graph reads the staging buffer just overwritten
+    if (ws->graph_exec) {  // one graph per workspace; it may read the staging buffer just overwritten
       if ((e = cudaGraphExecDestroy(ws->graph_exec)) != cudaSuccess)
         return fail_cuda(e, "graph release");
       ws->graph_exec = nullptr;
@@ -694,6 +696,12 @@ clue_status run_device(clue_workspace* ws, const clue_params* params, const clue
     io.event_base = piece->event_base;
   }
   io.stats = ws->profiling && !piece ? ws->b.stats : nullptr;
+  if (event) {
+    io.grid = &t.grids[0];
+    io.event = &t.events[0];
+    io.host_n_seeds = &ws->info->n_seeds;
+    io.host_status = &ws->info->status;
+  }
   const RunParams prm = make_run_params(params, pts, ws->tuning);
   reset_launch_count();
   if (sh.max_event_points <= kLocalLabelPoints)
@@ -701,14 +709,15 @@ clue_status run_device(clue_workspace* ws, const clue_params* params, const clue
   if (use_graph && (e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
     return fail_cuda(e, "stream capture");
   // Everything from here to the end of the capture is stream work.
-  if (!piece)
+  if (!piece && !event)
     s = copy_tables(ws, t, st, !use_graph);
   if (s == CLUE_OK && (e = launch_run(sh, prm, io, b, st, ws->profiling ? ws->marks : nullptr)) !=
                           cudaSuccess)
     s = fail_cuda(e, "kernel launch");
   // Seed count and status word come back with the run (read when needed); a
-  // pipelined batch reads them once, after its last piece.
-  if (s == CLUE_OK && !piece &&
+  // pipelined batch reads them once, after its last piece, and the last kernel
+  // of a single event writes them.
+  if (s == CLUE_OK && !piece && !event &&
       ((e = cudaMemcpyAsync(&ws->info->n_seeds, ws->b.counters + 1, sizeof(int32_t),
                             cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
        (e = cudaMemcpyAsync(&ws->info->status, ws->b.status, sizeof(uint32_t), cudaMemcpyDeviceToHost,

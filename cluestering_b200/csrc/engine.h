@@ -120,6 +120,14 @@ int32_t sort_runs(int64_t n, int32_t* len);
 constexpr int32_t kLocalLabelPoints = 1 << 16;
 bool local_labels_ready(int32_t points);
 
+// Single events of at most kEventPoints points and kEventTiles tiles run their
+// stages before and after the sweeps as one cluster launch each (event.cu).
+constexpr int32_t kEventPoints = 1 << 16;
+constexpr int32_t kEventTiles = 2560;
+// Whether a run of this shape takes that form; the first call on a device
+// grants the kernels their shared memory (outside stream capture).
+bool event_path(const RunShape& sh);
+
 // Pointers of one run's inputs and outputs (device memory).
 struct RunIO {
   const float* coords[kMaxDim] = {};
@@ -142,6 +150,14 @@ struct RunIO {
   // Sweep statistics: when set, the run zeroes these 8 counters and the sweeps
   // add to them (see SweepArgs::stats).
   unsigned long long* stats = nullptr;
+  // Host tables of a run that takes event_path (its kernels receive them as
+  // arguments and write the device tables), and where that run puts its seed
+  // count and status word: pinned host memory, or null to leave them on the
+  // device alone.
+  const GridDesc* grid = nullptr;
+  const EventDesc* event = nullptr;
+  int32_t* host_n_seeds = nullptr;
+  uint32_t* host_status = nullptr;
 };
 
 // Host tables built for a run.
@@ -159,13 +175,27 @@ bool build_tables(int32_t D, const uint32_t* sizes, int32_t n_events, int32_t gr
 // Bytes of device scratch a run of this shape needs.
 size_t scratch_bytes(const RunShape& s, bool sigma, bool unc, bool tags);
 
-// Enqueues the whole run on `stream`. Tables must already be on the device.
+// Enqueues the whole run on `stream`. Tables must already be on the device,
+// except those of a run with io.grid and io.event set (see there).
 // When `marks` is not null it holds kStages + 1 events recorded at the stage
 // boundaries (extents | tiles | gather | density | nearest higher | labels).
 constexpr int kStages = 6;
 cudaError_t launch_run(const RunShape& shape, const RunParams& prm, const RunIO& io,
                        const DeviceBuffers& b, cudaStream_t stream,
                        cudaEvent_t* marks = nullptr);
+
+// The stages of an event_path run before and after the sweeps. Tiles of more
+// than large_points points are listed as large.
+cudaError_t launch_event_front(const RunShape& shape, const RunParams& prm, const RunIO& io, const GridDesc& grid,
+                               const EventDesc& ev, const DeviceBuffers& b, int large_points,
+                               cudaStream_t stream);
+// launch_clusters_csr for at most kEventPoints points and kEventTiles clusters,
+// where event_map_path says so.
+bool event_map_path(int64_t n, int32_t n_clusters);
+cudaError_t launch_event_map(int64_t n, const int32_t* labels, int32_t n_clusters, int32_t* offsets,
+                             int32_t* points, cudaStream_t stream);
+cudaError_t launch_event_finish(const RunShape& shape, const RunIO& io, const DeviceBuffers& b,
+                                cudaStream_t stream);
 
 // Runs the tile scan's bounded wait on `desc` (zeroed: nothing publishes it);
 // the kernel sets a bit in `status` when the wait gives up.

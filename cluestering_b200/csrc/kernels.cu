@@ -1330,6 +1330,8 @@ cudaError_t launch_clusters_csr(const DeviceBuffers& b, int64_t n, const int32_t
   cudaError_t e;
   if (n_clusters == 0)
     return cudaMemsetAsync(offsets, 0, sizeof(int32_t), st);
+  if (event_map_path(n, n_clusters))
+    return launch_event_map(n, labels, n_clusters, offsets, points, st);
   if ((e = cudaMemsetAsync(count, 0, sizeof(int32_t) * n_clusters, st)))
     return e;
   k_hist<<<grid_for(n), kThreads, 0, st>>>(labels, n, count);
@@ -1358,15 +1360,6 @@ cudaError_t launch_localize(const DeviceBuffers& b, int32_t n_events, int64_t n,
   return cudaGetLastError();
 }
 
-cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io,
-                       const DeviceBuffers& b, cudaStream_t st, cudaEvent_t* marks) {
-  const int D = sh.D;
-  const int64_t n = sh.n;
-  CoordPtrs x{}, sig{};
-  for (int d = 0; d < D; ++d) {
-    x.p[d] = io.coords[d];
-    sig.p[d] = io.sigma[d];
-  }
 #define CLUE_CHECK(expr)          \
   do {                            \
     cudaError_t e_ = (expr);      \
@@ -1384,10 +1377,16 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
       CLUE_CHECK(cudaEventRecord(marks[i], st)); \
   } while (0)
 
-  // grid extents
-  CLUE_MARK(0);
-  if (io.stats)
-    CLUE_CHECK(fill32(io.stats, 16, 0, st));
+// The stages before the sweeps: grid extents, tile binning, gather.
+static cudaError_t launch_front(const RunShape& sh, const RunParams& prm, const RunIO& io, const DeviceBuffers& b,
+                         cudaStream_t st, cudaEvent_t* marks) {
+  const int D = sh.D;
+  const int64_t n = sh.n;
+  CoordPtrs x{}, sig{};
+  for (int d = 0; d < D; ++d) {
+    x.p[d] = io.coords[d];
+    sig.p[d] = io.sigma[d];
+  }
   // exact-sum bounds per event (2-D and 3-D runs: their workspace holds them)
   int32_t* exact = (D == 2 || D == 3) ? b.event_exact : nullptr;
   const int64_t init_items = std::max<int64_t>((int64_t)sh.n_grids * kMaxDim, exact ? 4 * (int64_t)sh.n_events : 0);
@@ -1449,6 +1448,24 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
                                              prm.kernel_kind == CLUE_KERNEL_FLAT, prm.kernel_p0,
                                              b.counters + 4);
   CLUE_LAUNCHED();
+  return cudaSuccess;
+}
+
+cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io,
+                       const DeviceBuffers& b, cudaStream_t st, cudaEvent_t* marks) {
+  const int D = sh.D;
+  const int64_t n = sh.n;
+  CLUE_MARK(0);
+  if (io.stats)
+    CLUE_CHECK(fill32(io.stats, 16, 0, st));
+  const bool event = io.event && event_path(sh);
+  if (event) {  // up to and including the gather: one cluster launch
+    CLUE_MARK(1);
+    CLUE_CHECK(launch_event_front(sh, prm, io, *io.grid, *io.event, b, kEventLargeTilePoints, st));
+    CLUE_MARK(2);
+  } else {
+    CLUE_CHECK(launch_front(sh, prm, io, b, st, marks));
+  }
 
   // the two sweeps
   SweepArgs a{};
@@ -1459,7 +1476,8 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
   a.cls_dens = b.cls_dens;
   a.cls_nh = b.cls_nh;
   a.queue = b.counters + 4;
-  a.large_tiles = b.large_tiles;  // listed by sort_segments above
+  a.large_points = event ? kEventLargeTilePoints : kLargeTilePoints;
+  a.large_tiles = b.large_tiles;
   a.large_count = b.counters + 3;
   a.rec_dens = b.rec_dens;
   a.rec_nh = b.rec_nh;
@@ -1504,6 +1522,11 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
   CLUE_MARK(5);
 
   // seeds and labels
+  if (event) {
+    CLUE_CHECK(launch_event_finish(sh, io, b, st));
+    CLUE_MARK(6);
+    return cudaSuccess;
+  }
   CLUE_CHECK(scan(b.seed_flag, b.seed_rank, n, b.counters + 1, b, st));
   const bool piece = io.piece_base != nullptr;
   int32_t* nh_shift = piece && io.point_base ? io.nh : nullptr;

@@ -117,12 +117,17 @@ extern "C" clue_status clue_make_clusters_device_noalloc(const clue_params* para
   e = cudaMemsetAsync(b.status, 0, sizeof(uint32_t), st);
   if (e != cudaSuccess)
     return fail_cuda(e, "status reset");
-  k_noalloc_tables<<<(sh.n_chunks + 31) / 32, 32, 0, st>>>(g, ev, kChunkPoints, b.grids, b.events,
-                                                           b.chunks, sh.n_chunks);
-  if ((e = cudaGetLastError()) != cudaSuccess)
-    return fail_cuda(e, "table setup");
-
   RunIO io;
+  if (event_path(sh)) {  // its kernels take the tables as arguments
+    io.grid = &g;
+    io.event = &ev;
+  } else {
+    k_noalloc_tables<<<(sh.n_chunks + 31) / 32, 32, 0, st>>>(g, ev, kChunkPoints, b.grids, b.events,
+                                                             b.chunks, sh.n_chunks);
+    if ((e = cudaGetLastError()) != cudaSuccess)
+      return fail_cuda(e, "table setup");
+  }
+
   for (int d = 0; d < D; ++d) {
     io.coords[d] = pts->coords[d];
     io.sigma[d] = pts->sigma[d];

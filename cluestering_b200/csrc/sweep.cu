@@ -1523,7 +1523,7 @@ __device__ void tile_cells(const RunParams& p, const SweepArgs& a, int64_t t, in
 }
 
 // Cell layouts of all tiles. Blocks [0, large_blocks) take the tiles of more
-// than kLargeTilePoints points, which the tile sort listed, one block each, so
+// than a.large_points points, which the binning listed, one block each, so
 // a dense tile of thousands of points does not hold up the launch on one warp;
 // they come first so that the heaviest tiles do not run as a tail. The other
 // blocks give one warp to each smaller tile. The kernel waits on dependent
@@ -1545,7 +1545,7 @@ __global__ void __launch_bounds__(kCellWarps * 32, D == 2 ? 6 : 4) k_cells(const
     const int64_t wb = (int64_t)blockIdx.x - large_blocks;
     const int64_t stride = ((int64_t)gridDim.x - large_blocks) * kCellWarps;
     for (int64_t t = wb * kCellWarps + warp; t < a.n_tiles; t += stride) {
-      if (a.tile_offset[t + 1] - a.tile_offset[t] > kLargeTilePoints)
+      if (a.tile_offset[t + 1] - a.tile_offset[t] > a.large_points)
         continue;
       tile_cells<D, 32>(p, a, t, s_cnt + warp * kWarpCellSlots, s_cls[warp],
                         s_cnt2 + warp * kWarpCellSlots);
@@ -1778,7 +1778,7 @@ cudaError_t launch_work_order(int D, const RunParams& p, const SweepArgs& a, cud
         (int)std::max<int64_t>(1, std::min<int64_t>((a.n_tiles + kCellWarps - 1) / kCellWarps, (int64_t)sm_count() * 32));
     // blocks for the large tiles: at most one per tile that can be large
     const int large_blocks =
-        (int)std::max<int64_t>(1, std::min<int64_t>(a.n / (kLargeTilePoints + 1), (int64_t)sm_count() * 24));
+        (int)std::max<int64_t>(1, std::min<int64_t>(a.n / (a.large_points + 1), (int64_t)sm_count() * 24));
     if (D == 2)
       k_cells<2><<<large_blocks + warp_blocks, kCellWarps * 32, 0, st>>>(p, a, large_blocks);
     else

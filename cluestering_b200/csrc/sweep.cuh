@@ -31,8 +31,9 @@ struct SweepArgs {
   // each counts the 32-point work items taken so far (k_gather resets
   // both), so warps that finish early take the next item.
   int32_t* queue;
-  // Tiles of more than 256 points (listed by the tile sort) and their count:
-  // k_cells gives each of them a whole block.
+  // Tiles of more than large_points points (listed by the binning or the tile
+  // sort) and their count: k_cells gives each of them a whole block.
+  int32_t large_points;
   const int32_t* large_tiles;
   const int32_t* large_count;
   // Exact-sum density (flat kernel): the density records again, in cell-layout
