@@ -116,3 +116,38 @@ def test_device_utilities_need_clustered_device_points():
     c, w = fixture("data_1024")
     with pytest.raises(TypeError):
         clue.cluster_centroids(clue.PointsHost(c, w), clue.Clusterer(1.3, 10.0, 1.3))
+
+
+# The warps that share 32 points take one cluster at a time: fewer clusters than
+# warps, one cluster, none, clusters of one point, sizes around the 32 points of
+# a tile, and every templated number of dimensions and the general one.
+@pytest.mark.gpu
+@pytest.mark.parametrize("ndim", [1, 2, 3, 4])
+@pytest.mark.parametrize("sizes", [[], [1], [33], [1, 31], [32, 64, 1], [5, 300, 2, 31, 97, 32, 1, 33, 64, 65]])
+def test_device_scores_of_given_clusters(ndim, sizes):
+    import torch
+    rng = np.random.default_rng(84 + ndim + len(sizes))
+    lab = np.concatenate([np.full(s, k) for k, s in enumerate(sizes)] + [np.full(17, -1)]).astype(np.int32)
+    c = (rng.normal(0.0, 1.0, (ndim, lab.size)) + 9.0 * lab).astype(np.float32)
+    order = rng.permutation(lab.size)
+    lab, c = lab[order], np.ascontiguousarray(c[:, order])
+    w = rng.exponential(1.0, lab.size).astype(np.float32)
+    k = len(sizes)
+    dev = torch.device("cuda", 0)
+    pts = clue.PointsDevice(torch.from_numpy(c).to(dev), torch.from_numpy(w).to(dev))
+    pts.cluster_index = torch.from_numpy(lab).to(dev)
+    offsets, members = clue.api.clusters_csr(lab)
+
+    class Given:  # a clusterer whose last run gave these labels
+        def getClustersDevice(self, stream=None):  # noqa: N802
+            return torch.from_numpy(offsets).to(dev), torch.from_numpy(members).to(dev)
+
+    pts.clustered = True
+    got = clue.silhouette_scores(pts, Given())
+    ref = O.silhouette(c, lab, k) if k else np.full(lab.size, np.nan, np.float32)
+    assert np.array_equal(np.isnan(got), np.isnan(ref))
+    keep = ~np.isnan(ref)
+    assert np.array_equal(got[keep].view(np.int32), ref[keep].view(np.int32))
+    for weighted in (False, True) if k else ():
+        cen = clue.cluster_centroids(pts, Given(), weighted=weighted)
+        assert np.array_equal(cen.view(np.int32), O.centroids(c, w, lab, k, weighted=weighted).view(np.int32))
