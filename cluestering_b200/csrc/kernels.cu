@@ -1434,8 +1434,8 @@ static cudaError_t launch_front(const RunShape& sh, const RunParams& prm, const 
     k_scatter<<<grid_for(n), kThreads, 0, st>>>(b.tile_of, n, b.tile_cursor, b.perm);
     CLUE_LAUNCHED();
     // Exact-sum events need no ascending order within their tiles when nothing
-    // else on this run reads it (flat kernel, cell path: no user tags).
-    const bool order_free_tiles = sweep_cells_path(prm) && prm.kernel_kind == CLUE_KERNEL_FLAT;
+    // else on this run reads it (flat kernel; user tags break ties by it).
+    const bool order_free_tiles = sweep_fast_path(prm) && !prm.has_tags && prm.kernel_kind == CLUE_KERNEL_FLAT;
     CLUE_CHECK(sort_segments(b.tile_offset, sh.n_tiles, b.perm, b, st, order_free_tiles ? exact : nullptr,
                              sh.n_events));
   }
@@ -1501,7 +1501,6 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
   a.stats = io.stats;
   a.status = b.status;
   if (sweep_fast_path(prm)) {
-    a.nh_cells = sweep_cells_path(prm);
     a.nh_pos = b.nh_pos;
     a.nh_q = b.nh_q;
     a.cell_slot = b.cell_slot;

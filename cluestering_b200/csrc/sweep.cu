@@ -172,9 +172,6 @@ __global__ void __launch_bounds__(kThreads) k_work_order(const RunParams p, cons
         local -= own[d] * g.stride[d];
       }
     }
-    // the cell search of the nearest higher visits points in layout order and
-    // needs no work order of its own
-    const bool nh_order = !a.nh_cells;
     for (int s = begin + threadIdx.x; s < end; s += blockDim.x) {
       float xi[D], si[D];
       load_point<D>(p, a, s, xi, si);
@@ -183,22 +180,19 @@ __global__ void __launch_bounds__(kThreads) k_work_order(const RunParams p, cons
       const int cd = box_class<D>(g, own, inf, sup);
       a.cls_dens[s] = cd;
       atomicAdd(&cnt[0][cd], 1);
-      if (nh_order) {
-        search_box<D>(g, p, xi, si, p.dm, inf, sup);
-        const int cn = box_class<D>(g, own, inf, sup);
-        a.cls_nh[s] = cn;
-        atomicAdd(&cnt[1][cn], 1);
-      }
+      search_box<D>(g, p, xi, si, p.dm, inf, sup);
+      const int cn = box_class<D>(g, own, inf, sup);
+      a.cls_nh[s] = cn;
+      atomicAdd(&cnt[1][cn], 1);
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5;
-    if (warp < (nh_order ? 2 : 1))
+    if (warp < 2)
       warp_scan_counts<E>(cnt[warp]);
     __syncthreads();
     for (int s = begin + threadIdx.x; s < end; s += blockDim.x) {
       a.work_dens[begin + atomicAdd(&cnt[0][a.cls_dens[s]], 1)] = s;
-      if (nh_order)
-        a.work_nh[begin + atomicAdd(&cnt[1][a.cls_nh[s]], 1)] = s;
+      a.work_nh[begin + atomicAdd(&cnt[1][a.cls_nh[s]], 1)] = s;
     }
     __syncthreads();
   }
@@ -363,7 +357,7 @@ __device__ __forceinline__ float sq_dist(const float* xi, const float4& r) {
   return __fadd_rn(sx, __fadd_rn(sy, __fmul_rn(dz, dz)));
 }
 
-// Row iteration shared by both fast sweeps: calls body(q) for every candidate
+// Row iteration: calls body(q) for every candidate
 // of the search box in the reference's order.
 template <int D, typename Body>
 __device__ __forceinline__ void for_each_candidate(const SweepArgs& a, const GridDesc& g, int base,
@@ -1150,11 +1144,8 @@ __global__ void __launch_bounds__(NT, MINB) k_density_fast(const RunParams p, co
     const uint32_t tag = p.has_tags ? a.stag[s] : (uint32_t)gi;
     const uint32_t kbits = rho_key(rho);
     const float key = __uint_as_float(kbits);
-    int pos = s;
-    if (a.nh_cells) {
-      pos = a.nh_pos[s];
-      atomicMax(&a.cell_info[a.cell_slot[s]].maxkey, ((unsigned long long)kbits << 32) | tag);
-    }
+    const int pos = a.nh_pos[s];
+    atomicMax(&a.cell_info[a.cell_slot[s]].maxkey, ((unsigned long long)kbits << 32) | tag);
     if (D == 2) {
       a.rec_nh[pos] = make_float4(xi[0], xi[1], key, __uint_as_float(tag));
     } else {
@@ -1219,72 +1210,22 @@ __device__ __forceinline__ void nh_take(NhBest& st, float d2, int q, uint64_t ke
 // ClusteringKernels.hpp:195-202 for one eligible candidate (higher key, d2 <=
 // eff2): it wins when its distance is smaller, or equal with a larger key.
 // Only squared distances inside the bracket take the exact square roots.
-__device__ __forceinline__ void nh_consider(NhBest& st, float d2, int q, uint64_t key) {
+// With user tags two candidates can have equal keys; the first in the layout then
+// wins, as the first visited does in the reference (tiles in order, points of a
+// tile in ascending index): nh_q maps layout positions to that order.
+template <bool TAGS = false>
+__device__ __forceinline__ void nh_consider(NhBest& st, float d2, int q, uint64_t key,
+                                            const int32_t* nh_q = nullptr) {
   if (d2 <= st.lo) {
     nh_take(st, d2, q, key);
   } else if (d2 < st.hi) {
     const float dist = __fsqrt_rn(d2), delta = __fsqrt_rn(st.d2b);
-    if ((dist < delta) || ((dist == delta) && (key > st.key_b)))
+    if ((dist < delta) ||
+        ((dist == delta) &&
+         ((key > st.key_b) || (TAGS && key == st.key_b && nh_q[q] < nh_q[st.best]))))
       nh_take(st, d2, q, key);
   }
 }
-
-// Nearest higher with (density, tag) as one ordered 64-bit key and distances
-// compared as squared distances. A candidate j of point i is eligible when it is
-// "higher" (key_j > key_i, which is rho_j > rho_i, or equal densities above zero
-// and tag_j > tag_i) and sqrt(d2) <= the effective distance (d2 <= eff2). Against
-// the current best (distance delta) it wins when sqrt(d2) < delta, or when
-// sqrt(d2) == delta and key_j > key_best (ClusteringKernels.hpp:195-202). The
-// bracket decides all but the candidates whose squared distance falls in
-// (lo, hi); those take the exact square root.
-template <int D>
-__global__ void __launch_bounds__(kThreads, 4) k_nearest_higher_fast(const RunParams p,
-                                                                  const SweepArgs a) {
-  const int64_t n = a.n;
-  const float4* __restrict__ rec = a.rec_nh;
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n;
-       w += (int64_t)gridDim.x * blockDim.x) {
-    const int s = a.work_nh[w];
-    const EventDesc ev = a.events[a.sevt[s]];
-    const GridDesc& g = a.grids[ev.grid];
-    const float4 ri = rec[s];
-    const float xi[3] = {ri.x, ri.y, ri.z};
-    const float zero[3] = {0.0f, 0.0f, 0.0f};
-    const float rho_i = a.srho[s];
-    const uint32_t tag_i = D == 2 ? __float_as_uint(ri.w) : a.rec_tag[s];
-    const float unc = p.has_unc ? a.sunc[s] : 1.0f;
-    const float min_density = __fmul_rn(p.rhoc, unc);
-    const bool seedlike = rho_i >= min_density;  // ClusteringKernels.hpp:168
-    const float eff2 = seedlike ? p.seed2 : p.dm2;
-    // rho_j == rho_i && rho_j > 0 && tag_j > tag_i: with rho_i <= 0 (or NaN)
-    // equal densities never count, so the tag part of the key is saturated.
-    const bool nan_i = rho_i != rho_i;
-    const uint64_t key_i =
-        ((uint64_t)(nan_i ? 0xffffffffu : rho_key(rho_i)) << 32) |
-        ((nan_i || !(rho_i > 0.0f)) ? 0xffffffffu : tag_i);
-    int inf[D], sup[D];
-    search_box<D>(g, p, xi, zero, p.dm, inf, sup);
-    NhBest bs = nh_none();
-    for_each_candidate<D>(a, g, ev.tile_base, inf, sup, [&](int q) {
-      const float4 r = __ldg(&rec[q]);
-      const uint32_t tag_j = D == 2 ? __float_as_uint(r.w) : __ldg(&a.rec_tag[q]);
-      const uint64_t key_j = ((uint64_t)__float_as_uint(D == 2 ? r.z : r.w) << 32) | tag_j;
-      const float d2 = sq_dist<D>(xi, r);
-      if ((key_j > key_i) && (d2 <= eff2))
-        nh_consider(bs, d2, q, key_j);
-    });
-    const int best = bs.best;
-    const int gi = a.perm[s];
-    const int nh = best >= 0 ? a.perm[best] : -1;
-    a.out_nh[gi] = nh;
-    a.parent[s] = best >= 0 ? best : s;
-    const int seed = (nh == -1) && seedlike;
-    a.seed_flag[gi] = seed;
-    if (a.out_seed)
-      a.out_seed[gi] = seed;
-  }
-}
-
 
 // Exclusive scan of cnt[0..S) in place by one warp (any S).
 __device__ void warp_scan_range(int* cnt, int S) {
@@ -1557,10 +1498,19 @@ __global__ void __launch_bounds__(kCellWarps * 32, D == 2 ? 6 : 4) k_cells(const
   }
 }
 
+// Nearest higher with (density, tag) as one ordered 64-bit key and distances
+// compared as squared distances. A candidate j of point i is eligible when it is
+// "higher" (key_j > key_i, which is rho_j > rho_i, or equal densities above zero
+// and tag_j > tag_i) and sqrt(d2) <= the effective distance (d2 <= eff2). Against
+// the current best (distance delta) it wins when sqrt(d2) < delta, or when
+// sqrt(d2) == delta and key_j > key_best (ClusteringKernels.hpp:195-202). The
+// bracket decides all but the candidates whose squared distance falls in
+// (lo, hi); those take the exact square root.
+
 // Tests the members of one cell unless the cell is empty, holds no higher
 // key, or its box is out of reach.
 // `cnt` counts cells checked, cells entered and members tested (statistics).
-template <int D, bool STATS>
+template <int D, bool TAGS, bool STATS>
 __device__ __forceinline__ void visit_cell(const SweepArgs& a, int slot, const float* xi,
                                            uint64_t key_i, float eff2, NhBest& st, int* cnt) {
   if (STATS)
@@ -1585,17 +1535,18 @@ __device__ __forceinline__ void visit_cell(const SweepArgs& a, int slot, const f
     const uint64_t key_j = ((uint64_t)__float_as_uint(D == 2 ? r.z : r.w) << 32) | tag_j;
     const float d2 = sq_dist<D>(xi, r);
     if ((key_j > key_i) && (d2 <= eff2))
-      nh_consider(st, d2, q, key_j);
+      nh_consider<TAGS>(st, d2, q, key_j, a.nh_q);
   }
 }
 
-// Nearest higher over the cell layout. Thread w takes the w-th point of the
+// Nearest higher over the cell layout, one point per lane, for runs whose points
+// fill the GPU that way (nh_lanes). Thread w takes the w-th point of the
 // walk order, so a warp holds neighbouring points. The own cell and its neighbours in the own
 // tile come first, which usually fixes a small delta; then every tile of the
 // reference's search box is visited, but only its cells that can hold a point
 // within the current bound. The result is the eligible candidate of least
-// distance, ties to the larger key (ClusteringKernels.hpp:195-202), as in
-// k_nearest_higher_fast, over exactly the same candidates.
+// distance, ties to the larger key (ClusteringKernels.hpp:195-202), then (with
+// user tags) to the first in the layout.
 // The search is bound by the latency of its dependent loads (cell info, box,
 // members), so the 2-D form trades registers for resident warps: 8 blocks of
 // 256 threads per SM measured 8.3 ms on the 46.5 M-point batch against 9.4 ms
@@ -1603,7 +1554,7 @@ __device__ __forceinline__ void visit_cell(const SweepArgs& a, int slot, const f
 // per lane, stays at 4.
 // STATS: the profiling instantiation, which also counts the candidates tested
 // (SweepArgs::stats); the counters cost registers, so timed runs go without.
-template <int D, int NT, int MINB, bool STATS>
+template <int D, int NT, int MINB, bool TAGS, bool STATS>
 __global__ void __launch_bounds__(NT, MINB) k_nearest_higher_cells(const RunParams p, const SweepArgs a) {
   const int64_t n = a.n;
   const float4* __restrict__ rec = a.rec_nh;
@@ -1702,7 +1653,7 @@ __global__ void __launch_bounds__(NT, MINB) k_nearest_higher_cells(const RunPara
             seen &= abs(cd - c0[d]) <= 1;
           }
           if (valid && !seen)
-            visit_cell<D, STATS>(a, base + lin, xi, key_i, eff2, bs, cnt);
+            visit_cell<D, TAGS, STATS>(a, base + lin, xi, key_i, eff2, bs, cnt);
         } while (next_tile<D>(c, c_lo, c_hi));
       }
       if (first)
@@ -1735,6 +1686,300 @@ __global__ void __launch_bounds__(NT, MINB) k_nearest_higher_cells(const RunPara
   }
 }
 
+// Nearest higher over the cell layout, G lanes per point (a divisor of 32). The
+// lanes of a group look at different cells at once, and the few cells that can
+// hold a closer higher point are entered one after another with their members
+// spread over the lanes. The result is the eligible candidate of least distance,
+// ties to the larger key (ClusteringKernels.hpp:195-202), then (with user tags,
+// where keys can be equal) to the first in the layout, whatever the order they
+// are looked at in: exactly the reference's choice.
+// Phase 0: the own cell and its neighbours in the own tile, which usually fix a
+// small bound. Phase 1: the tiles of the reference's search box, G at a time,
+// one per lane, each with its range of cells within the bound; these ranges are
+// laid end to end and dealt to the lanes. Bound by the latency of dependent loads
+// (tile, cell info, box, members), which G lanes pay once; nh_lanes has the figures.
+// The warp stays converged: groups that are done wait for the others, and every
+// shuffle and vote is reached by all 32 lanes.
+// STATS: the profiling instantiation, which also counts the candidates tested
+// (SweepArgs::stats); the counters cost registers, so timed runs go without.
+struct NhTile {
+  int first;      // cells of the group's earlier tiles
+  int base;       // the tile's first slot
+  int s;          // cells per dimension
+  int lo[3];      // first cell in reach
+  int n1, n2;     // cells in reach along dimensions 1 and 2
+};
+
+template <int D, int G, int NT, int MINB, bool TAGS, bool STATS>
+__global__ void __launch_bounds__(NT, MINB) k_nearest_higher_group(const RunParams p, const SweepArgs a) {
+  constexpr int P = 32 / G;  // points of a warp at a time
+  constexpr unsigned kGroup = G == 32 ? kFullMask : (1u << G) - 1u;
+  // cells of phase 0: one per lane, the own cell and its nearest neighbours
+  constexpr int kNear = G < (D == 2 ? 9 : 27) ? G : (D == 2 ? 9 : 27);
+  __shared__ NhTile s_tile[NT];
+  const int64_t n = a.n;
+  const float4* __restrict__ rec = a.rec_nh;
+  const int lane = threadIdx.x & 31, l = lane % G, g0 = lane - l;
+  NhTile* tiles = s_tile + (threadIdx.x - l);  // the group's
+  for (;;) {
+    // the next P points of the walk order (work per point varies a lot: points
+    // in dense cells test many more candidates)
+    int64_t w0 = 0;
+    if (lane == 0)
+      w0 = atomicAdd(reinterpret_cast<unsigned*>(&a.queue[1]), (unsigned)P);
+    w0 = __shfl_sync(kFullMask, w0, 0);
+    if (w0 >= n)
+      break;
+    const int64_t w = w0 + lane / G;
+    // groups past the end shadow the warp's first point and write nothing
+    const bool active = w < n;
+    const int pi = a.walk[active ? w : w0];
+    const int s = a.nh_q[pi];
+    int cnt[3] = {0, 0, 0};  // cells checked, cells entered, members tested
+    const float4 ri = rec[pi];
+    const float xi[3] = {ri.x, ri.y, ri.z};
+    const float zero[3] = {0.0f, 0.0f, 0.0f};
+    const float rho_i = a.srho[s];
+    const uint32_t tag_i = D == 2 ? __float_as_uint(ri.w) : a.rec_tag[pi];
+    const float unc = p.has_unc ? a.sunc[s] : 1.0f;
+    const float min_density = __fmul_rn(p.rhoc, unc);
+    const bool seedlike = rho_i >= min_density;  // ClusteringKernels.hpp:168
+    const float eff2 = seedlike ? p.seed2 : p.dm2;
+    // rho_j == rho_i && rho_j > 0 && tag_j > tag_i: with rho_i <= 0 (or NaN)
+    // equal densities never count, so the tag part of the key is saturated.
+    const bool nan_i = rho_i != rho_i;
+    const uint64_t key_i = ((uint64_t)(nan_i ? 0xffffffffu : rho_key(rho_i)) << 32) |
+                           ((nan_i || !(rho_i > 0.0f)) ? 0xffffffffu : tag_i);
+    const EventDesc ev = a.events[a.sevt[s]];
+    const GridDesc& g = a.grids[ev.grid];
+    int inf[D], sup[D], own[D];
+    search_box<D>(g, p, xi, zero, p.dm, inf, sup);
+    // The own tile is skipped when the box leaves it out: get_bin sends a
+    // coordinate beyond the int range to bin 0 (x86 conversion), so a huge
+    // radius can give a box that misses the point's own tile.
+    bool in_box = true;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      own[d] = get_bin(g, p, xi[d], d);
+      in_box &= inf[d] <= own[d] && own[d] <= sup[d];
+    }
+    const int t0 = tile_id<D>(g, p, ev.tile_base, own);
+
+    NhBest bs = nh_none();  // this lane's best
+    float bound = bs.hi;    // no candidate at d2 >= bound can win in the group
+    // Enters the cells that lanes have flagged, the group's cells one by one.
+    auto enter = [&](bool flag, int start, int end, float lb2) {
+      const unsigned vote = __ballot_sync(kFullMask, flag);
+      unsigned mine = (vote >> g0) & kGroup;
+      while (__any_sync(kFullMask, mine != 0)) {
+        const int j = mine ? g0 + __ffs(mine) - 1 : lane;
+        int q = __shfl_sync(kFullMask, start, j);
+        int q1 = __shfl_sync(kFullMask, end, j);
+        const float lb = __shfl_sync(kFullMask, lb2, j);
+        if (!mine || lb >= bound)
+          q1 = q;
+        mine &= mine - 1;
+        if (STATS && l == 0 && q1 > q) {
+          ++cnt[1];
+          cnt[2] += q1 - q;
+        }
+        for (q += l; q < q1; q += G) {
+          const float4 r = __ldg(&rec[q]);
+          const uint32_t tag_j = D == 2 ? __float_as_uint(r.w) : __ldg(&a.rec_tag[q]);
+          const uint64_t key_j = ((uint64_t)__float_as_uint(D == 2 ? r.z : r.w) << 32) | tag_j;
+          const float d2 = sq_dist<D>(xi, r);
+          if (key_j > key_i && d2 <= eff2 && d2 < bound)
+            nh_consider<TAGS>(bs, d2, q, key_j, a.nh_q);
+        }
+        __syncwarp();
+        bound = bs.hi;
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1)
+          bound = fminf(bound, __shfl_xor_sync(kFullMask, bound, o));
+      }
+    };
+    // Whether a cell can hold a closer higher point, and its members.
+    auto check = [&](int slot, int& start, int& end, float& lb2) {
+      if (STATS)
+        ++cnt[0];
+      const CellInfo ci = a.cell_info[slot];
+      start = ci.start;
+      end = ci.end;
+      if (ci.start == ci.end || ci.maxkey <= key_i)
+        return false;
+      float mn[D], mx[D];
+      load_box<D>(a, slot, mn, mx);
+      lb2 = box_lower_bound<D>(xi, mn, mx);
+      return !(lb2 > eff2 || lb2 >= bound);
+    };
+
+    // phase 0
+    int c0[D];
+    {
+      const int base = a.tile_offset[t0];
+      const bool tile0 = in_box && a.tile_offset[t0 + 1] != base;
+      int st = 1;
+      float lo[D], inv[D];
+#pragma unroll
+      for (int d = 0; d < D; ++d)
+        lo[d] = inv[d] = 0.0f;
+      if (tile0) {
+        st = a.cell_s[t0];
+        load_geom<D>(a, t0, lo, inv);
+      }
+#pragma unroll
+      for (int d = 0; d < D; ++d)
+        c0[d] = cell_coord(xi[d], lo[d], inv[d], st);
+      // offsets 0, 1, -1 per dimension: the own cell is the first
+      int rem = l, lin = 0;
+      bool valid = tile0 && l < kNear;
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        const int div = D == 2 ? (d == 0 ? 3 : 1) : (d == 0 ? 9 : d == 1 ? 3 : 1);
+        const int o = rem / div;
+        rem -= o * div;
+        const int c = c0[d] + (o == 2 ? -1 : o);
+        valid &= c >= 0 && c < st;
+        lin = lin * st + c;
+      }
+      int start = 0, end = 0;
+      float lb2 = 0.0f;
+      const bool flag = valid && check(base + lin, start, end, lb2);
+      enter(flag, start, end, lb2);
+    }
+
+    // phase 1: lane l takes the box's tiles l, l + G, ...
+    int64_t box = 1;
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+      box *= max(sup[d] - inf[d] + 1, 0);
+    for (int64_t tb = 0; __any_sync(kFullMask, tb < box); tb += G) {
+      int cells = 0;
+      NhTile nt;
+      nt.base = 0, nt.s = 1, nt.n1 = nt.n2 = 1;
+      nt.lo[0] = nt.lo[1] = nt.lo[2] = 0;
+      if (tb + l < box) {
+        int b[D];
+        int64_t rem = tb + l;
+        // (boxes of fewer than 2^31 tiles: tile ids are 32-bit)
+#pragma unroll
+        for (int d = D - 1; d > 0; --d) {
+          const int nd = sup[d] - inf[d] + 1;
+          const int q = (int)((unsigned)rem / (unsigned)nd);
+          b[d] = inf[d] + (int)rem - q * nd;
+          rem = q;
+        }
+        b[0] = inf[0] + (int)rem;
+        const int t = tile_id<D>(g, p, ev.tile_base, b);
+        nt.base = a.tile_offset[t];
+        if (a.tile_offset[t + 1] != nt.base) {
+          nt.s = a.cell_s[t];
+          float lo[D], inv[D];
+          load_geom<D>(a, t, lo, inv);
+          // |x_j - x_i| <= R for every member that can still win
+          const float R = reach(fminf(eff2, bound));
+          cells = 1;
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            nt.lo[d] = cell_coord(__fsub_rd(xi[d], R), lo[d], inv[d], nt.s);
+            const int hi = cell_coord(__fadd_ru(xi[d], R), lo[d], inv[d], nt.s);
+            cells *= hi - nt.lo[d] + 1;
+            if (d == 1)
+              nt.n1 = hi - nt.lo[d] + 1;
+            if (d == 2)
+              nt.n2 = hi - nt.lo[d] + 1;
+          }
+          if (t == t0 && in_box)
+            nt.s = -nt.s;  // marks the own tile, whose near cells phase 0 has seen
+        }
+      }
+      int incl = cells;
+#pragma unroll
+      for (int o = 1; o < G; o <<= 1) {
+        const int y = __shfl_up_sync(kFullMask, incl, o);
+        if (l >= o)
+          incl += y;
+      }
+      const int total = __shfl_sync(kFullMask, incl, g0 + G - 1);
+      nt.first = incl - cells;
+      tiles[l] = nt;
+      __syncwarp();
+      for (int f0 = 0; __any_sync(kFullMask, f0 < total); f0 += G) {
+        const int f = f0 + l;
+        bool flag = false;
+        int start = 0, end = 0;
+        float lb2 = 0.0f;
+        if (f < total) {
+          // the last tile whose cells start at or before f: tiles without
+          // cells share their successor's start
+          int t = 0;
+#pragma unroll
+          for (int o = G / 2; o > 0; o >>= 1)
+            if (tiles[t + o].first <= f)
+              t += o;
+          const NhTile ct = tiles[t];
+          int r = f - ct.first, c[D];
+          // quotients of integers below 2^11: (r + 0.5) / n is at least 0.5 / n
+          // away from the next integer, far more than the rounding
+          if (D == 3) {
+            const int q = (int)__fdividef((float)r + 0.5f, (float)ct.n2);
+            c[D - 1] = ct.lo[2] + r - q * ct.n2;
+            r = q;
+          }
+          const int q = (int)__fdividef((float)r + 0.5f, (float)ct.n1);
+          c[1] = ct.lo[1] + r - q * ct.n1;
+          c[0] = ct.lo[0] + q;
+          const int st = abs(ct.s);
+          bool seen = ct.s < 0;
+          int lin = 0, near = 0;  // near: the cell's number among phase 0's
+#pragma unroll
+          for (int d = 0; d < D; ++d) {
+            lin = lin * st + c[d];
+            const int o = c[d] - c0[d];
+            seen &= abs(o) <= 1;
+            near = near * 3 + (o < 0 ? 2 : o);
+          }
+          seen &= near < kNear;
+          flag = !seen && check(ct.base + lin, start, end, lb2);
+        }
+        enter(flag, start, end, lb2);
+      }
+      __syncwarp();  // the table is rewritten for the next tiles
+    }
+
+    // the group's best
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) {
+      const float d2 = __shfl_xor_sync(kFullMask, bs.d2b, o);
+      const int q = __shfl_xor_sync(kFullMask, bs.best, o);
+      const uint64_t key = __shfl_xor_sync(kFullMask, bs.key_b, o);
+      if (q >= 0)
+        nh_consider<TAGS>(bs, d2, q, key, a.nh_q);
+    }
+    if (STATS) {  // every lane gets here
+      const int members = __reduce_add_sync(kFullMask, active ? cnt[2] : 0);
+      const int checked = __reduce_add_sync(kFullMask, active ? cnt[0] : 0);
+      const int entered = __reduce_add_sync(kFullMask, active ? cnt[1] : 0);
+      if (lane == 0) {
+        atomicAdd(&a.stats[2], (unsigned long long)members);
+        atomicAdd(&a.stats[3], (unsigned long long)checked);
+        atomicAdd(&a.stats[4], (unsigned long long)entered);
+      }
+    }
+    if (!active || l != 0)
+      continue;
+    const int gi = a.perm[s];
+    const int qb = bs.best >= 0 ? a.nh_q[bs.best] : s;
+    const int nh = bs.best >= 0 ? a.perm[qb] : -1;
+    a.out_nh[gi] = nh;
+    a.parent[s] = qb;
+    const int seed = (nh == -1) && seedlike;
+    a.seed_flag[gi] = seed;
+    if (a.out_seed)
+      a.out_seed[gi] = seed;
+  }
+}
+
 }  // namespace
 
 bool sweep_fast_path(const RunParams& p) {
@@ -1745,8 +1990,6 @@ bool sweep_fast_path(const RunParams& p) {
       return false;
   return true;
 }
-
-bool sweep_cells_path(const RunParams& p) { return sweep_fast_path(p) && !p.has_tags; }
 
 #define CLUE_DISPATCH_D(D, KERNEL, ...)                \
   switch (D) {                                        \
@@ -1766,9 +2009,8 @@ bool sweep_cells_path(const RunParams& p) { return sweep_fast_path(p) && !p.has_
 cudaError_t launch_work_order(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   if (a.n == 0)
     return cudaSuccess;
-  // With cells, k_cells writes the density work order; k_work_order is still
-  // needed for the nearest-higher order when the cell search is off (tags).
-  if (!a.nh_cells) {
+  // On the fast path k_cells writes the density work order.
+  if (!sweep_fast_path(p)) {
     const int blocks = (int)std::min<int64_t>(a.n_tiles, (int64_t)sm_count() * 16);
     CLUE_DISPATCH_D(D, k_work_order, blocks, kThreads, 0, st)
     count_launches(1);
@@ -1829,22 +2071,61 @@ cudaError_t launch_density_fast(const RunParams& p, const SweepArgs& a, cudaStre
   return cudaGetLastError();
 }
 
-// Block shapes of the nearest-higher cell search (clue_tuning::nh_shape):
-// 0: 256 threads with 8 blocks per SM in 2-D, 4 in 3-D; 1: 256 threads, 6 per
-// SM; 2: 128 threads with 16 blocks per SM in 2-D, 8 in 3-D.
-template <int D, bool STATS>
+// Lanes per point of the nearest-higher search. One lane per point is the least
+// work where the points fill the GPU; below that more lanes per point shorten
+// the chain of dependent loads that bounds the kernel. Measured on B200 (us, 1 /
+// 8 / 16 / 32 lanes): 2-D events of 1,024 points 125 / 29 / 21 / 16; 4,096: 59 /
+// 18 / 16 / 16; 16,384: 84 / 25 / 25 / 35; 65,536: 199 / 59 / 68 / 98; 262,144:
+// 240 / 162 / 201 / 322 (and 115 / 113 with 31 blobs per 16,384 points); 524,288:
+// 364 / 358 (168 / 201). In 3-D, where a point has 27 neighbour cells: 16,384
+// hits 113 / 27 / 27 / 39; 262,144: 378 / 219 / 257 / 404; 524,288: 835 / 512.
+int nh_lanes(int D, int64_t n) {
+  if (n <= 4096)
+    return 32;
+  if (n <= 16384)
+    return 16;
+  return D == 3 || n <= (int64_t)1 << 18 ? 8 : 1;
+}
+
+template <int D, bool TAGS, bool STATS>
+void launch_nh_group(const RunParams& p, const SweepArgs& a, int G, cudaStream_t st) {
+  constexpr int kMinBlocks = D == 2 ? 5 : 4;
+  const int blocks = sweep_grid(a.n * G, 256, 16);
+  if (G == 32)
+    k_nearest_higher_group<D, 32, 256, kMinBlocks, TAGS, STATS><<<blocks, 256, 0, st>>>(p, a);
+  else if (G == 16)
+    k_nearest_higher_group<D, 16, 256, kMinBlocks, TAGS, STATS><<<blocks, 256, 0, st>>>(p, a);
+  else
+    k_nearest_higher_group<D, 8, 256, kMinBlocks, TAGS, STATS><<<blocks, 256, 0, st>>>(p, a);
+}
+
+// Block shapes of the nearest-higher search with one lane per point
+// (clue_tuning::nh_shape): 0: 256 threads with 8 blocks per SM; 1: 256 threads, 6
+// per SM; 2: 128 threads with 16 blocks per SM. (2-D only: nh_lanes.)
+template <bool TAGS, bool STATS>
 void launch_nh_cells(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   switch (p.nh_shape) {
     case 1:
-      k_nearest_higher_cells<D, 256, 6, STATS><<<sweep_grid(a.n, 256, 16), 256, 0, st>>>(p, a);
+      k_nearest_higher_cells<2, 256, 6, TAGS, STATS><<<sweep_grid(a.n, 256, 16), 256, 0, st>>>(p, a);
       break;
     case 2:
-      k_nearest_higher_cells<D, 128, D == 2 ? 16 : 8, STATS><<<sweep_grid(a.n, 128, 32), 128, 0, st>>>(p, a);
+      k_nearest_higher_cells<2, 128, 16, TAGS, STATS><<<sweep_grid(a.n, 128, 32), 128, 0, st>>>(p, a);
       break;
     default:
-      k_nearest_higher_cells<D, 256, D == 2 ? 8 : 4, STATS><<<sweep_grid(a.n, 256, 16), 256, 0, st>>>(p, a);
+      k_nearest_higher_cells<2, 256, 8, TAGS, STATS><<<sweep_grid(a.n, 256, 16), 256, 0, st>>>(p, a);
       break;
   }
+}
+
+template <bool TAGS, bool STATS>
+void launch_nh(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
+  const int G = nh_lanes(D, a.n);
+  if (G == 1)
+    launch_nh_cells<TAGS, STATS>(p, a, st);
+  else if (D == 2)
+    launch_nh_group<2, TAGS, STATS>(p, a, G, st);
+  else
+    launch_nh_group<3, TAGS, STATS>(p, a, G, st);
 }
 
 cudaError_t launch_density(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
@@ -1861,18 +2142,11 @@ cudaError_t launch_nearest_higher(int D, const RunParams& p, const SweepArgs& a,
   if (a.n == 0)
     return cudaSuccess;
   count_launches(1);  // one kernel on every path below
-  if (a.nh_cells) {
-    if (D == 2)
-      a.stats ? launch_nh_cells<2, true>(p, a, st) : launch_nh_cells<2, false>(p, a, st);
-    else
-      a.stats ? launch_nh_cells<3, true>(p, a, st) : launch_nh_cells<3, false>(p, a, st);
-    return cudaGetLastError();
-  }
   if (sweep_fast_path(p)) {
-    if (D == 2)
-      k_nearest_higher_fast<2><<<grid_for(a.n), kThreads, 0, st>>>(p, a);
+    if (p.has_tags)
+      a.stats ? launch_nh<true, true>(D, p, a, st) : launch_nh<true, false>(D, p, a, st);
     else
-      k_nearest_higher_fast<3><<<grid_for(a.n), kThreads, 0, st>>>(p, a);
+      a.stats ? launch_nh<false, true>(D, p, a, st) : launch_nh<false, false>(D, p, a, st);
     return cudaGetLastError();
   }
   CLUE_DISPATCH_D(D, k_nearest_higher, grid_for(a.n), kThreads, 0, st)

@@ -61,16 +61,15 @@ struct SweepArgs {
   // Nearest higher as a sorted position (the point itself when it has none):
   // the follower tree in the tile-contiguous layout, where chains stay local.
   int32_t* parent;
-  // Cell layout of the nearest-higher search (null unless sweep_cells_path):
+  // Cell layout of the nearest-higher search (null unless sweep_fast_path):
   // every tile is split into s^D cells (s per tile in cell_s, origin and
   // inverse cell width per dimension in cell_geom); the points of a tile are
   // reordered cell by cell inside the tile's range. A tile starting at sorted
   // position b keeps its cells in slots b .. b + s^D - 1 (s^D never exceeds
   // the tile's point count).
-  // The cells are built for every fast-path run (the density sweep uses them to
-  // skip out-of-reach candidates); the nearest-higher search runs over them
-  // when nh_cells is set (no user tags), and then its records are in cell order.
-  bool nh_cells;
+  // The cells are built for every fast-path run: the density sweep uses them to
+  // skip out-of-reach candidates, and the nearest-higher search runs over them
+  // (its records are in cell order).
   int32_t* nh_pos;        // sorted position -> layout position
   int32_t* nh_q;          // layout position -> sorted position
   int32_t* cell_slot;     // sorted position -> slot of its cell
@@ -89,12 +88,6 @@ struct SweepArgs {
 // True when the packed fast path applies: D = 2 or 3, Euclidean metric, no
 // per-point sigma and no wrapped coordinate.
 bool sweep_fast_path(const RunParams& p);
-
-// True when the nearest-higher sweep runs over the cell layout: the fast path
-// without user tags. Keys (density, tag) are then unique, so the nearest
-// higher is the candidate of least distance, ties to the larger key, whatever
-// order the candidates are visited in.
-bool sweep_cells_path(const RunParams& p);
 
 cudaError_t launch_work_order(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 cudaError_t launch_density(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);

@@ -1,0 +1,45 @@
+"""The nearest-higher search with 32, 16, 8 and 1 lanes per point (chosen by the
+dimension and the number of points), at sizes on both sides of every line, with
+real-valued weights and on lattices of coincident points and few distinct tags,
+where distances, densities and tags all tie and the first candidate in the
+reference's visiting order wins. Compared with the checker bit for bit.
+"""
+
+import numpy as np
+import pytest
+
+from cluestering_b200 import workloads as W
+from tests.test_gpu_parity import check
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(2, 4095), (2, 4097), (2, 16385), (2, 70001), (2, 262145), (3, 4096), (3, 16383), (3, 16387), (3, 70003)]
+
+
+@pytest.mark.parametrize("D,n", SIZES)
+def test_lattice_with_equal_tags(D, n):
+    rng = np.random.default_rng(n)
+    side = max(2, int(round((n / 2.0) ** (1.0 / D))))  # about two points per lattice site
+    c = rng.integers(0, side, (D, n)).astype(np.float32)
+    check(c, np.ones(n, np.float32), 1.0, 2.0, 1.5, path="device", tags=rng.integers(0, 3, n).astype(np.uint32))
+
+
+@pytest.mark.parametrize("D,n", SIZES)
+def test_blobs(D, n):
+    ev = W.blobs(n, max(2, n // 800), 0.0, 100.0 if n < 1 << 18 else 400.0, 1.0, 0.1, seed=n, ndim=D,
+                 weights="exponential")
+    check(ev.coords, ev.weights, 1.5, 4.0, 2.0, 1.0, path="device")
+
+
+@pytest.mark.parametrize("D,n", [(2, 3001), (2, 9001), (3, 3001), (3, 20011)])
+def test_search_box_of_many_tiles(D, n):
+    # a few points per tile and a radius of many tiles: more tiles in the box
+    # than lanes, most of them empty
+    rng = np.random.default_rng(n + D)
+    import cluestering_b200 as clue
+    from tests.test_gpu_parity import assert_identical, run_gpu
+    from oracle import oracle as O
+    c = rng.normal(0.0, 3.0, (D, n)).astype(np.float32)
+    w = rng.exponential(1.0, n).astype(np.float32)
+    g = run_gpu(c, w, 1.0, 2.0, 2.5, path="device", clusterer=clue.Clusterer(1.0, 2.0, 2.5, points_per_tile=4))
+    assert_identical(g, O.make_clusters(c, w, 1.0, 2.0, 2.5, points_per_tile=4, exp_mode=O.EXP_CLUE, n_threads=8))
