@@ -519,25 +519,34 @@ __global__ void __launch_bounds__(kBlock, 1)
     }
   // All of the thread's chains at once, so that their steps overlap, each step
   // leaving its point on its grandparent: every write stores an ancestor, so
-  // the threads' walks shorten each other's.
-  for (int steps = 0;; ++steps) {
-    bool moved = false;
+  // the threads' walks shorten each other's. Where some chain is still longer
+  // after kWalk steps, a round over the whole tree at least halves every path.
+  constexpr int kWalk = 16;
+  for (int round = 0;; ++round) {
+    bool moved = true;
+    for (int step = 0; step < kWalk && moved; ++step) {
+      moved = false;
 #pragma unroll
-    for (int k = 0; k < kRounds; ++k)
-      if (root[k] >= 0) {
-        const int q = up[root[k]];
-        const int qq = up[q];
-        if (qq != q)
-          up[root[k]] = (uint16_t)qq;
-        moved |= qq != root[k];
-        root[k] = qq;
-      }
-    if (!moved)
+      for (int k = 0; k < kRounds; ++k)
+        if (root[k] >= 0) {
+          const int q = up[root[k]];
+          const int qq = up[q];
+          if (qq != q)
+            up[root[k]] = (uint16_t)qq;
+          moved |= qq != root[k];
+          root[k] = qq;
+        }
+    }
+    if (!__syncthreads_or(moved))
       break;
-    if (steps > n) {  // a cycle: never
+    if (round > 16) {  // a cycle: never (16 rounds shorten 65,536 steps to one)
       atomicOr(status, kStatusLabelTimeout);
       break;
     }
+#pragma unroll 8
+    for (int s = threadIdx.x; s < n; s += kBlock)
+      up[s] = up[up[s]];
+    __syncthreads();
   }
   // every seed rank is written before any block reads one (and the totals have
   // been read)
