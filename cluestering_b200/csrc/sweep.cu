@@ -18,72 +18,15 @@
 #include <cfloat>
 
 #include "engine.h"
-#include "sweep.cuh"
+#include "sweep_device.cuh"
 
 namespace clue_impl {
 
 namespace {
 
-constexpr int kThreads = 256;
-constexpr unsigned kFullMask = 0xffffffffu;
-// sqrtf(2.0f), correctly rounded (the reference's math::sqrt(TData{2})).
-constexpr float kSqrt2 = 1.41421356237309504880f;
-
 int grid_for(int64_t n) {
   const int64_t b = (n + kThreads - 1) / kThreads;
   return (int)std::max<int64_t>(1, std::min<int64_t>(b, (int64_t)sm_count() * 16));
-}
-
-// Search box of point s: bins [inf, sup] per dimension (TilesView.hpp:77-87),
-// half width max(r, r * sigma * sqrt(2)) (ClusteringKernels.hpp:112-118).
-template <int D>
-__device__ __forceinline__ void search_box(const GridDesc& g, const RunParams& p, const float* xi,
-                                           const float* si, float radius, int* inf, int* sup) {
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    const float r = std_max(radius, __fmul_rn(__fmul_rn(radius, si[d]), kSqrt2));
-    inf[d] = get_bin(g, p, __fsub_rn(xi[d], r), d);
-    sup[d] = get_bin(g, p, __fadd_rn(xi[d], r), d);
-    if (p.wrapped[d] && inf[d] > sup[d])
-      sup[d] += g.k;
-  }
-}
-
-// Advances the tile odometer (last dimension fastest); false when exhausted.
-template <int D>
-__device__ __forceinline__ bool next_tile(int* b, const int* inf, const int* sup) {
-  bool carry = true;
-#pragma unroll
-  for (int d = D - 1; d >= 0; --d) {
-    if (carry) {
-      if (b[d] < sup[d]) {
-        ++b[d];
-        carry = false;
-      } else {
-        b[d] = inf[d];
-      }
-    }
-  }
-  return !carry;
-}
-
-template <int D>
-__device__ __forceinline__ int tile_id(const GridDesc& g, const RunParams& p, int base, const int* b) {
-  int t = base;
-#pragma unroll
-  for (int d = 0; d < D; ++d)
-    t += g.stride[d] * wrap_bin(g, p, b[d], d);
-  return t;
-}
-
-template <int D>
-__device__ __forceinline__ void load_point(const RunParams& p, const SweepArgs& a, int64_t s, float* x,
-                                           float* sg) {
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    x[d] = a.sx[d * a.n + s];
-    sg[d] = ((p.has_sigma >> d) & 1) ? a.ssig[d * a.n + s] : 0.0f;
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -199,163 +142,11 @@ __global__ void __launch_bounds__(kThreads) k_work_order(const RunParams p, cons
 }
 
 // ---------------------------------------------------------------------------
-// Generic sweeps: any D, metric, kernel and option
-// ---------------------------------------------------------------------------
-
-template <int D>
-__global__ void __launch_bounds__(kThreads) k_density(const RunParams p, const SweepArgs a) {
-  const int64_t n = a.n;
-  const bool mahalanobis = p.metric_kind == CLUE_METRIC_MAHALANOBIS;
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n;
-       w += (int64_t)gridDim.x * blockDim.x) {
-    const int s = a.work_dens[w];
-    const EventDesc ev = a.events[a.sevt[s]];
-    const GridDesc& g = a.grids[ev.grid];
-    float xi[D], si[D];
-    load_point<D>(p, a, s, xi, si);
-    const int gi = a.perm[s];
-    int inf[D], sup[D], b[D];
-    search_box<D>(g, p, xi, si, p.dc, inf, sup);
-#pragma unroll
-    for (int d = 0; d < D; ++d)
-      b[d] = inf[d];
-    float rho = 0.0f;
-    do {
-      const int t = tile_id<D>(g, p, ev.tile_base, b);
-      const int q1 = a.tile_offset[t + 1];
-      for (int q = a.tile_offset[t]; q < q1; ++q) {
-        float xj[D], sj[D];
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          xj[d] = a.sx[d * n + q];
-          sj[d] = mahalanobis ? a.ssig[d * n + q] : 0.0f;
-        }
-        const int gj = a.perm[q];
-        const float dist = metric_finish(p, metric_inner<D>(p, xi, xj, si, sj));
-        const float k = kernel_value(p, dist, gi == gj);
-        // rho_i += static_cast<int>(distance <= density_radius) * k * w_j
-        rho = __fadd_rn(rho, __fmul_rn(__fmul_rn((float)(int)(dist <= p.dc), k), a.sw[q]));
-      }
-    } while (next_tile<D>(b, inf, sup));
-    a.srho[s] = rho;
-    if (a.out_rho)
-      a.out_rho[gi] = rho;
-  }
-}
-
-template <int D>
-__global__ void __launch_bounds__(kThreads) k_nearest_higher(const RunParams p, const SweepArgs a) {
-  const int64_t n = a.n;
-  const bool mahalanobis = p.metric_kind == CLUE_METRIC_MAHALANOBIS;
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < n;
-       w += (int64_t)gridDim.x * blockDim.x) {
-    const int s = a.work_nh[w];
-    const EventDesc ev = a.events[a.sevt[s]];
-    const GridDesc& g = a.grids[ev.grid];
-    float xi[D], si[D];
-    load_point<D>(p, a, s, xi, si);
-    const int gi = a.perm[s];
-    const float rho_i = a.srho[s];
-    const float unc = p.has_unc ? a.sunc[s] : 1.0f;
-    const float min_density = __fmul_rn(p.rhoc, unc);
-    // ClusteringKernels.hpp:168
-    const float eff = (rho_i >= min_density) ? p.seed_dc : p.dm;
-    const uint32_t tag_i = p.has_tags ? a.stag[s] : (uint32_t)gi;
-    int inf[D], sup[D], b[D];
-    search_box<D>(g, p, xi, si, p.dm, inf, sup);
-#pragma unroll
-    for (int d = 0; d < D; ++d)
-      b[d] = inf[d];
-    float delta = FLT_MAX;
-    int nh = -1, nh_pos = s;
-    float rho_nh = 0.0f;
-    uint32_t tag_nh = 0;
-    do {
-      const int t = tile_id<D>(g, p, ev.tile_base, b);
-      const int q1 = a.tile_offset[t + 1];
-      for (int q = a.tile_offset[t]; q < q1; ++q) {
-        const float rho_j = a.srho[q];
-        const int gj = a.perm[q];
-        const uint32_t tag_j = p.has_tags ? a.stag[q] : (uint32_t)gj;
-        // ClusteringKernels.hpp:180-182
-        const bool higher =
-            (rho_j > rho_i) || ((rho_j == rho_i) && (rho_j > 0.0f) && (tag_j > tag_i));
-        if (!higher)
-          continue;
-        float xj[D], sj[D];
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          xj[d] = a.sx[d * n + q];
-          sj[d] = mahalanobis ? a.ssig[d * n + q] : 0.0f;
-        }
-        const float dist = metric_finish(p, metric_inner<D>(p, xi, xj, si, sj));
-        // ClusteringKernels.hpp:195-202
-        if (dist <= eff &&
-            ((dist < delta) ||
-             ((dist == delta) && (nh >= 0) &&
-              ((rho_j > rho_nh) || ((rho_j == rho_nh) && (tag_j > tag_nh)))))) {
-          delta = dist;
-          nh = gj;
-          nh_pos = q;
-          rho_nh = rho_j;
-          tag_nh = tag_j;
-        }
-      }
-    } while (next_tile<D>(b, inf, sup));
-    a.out_nh[gi] = nh;
-    a.parent[s] = nh_pos;
-    // KernelFindClusters, ClusteringKernels.hpp:301-313
-    const int seed = (nh == -1) && (rho_i >= min_density);
-    a.seed_flag[gi] = seed;
-    if (a.out_seed)
-      a.out_seed[gi] = seed;
-  }
-}
-
-// ---------------------------------------------------------------------------
 // Fast path: D = 2 or 3, Euclidean, no sigma, no wrapped coordinate.
 // Candidates are packed float4 records; `sqrt(d2) <= r` is tested as
 // `d2 <= thr` with the exact threshold computed on the host; the tiles of one
 // row of the search box (last dimension) are contiguous and read as one range.
 // ---------------------------------------------------------------------------
-
-// Order-preserving image of a density: key(a) > key(b) iff a > b and equal
-// densities give equal keys. NaN maps to 0, below every number, so a NaN
-// density is never "higher" (every comparison with NaN is false). Densities
-// are never -0 (they start at +0 and round-to-nearest sums of opposite values
-// give +0), so no other pair of equal values has different keys.
-__device__ __forceinline__ uint32_t rho_key(float rho) {
-  if (rho != rho)
-    return 0u;
-  const uint32_t b = __float_as_uint(rho);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
-// (x_i - x_j)^2 and (y_i - y_j)^2 with one packed subtract and one packed
-// multiply (sm_100 f32x2): each half is the IEEE round-to-nearest result of
-// the scalar operation, so the values equal __fsub_rn / __fmul_rn.
-__device__ __forceinline__ void sq_diff_xy(float xi, float yi, float xj, float yj, float& sx,
-                                           float& sy) {
-  asm("{\n\t.reg .b64 a, b, d, s;\n\t"
-      "mov.b64 a, {%2, %3};\n\t"
-      "mov.b64 b, {%4, %5};\n\t"
-      "sub.rn.f32x2 d, a, b;\n\t"
-      "mul.rn.f32x2 s, d, d;\n\t"
-      "mov.b64 {%0, %1}, s;\n\t}"
-      : "=f"(sx), "=f"(sy)
-      : "f"(xi), "f"(yi), "f"(xj), "f"(yj));
-}
-
-template <int D>
-__device__ __forceinline__ float sq_dist(const float* xi, const float4& r) {
-  // meta::accumulate right fold: dx^2 + (dy^2 [+ dz^2])
-  float sx, sy;
-  sq_diff_xy(xi[0], xi[1], r.x, r.y, sx, sy);
-  if (D == 2)
-    return __fadd_rn(sx, sy);
-  const float dz = __fsub_rn(xi[2], r.z);
-  return __fadd_rn(sx, __fadd_rn(sy, __fmul_rn(dz, dz)));
-}
 
 // Row iteration: calls body(q) for every candidate
 // of the search box in the reference's order.
@@ -382,19 +173,6 @@ __device__ __forceinline__ void for_each_candidate(const SweepArgs& a, const Gri
   }
 }
 
-// ---------------------------------------------------------------------------
-// Cell layout (fast path).
-//
-// Every tile of m points is split into s^D cells, s the largest value with
-// s^D * kCellTarget <= m (at least 1, at most cell_dim_max). A point's cell
-// comes from cell_coord, which is monotone in the coordinate; a search
-// therefore finds every point of [a, b] in the cells cell_coord(a) ..
-// cell_coord(b), whatever rounding placed it there. Each cell records the
-// bounding box of its members and (for the nearest-higher search) their
-// largest key. The density sweep uses the cells to skip candidates no lane of
-// a warp can reach; the nearest-higher search visits them nearest-first.
-// ---------------------------------------------------------------------------
-
 // Average points per cell: a launch tuning (clue_tuning::cell_points, 1..8,
 // default 2). Cells only order and prune the candidates of the sweeps, so the
 // choice never changes a result.
@@ -419,130 +197,12 @@ __device__ __forceinline__ int cells_per_dim(int m, int target) {
   return s;
 }
 
-// Cell coordinate of x in a tile with origin lo and inverse cell width inv
-// (0 for a degenerate tile): monotone non-decreasing in x for every non-NaN x,
-// clamped to [0, s); NaN lands in cell 0.
-__device__ __forceinline__ int cell_coord(float x, float lo, float inv, int s) {
-  float u = __fmul_rn(__fsub_rn(x, lo), inv);
-  u = fminf(fmaxf(u, 0.0f), (float)(s - 1));
-  return (int)u;
-}
-
 // Origin and inverse cell width of the tiles' cells, dimension d.
 __device__ __forceinline__ void cell_axis(const GridDesc& g, int b, int s, int d, float& lo,
                                           float& inv) {
   lo = __fadd_rn(g.minv[d], __fmul_rn((float)b, g.tile[d]));
   const float v = __fdiv_rn((float)s, g.tile[d]);
   inv = (g.tile[d] > 0.0f && v < INFINITY) ? v : 0.0f;
-}
-
-template <int D>
-__device__ __forceinline__ void load_geom(const SweepArgs& a, int t, float* lo, float* inv) {
-  const float4 g0 = a.cell_geom[D == 2 ? t : 2 * t];
-  if (D == 2) {
-    lo[0] = g0.x, lo[1] = g0.y, inv[0] = g0.z, inv[1] = g0.w;
-  } else {
-    const float4 g1 = a.cell_geom[2 * t + 1];
-    lo[0] = g0.x, lo[1] = g0.y, lo[D - 1] = g0.z, inv[0] = g0.w, inv[1] = g1.x, inv[D - 1] = g1.y;
-  }
-}
-
-template <int D>
-__device__ __forceinline__ void load_box(const SweepArgs& a, int slot, float* mn, float* mx) {
-  const float4 b0 = a.cell_box[D == 2 ? slot : 2 * slot];
-  if (D == 2) {
-    mn[0] = b0.x, mn[1] = b0.y, mx[0] = b0.z, mx[1] = b0.w;
-  } else {
-    const float4 b1 = a.cell_box[2 * slot + 1];
-    mn[0] = b0.x, mn[1] = b0.y, mn[D - 1] = b0.z, mx[0] = b0.w, mx[1] = b1.x, mx[D - 1] = b1.y;
-  }
-}
-
-// Lower bound of the squared distance from xi to any member of a cell, with
-// the operations of sq_dist: per dimension the gap to the box is at most
-// |fl(x_i - x_j)| of every member (rounding is monotone), and squares and the
-// right fold are monotone too.
-template <int D>
-__device__ __forceinline__ float box_lower_bound(const float* xi, const float* mn, const float* mx) {
-  float gap[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d)
-    gap[d] = fmaxf(fmaxf(__fsub_rn(mn[d], xi[d]), __fsub_rn(xi[d], mx[d])), 0.0f);
-  if (D == 2)
-    return __fadd_rn(__fmul_rn(gap[0], gap[0]), __fmul_rn(gap[1], gap[1]));
-  return __fadd_rn(__fmul_rn(gap[0], gap[0]),
-                   __fadd_rn(__fmul_rn(gap[1], gap[1]), __fmul_rn(gap[D - 1], gap[D - 1])));
-}
-
-// |x_j - x_i| <= reach(bound2) in every coordinate for every point with
-// fl(d2) <= bound2: each square and sum is rounded to nearest, so
-// |x_j - x_i| <= sqrt(bound2) (1 + 2^-22); the factor 1 + 10^-6 and the
-// absolute 10^-19 (square roots near the smallest normal) cover that, rounded up.
-__device__ __forceinline__ float reach(float bound2) {
-  return __fadd_ru(__fmul_ru(__fsqrt_ru(bound2), 1.000001f), 1e-19f);
-}
-
-// Asynchronous 16-byte global -> shared copies (per thread, completion by
-// commit groups).
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// Bulk copies (the copy engine inside each SM) into this CTA's shared memory,
-// completed on an mbarrier by transaction bytes. Sources are this GPU's own
-// memory; nothing is multicast.
-__device__ __forceinline__ unsigned smem_u32(const void* p) {
-  return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_init_fence() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-// Orders this thread's earlier shared-memory accesses before later bulk copies
-// into the same buffer.
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-// dst and src 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Waits for the phase of `bar` with this parity, at most kCopyWaitLimit polls
-// (each poll itself bounded by the hardware's try-wait time limit). On giving
-// up it records kStatusCopyTimeout, so the host call reports CLUE_ERR_TIMEOUT.
-constexpr int kCopyWaitLimit = 1 << 22;
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity, uint32_t* status) {
-  for (int it = 0; it < kCopyWaitLimit; ++it)
-    if (mbar_try_wait(bar, parity))
-      return true;
-  atomicOr(status, kStatusCopyTimeout);
-  return false;
 }
 
 // Contribution of candidate record r (sorted position q) to rho_i.
@@ -559,35 +219,6 @@ __device__ __forceinline__ void density_add(const RunParams& p, const float* xi,
       rho = __fadd_rn(rho, __fmul_rn(k, v));
     }
   }
-}
-
-// (a, b) as one 64-bit register pair, the operand of the f32x2 instructions.
-__device__ __forceinline__ unsigned long long pack2(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-
-// Squared distance and contribution weight of a streamed record: xi_xy holds
-// (x_i, y_i) packed, the record arrives as two packed halves {(x, y), (z or v,
-// v or w)}; the arithmetic is that of sq_dist.
-template <int D>
-__device__ __forceinline__ float packed_d2(unsigned long long xi_xy, float zi, const ulonglong2& r,
-                                           float& v) {
-  float sx, sy;
-  asm("{\n\t.reg .b64 d, s;\n\t"
-      "sub.rn.f32x2 d, %2, %3;\n\t"
-      "mul.rn.f32x2 s, d, d;\n\t"
-      "mov.b64 {%0, %1}, s;\n\t}"
-      : "=f"(sx), "=f"(sy)
-      : "l"(xi_xy), "l"(r.x));
-  float hi_lo, hi_hi;  // the record's second half: D = 2 {v, w}; D = 3 {z, v}
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(hi_lo), "=f"(hi_hi) : "l"(r.y));
-  v = D == 2 ? hi_lo : hi_hi;
-  if (D == 2)
-    return __fadd_rn(sx, sy);
-  const float dz = __fsub_rn(zi, hi_lo);
-  return __fadd_rn(sx, __fadd_rn(sy, __fmul_rn(dz, dz)));
 }
 
 // Streamed form of density_add (same arithmetic).
@@ -2133,24 +1764,21 @@ cudaError_t launch_density(int D, const RunParams& p, const SweepArgs& a, cudaSt
     return cudaSuccess;
   if (sweep_fast_path(p))
     return D == 2 ? launch_density_fast<2>(p, a, st) : launch_density_fast<3>(p, a, st);
-  CLUE_DISPATCH_D(D, k_density, grid_for(a.n), kThreads, 0, st)
-  count_launches(1);
-  return cudaGetLastError();
+  return launch_density_any(D, p, a, st);
 }
 
 cudaError_t launch_nearest_higher(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   if (a.n == 0)
     return cudaSuccess;
-  count_launches(1);  // one kernel on every path below
   if (sweep_fast_path(p)) {
+    count_launches(1);
     if (p.has_tags)
       a.stats ? launch_nh<true, true>(D, p, a, st) : launch_nh<true, false>(D, p, a, st);
     else
       a.stats ? launch_nh<false, true>(D, p, a, st) : launch_nh<false, false>(D, p, a, st);
     return cudaGetLastError();
   }
-  CLUE_DISPATCH_D(D, k_nearest_higher, grid_for(a.n), kThreads, 0, st)
-  return cudaGetLastError();
+  return launch_nearest_higher_any(D, p, a, st);
 }
 
 }  // namespace clue_impl

@@ -90,6 +90,10 @@ struct SweepArgs {
 bool sweep_fast_path(const RunParams& p);
 
 cudaError_t launch_work_order(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
+// The sweeps off the fast path: any number of dimensions, metric, kernel and
+// option (sweep_any.cu).
+cudaError_t launch_density_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
+cudaError_t launch_nearest_higher_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 cudaError_t launch_density(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 cudaError_t launch_nearest_higher(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 

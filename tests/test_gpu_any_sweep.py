@@ -1,0 +1,83 @@
+"""The sweeps off the fast path (csrc/sweep_any.cu: a block per 32 points of one
+tile, walking the union of their search boxes) where that union is unusual, against
+the checker bit for bit: items that span events, boxes that wrap round or cover the
+whole circle, boxes of more tiles than the block stages at a time, boxes that differ
+much in many dimensions, boxes without the point's own tile, and weights or kernels
+whose out-of-range terms are not zero.
+"""
+
+import math
+
+import numpy as np
+import pytest
+
+import cluestering_b200 as clue
+from cluestering_b200 import workloads as W
+from oracle import oracle as O
+from tests.test_gpu_parity import assert_identical, check, run_gpu, run_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mode", [clue.GRID_PER_EVENT, clue.GRID_SHARED])
+def test_items_across_events(mode):
+    ev, sizes = W.batch_2d(40, 1, 700, seed=31)
+    w = np.random.default_rng(32).exponential(1.0, ev.n).astype(np.float32)
+    check(ev.coords, w, 1.5, 3.0, 2.0, metric="manhattan", sizes=sizes, grid_mode=mode, path="device")
+
+
+@pytest.mark.parametrize("r", [0.05, 0.7, 2.9, 7.0])
+@pytest.mark.parametrize("wrapped", [[0, 1], [1, 0], [1, 1]])
+def test_wrapped_boxes(r, wrapped):
+    rng = np.random.default_rng(33)
+    n = 4099
+    c = np.mod(np.stack([rng.normal(0.1, 0.8, n), rng.normal(6.2, 0.9, n)]), 2 * math.pi).astype(np.float32)
+    w = rng.exponential(1.0, n).astype(np.float32)
+    check(c, w, r, 2.0, 1.3 * r, metric="periodic_euclidean", metric_params=(2 * math.pi, 2 * math.pi),
+          wrapped=wrapped, path="device")
+
+
+@pytest.mark.parametrize("D,n,ppt,r", [(1, 3001, 2, 2.0), (2, 3001, 2, 12.0), (4, 6001, 4, 6.0), (5, 20011, 16, 2.0),
+                                       (6, 5003, 4, 1.0)])
+def test_boxes_of_many_tiles(D, n, ppt, r):
+    rng = np.random.default_rng(34 + D)
+    c = rng.uniform(0.0, 20.0, (D, n)).astype(np.float32)
+    w = rng.exponential(1.0, n).astype(np.float32)
+    g = run_gpu(c, w, r, 2.0, r, metric="chebyshev", path="device",
+                clusterer=clue.Clusterer(r, 2.0, r, points_per_tile=ppt))
+    assert_identical(g, O.make_clusters(c, w, r, 2.0, r, metric="chebyshev", points_per_tile=ppt,
+                                        exp_mode=O.EXP_CLUE, n_threads=8))
+
+
+def test_box_without_the_own_tile():
+    # a radius beyond the int range of get_bin's conversion sends the box's upper
+    # end to bin 0 (x86 conversion)
+    ev = W.blobs(3000, 6, 0.0, 30.0, 1.0, 0.1, seed=35, weights="exponential")
+    check(ev.coords, ev.weights, 1.0, 3.0, 1e13, metric="manhattan", path="device")
+    check(ev.coords, ev.weights, 3e12, 3.0, 1e13, metric="weighted_euclidean", metric_params=(1.0, 2.0), path="device")
+
+
+@pytest.mark.parametrize("kernel,params", [("flat", (0.5,)), ("gaussian", (0.8, 2.0)), ("exponential", (1.2, 0.7))])
+def test_infinite_and_nan_weights(kernel, params):
+    # 0 * k * w of a candidate out of range is NaN for such a weight, and so is
+    # every density whose search box holds it
+    ev = W.blobs(2500, 5, 0.0, 60.0, 1.0, 0.1, seed=36, weights="exponential")
+    w = ev.weights.copy()
+    w[[7, 900]] = np.inf
+    w[1400] = np.nan
+    kw = dict(metric="manhattan", kernel=kernel, kernel_params=params)
+    g = run_gpu(ev.coords, w, 1.5, 3.0, 2.0, path="device", **kw)
+    o = run_oracle(ev.coords, w, 1.5, 3.0, 2.0, **kw)
+    assert np.isnan(o.rho).sum() > 100
+    assert np.array_equal(np.isnan(g["rho"]), np.isnan(o.rho))
+    keep = ~np.isnan(o.rho)
+    assert np.array_equal(g["rho"][keep].view(np.int32), o.rho[keep].view(np.int32))
+    assert np.array_equal(g["nh"], o.nearest_higher)
+    assert np.array_equal(g["ci"], o.cluster_index)
+
+
+def test_lattice_ties_and_equal_tags_in_four_dimensions():
+    rng = np.random.default_rng(37)
+    n = 6000
+    c = rng.integers(0, 7, (4, n)).astype(np.float32)
+    check(c, np.ones(n, np.float32), 1.0, 2.0, 1.5, tags=rng.integers(0, 3, n).astype(np.uint32), path="device")
