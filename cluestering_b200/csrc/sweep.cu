@@ -1762,6 +1762,8 @@ void launch_nh(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
 cudaError_t launch_density(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   if (a.n == 0)
     return cudaSuccess;
+  if (sweep_fast_path(p) && a.n <= kGroupPoints)
+    return launch_density_group(D, p, a, st);
   if (sweep_fast_path(p))
     return D == 2 ? launch_density_fast<2>(p, a, st) : launch_density_fast<3>(p, a, st);
   return launch_density_any(D, p, a, st);

@@ -78,7 +78,7 @@ struct SweepArgs {
   CellInfo* cell_info;    // per slot
   float4* cell_box;       // per slot: bounding box of the members (D = 3: two entries)
   // Sweep statistics (null unless the run counts them): [0] density candidate
-  // tests (a lane testing one record), [1] density work items, [2] nearest-
+  // tests (a point testing one record), [1] density work items of 32 points, [2] nearest-
   // higher members tested, [3] cells checked, [4] cells whose members were tested.
   unsigned long long* stats;
   // Status word of the run: kernels with bounded waits set bits here.
@@ -90,6 +90,10 @@ struct SweepArgs {
 bool sweep_fast_path(const RunParams& p);
 
 cudaError_t launch_work_order(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
+// The density with 16 or 32 lanes per point, for fast-path runs of at most
+// kGroupPoints points (density_group.cu).
+constexpr int64_t kGroupPoints = 1 << 16;
+cudaError_t launch_density_group(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 // The sweeps off the fast path: any number of dimensions, metric, kernel and
 // option (sweep_any.cu).
 cudaError_t launch_density_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);

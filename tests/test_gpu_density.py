@@ -1,0 +1,86 @@
+"""The density sweep's forms (16 or 32 lanes per point, 32 points per warp) where
+the lists of candidates are unusual, against the checker bit for bit: tiles of more
+points than a candidate bitmap covers, search boxes of many tiles, events with exact
+and with ordered sums in one run, coordinates far from the origin, degenerate tiles.
+"""
+
+import numpy as np
+import pytest
+
+import cluestering_b200 as clue
+from cluestering_b200 import workloads as W
+from oracle import oracle as O
+from tests.test_gpu_parity import assert_identical, check, run_gpu
+
+pytestmark = pytest.mark.gpu
+
+KERNELS = [("flat", (0.5,), "unit"), ("flat", (0.3,), "exponential"), ("gaussian", (0.7, 1.5), "exponential"),
+           ("exponential", (1.1, 0.9), "unit")]
+# both sides of the lines between the forms
+SIZES = [700, 8192, 8193, 65536, 65537]
+
+
+def event(D, n, weights, seed):
+    ev = W.blobs(n, max(1, n // 3000), 0.0, 60.0, 1.0, 0.15, seed=seed, ndim=D, weights=weights)
+    order = np.random.default_rng(seed).permutation(n)
+    return np.ascontiguousarray(ev.coords[:, order]), ev.weights[order]
+
+
+def check_ppt(c, w, dc, rhoc, dm, ppt, **kw):
+    g = run_gpu(c, w, dc, rhoc, dm, path="device", clusterer=clue.Clusterer(dc, rhoc, dm, points_per_tile=ppt), **kw)
+    assert_identical(g, O.make_clusters(c, w, dc, rhoc, dm, points_per_tile=ppt, exp_mode=O.EXP_CLUE, n_threads=8,
+                                        **kw))
+
+
+@pytest.mark.parametrize("kernel,params,weights", KERNELS)
+@pytest.mark.parametrize("D", [2, 3])
+@pytest.mark.parametrize("n", SIZES)
+def test_shuffled_blobs(D, n, kernel, params, weights):
+    c, w = event(D, n, weights, 1000 + n % 97 + D)
+    check(c, w, 1.2, 3.0, 1.5, kernel=kernel, kernel_params=params, path="device")
+
+
+@pytest.mark.parametrize("kernel,params,weights", KERNELS)
+@pytest.mark.parametrize("D,n,ppt", [(2, 9000, 20000), (3, 9000, 20000), (2, 70000, 30000), (3, 70000, 12000)])
+def test_tiles_larger_than_the_bitmap(D, n, ppt, kernel, params, weights):
+    c, w = event(D, n, weights, 1100 + D)
+    check_ppt(c, w, 0.4, 3.0, 0.5, ppt, kernel=kernel, kernel_params=params)
+
+
+@pytest.mark.parametrize("kernel,params,weights", KERNELS)
+@pytest.mark.parametrize("D,n,r", [(2, 3000, 6.0), (3, 3000, 9.0), (2, 66000, 1.5), (3, 66000, 4.0)])
+def test_search_boxes_of_many_tiles(D, n, r, kernel, params, weights):
+    c, w = event(D, n, weights, 1200 + D)
+    check_ppt(c, w, r, 3.0, r, 4, kernel=kernel, kernel_params=params)
+
+
+@pytest.mark.parametrize("scale", [1, 12])
+@pytest.mark.parametrize("mode", [clue.GRID_PER_EVENT, clue.GRID_SHARED])
+def test_exact_and_ordered_events_together(scale, mode):
+    ev, sizes = W.batch_2d(24, 60, 1500 * scale, seed=1300)
+    w = ev.weights.copy()
+    begin = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    rng = np.random.default_rng(1301)
+    for e in range(0, len(sizes), 2):  # every other event
+        w[begin[e]:begin[e + 1]] = rng.exponential(1.0, int(sizes[e])).astype(np.float32)
+    check(ev.coords, w, 1.5, 3.0, 2.0, sizes=sizes, grid_mode=mode, path="device")
+
+
+@pytest.mark.parametrize("kernel,params,weights", KERNELS)
+@pytest.mark.parametrize("n", [5000, 66000])
+def test_far_from_the_origin(n, kernel, params, weights):
+    # the tiles' edges round to 1/16 here, a quarter of the radius
+    c, w = event(2, n, weights, 1400)
+    c = c + np.array([[9e5], [-7e5]], np.float32)
+    check(c, w, 0.25, 3.0, 0.5, kernel=kernel, kernel_params=params, path="device")
+
+
+@pytest.mark.parametrize("kernel,params,weights", KERNELS)
+def test_points_on_a_line_and_coincident_points(kernel, params, weights):
+    rng = np.random.default_rng(1500)
+    n = 6000
+    w = np.ones(n, np.float32) if weights == "unit" else rng.exponential(1.0, n).astype(np.float32)
+    c = np.stack([np.full(n, 3.5), rng.normal(0.0, 4.0, n)]).astype(np.float32)  # tiles of no width
+    check(c, w, 0.3, 3.0, 0.5, kernel=kernel, kernel_params=params, path="device")
+    c = np.repeat(rng.uniform(0.0, 5.0, (2, 12)), n // 12, axis=1).astype(np.float32)
+    check(c, w, 0.3, 3.0, 0.5, kernel=kernel, kernel_params=params, path="device")
