@@ -21,11 +21,6 @@ constexpr int kMaxDim = CLUE_MAX_DIM;
 // (DeviceBuffers::large_tiles) and the kernels that work tile by tile give
 // each of them a whole block instead of one warp.
 constexpr int kLargeTilePoints = 256;
-// On a single event (event_path) already tiles of more than this are: its few
-// hundred tiles leave most of the GPU idle, and a warp takes one of 128 points
-// through ten dependent passes of four rounds each, a block of one round each
-// (k_cells 21 -> 16 us on a 10,000-hit 3-D event).
-constexpr int kEventLargeTilePoints = 32;
 
 // ---------------------------------------------------------------------------
 // Tables the host builds for a run

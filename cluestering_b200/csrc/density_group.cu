@@ -94,7 +94,8 @@ __global__ void __launch_bounds__(NT, MINB) k_density_group(const RunParams p, c
     const int64_t w = w0 + lane / G;
     // groups past the end shadow the warp's first point and write nothing
     const bool active = w < n;
-    const int s = a.work_dens[active ? w : w0];
+    const int64_t at = active ? w : w0;
+    const int s = a.work_dens ? a.work_dens[at] : a.nh_q[at];  // neighbours follow one another
     const int event = a.sevt[s];
     const EventDesc ev = a.events[event];
     const GridDesc& g = a.grids[ev.grid];

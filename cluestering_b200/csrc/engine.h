@@ -184,11 +184,9 @@ cudaError_t launch_run(const RunShape& shape, const RunParams& prm, const RunIO&
                        const DeviceBuffers& b, cudaStream_t stream,
                        cudaEvent_t* marks = nullptr);
 
-// The stages of an event_path run before and after the sweeps. Tiles of more
-// than large_points points are listed as large.
+// The stages of an event_path run before and after the sweeps.
 cudaError_t launch_event_front(const RunShape& shape, const RunParams& prm, const RunIO& io, const GridDesc& grid,
-                               const EventDesc& ev, const DeviceBuffers& b, int large_points,
-                               cudaStream_t stream);
+                               const EventDesc& ev, const DeviceBuffers& b, cudaStream_t stream);
 // launch_clusters_csr for at most kEventPoints points and kEventTiles clusters,
 // where event_map_path says so.
 bool event_map_path(int64_t n, int32_t n_clusters);

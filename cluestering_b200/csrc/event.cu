@@ -8,7 +8,7 @@
 // microseconds of launch and memory latency; its stable binning runs one warp
 // per 1,024 points and its label kernel one block per event. Measured on B200
 // (16,384-point 2-D event, sums of kernel times): 153 us before the sweeps and
-// 45 us after them there, 14 us and 20 us here.
+// 45 us after them there, 14 us and 16 us here.
 #include <atomic>
 #include <cfloat>
 #include <type_traits>
@@ -51,8 +51,6 @@ struct FrontArgs {
   float* sunc;
   uint32_t* stag;
   float4* rec;  // density records of the fast sweeps, or null
-  int32_t* large_tiles;
-  int32_t large_points;
   int32_t* event_exact;  // or null
   int32_t* counters;
 };
@@ -139,7 +137,7 @@ struct ClusterSort {
     }
   }
   // Bases of this block's elements, from the totals of every block, and the
-  // first position of every key, which block 0 hands to emit(key, first, count).
+  // first position of every key, which block 0 hands to emit(key, first).
   // Returns the number of elements. The others' shared memory has been read
   // when it returns.
   template <typename Emit>
@@ -172,7 +170,7 @@ struct ClusterSort {
       if (k0 + j < k1) {
         base[k0 + j] += block_first;
         if (rank == 0)
-          emit(k0 + j, first, counts[j]);
+          emit(k0 + j, first);
         first += counts[j];
       }
     return total;
@@ -207,7 +205,6 @@ __global__ void __launch_bounds__(kBlock, 1) k_event_front(const RunParams p, co
   __shared__ float s_ext[2 * kMaxDim];  // this block's extremes (read by the others)
   __shared__ int s_sum[4];              // this block's exact-sum bounds (idem)
   __shared__ int s_warp[kWarps];
-  __shared__ int s_large;
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -220,10 +217,8 @@ __global__ void __launch_bounds__(kBlock, 1) k_event_front(const RunParams p, co
 
   if (threadIdx.x < 4)
     s_sum[threadIdx.x] = threadIdx.x == 0 ? INT_MAX : 0;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0)
     sg = a.grid;
-    s_large = 0;
-  }
   float x[kRounds][DD ? DD : 1], w[kRounds];
 #pragma unroll
   for (int k = 0; k < kRounds; ++k) {
@@ -364,20 +359,14 @@ __global__ void __launch_bounds__(kBlock, 1) k_event_front(const RunParams p, co
     }
     a.counters[4] = a.counters[5] = 0;  // the sweeps' work queues
   }
-  sort.bases(cluster, T, s_warp, [&](int t, int first, int count) {
-    a.tile_offset[t] = first;
-    if (count > a.large_points)
-      a.large_tiles[atomicAdd(&s_large, 1)] = t;
-  });
+  sort.bases(cluster, T, s_warp, [&](int t, int first) { a.tile_offset[t] = first; });
   // the others' shared memory has been read: after the matching wait at the
   // end every block may exit
   __syncwarp();
   cluster.barrier_arrive();
   __syncthreads();
-  if (rank == 0 && threadIdx.x == 0) {
+  if (rank == 0 && threadIdx.x == 0)
     a.tile_offset[T] = n;
-    a.counters[3] = s_large;
-  }
 
   // ---- placement and the tile-contiguous copy ----
 #pragma unroll
@@ -388,15 +377,19 @@ __global__ void __launch_bounds__(kBlock, 1) k_event_front(const RunParams p, co
     const int64_t s = sort.place(tile[k]);
     if (s < 0)
       continue;
-    a.perm[s] = i;
-    a.sevt[s] = 0;
+    a.sevt[i] = 0;
     a.point_event[i] = 0;
+    // The stores are scattered, and 16 SMs make them all: as few as possible. The
+    // event of every position is the same, and where the sweeps read records
+    // nothing reads the coordinate planes.
+    a.perm[s] = i;
     a.sw[s] = w[k];
+    if (!(DD && a.rec)) {
 #pragma unroll
-    for (int d = 0; d < (DD ? DD : kMaxDim); ++d)
-      if (d < D)
-        a.sx[(int64_t)d * n + s] = DD ? x[k][DD ? d : 0] : a.x[d][i];
-    if (DD && a.rec) {  // {x, y, v, w} or {x, y, z, v}, as k_gather writes them
+      for (int d = 0; d < (DD ? DD : kMaxDim); ++d)
+        if (d < D)
+          a.sx[(int64_t)d * n + s] = DD ? x[k][DD ? d : 0] : a.x[d][i];
+    } else {  // {x, y, v, w} or {x, y, z, v}, as k_gather writes them
       const float v = p.kernel_kind == CLUE_KERNEL_FLAT ? __fmul_rn(p.kernel_p0, w[k]) : w[k];
       a.rec[s] = DD == 2 ? make_float4(x[k][0], x[k][DD ? 1 : 0], v, w[k])
                          : make_float4(x[k][0], x[k][DD ? 1 : 0], x[k][DD == 3 ? 2 : 0], v);
@@ -442,7 +435,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_event_map(int n, const int32_t* l
   __syncthreads();
   sort.block_prefix(n_clusters);
   cluster.sync();
-  const int total = sort.bases(cluster, n_clusters, s_warp, [&](int c, int first, int) { offsets[c] = first; });
+  const int total = sort.bases(cluster, n_clusters, s_warp, [&](int c, int first) { offsets[c] = first; });
   __syncwarp();
   cluster.barrier_arrive();
   __syncthreads();
@@ -489,13 +482,15 @@ __global__ void __launch_bounds__(kBlock, 1)
     root[k] = s < n ? s : -1;
     gi[k] = s < n ? perm[s] : 0;
   }
+  bool outside = false;
 #pragma unroll 8
   for (int s = threadIdx.x; s < n; s += kBlock) {
     const unsigned q = (unsigned)parent[s];
     up[s] = (uint16_t)(q < (unsigned)n ? q : (unsigned)s);
-    if (q >= (unsigned)n)  // a chain leaving its event: never
-      atomicOr(status, kStatusLabelRange);
+    outside |= q >= (unsigned)n;
   }
+  if (outside)  // a chain leaving its event: never
+    atomicOr(status, kStatusLabelRange);
   int total;
   int at = block_exclusive(__popc(flags), s_warp, &total);
   if (threadIdx.x == 0)
@@ -521,7 +516,7 @@ __global__ void __launch_bounds__(kBlock, 1)
   // leaving its point on its grandparent: every write stores an ancestor, so
   // the threads' walks shorten each other's. Where some chain is still longer
   // after kWalk steps, a round over the whole tree at least halves every path.
-  constexpr int kWalk = 16;
+  constexpr int kWalk = 32;
   for (int round = 0;; ++round) {
     bool moved = true;
     for (int step = 0; step < kWalk && moved; ++step) {
@@ -650,8 +645,7 @@ bool event_map_path(int64_t n, int32_t n_clusters) {
 }
 
 cudaError_t launch_event_front(const RunShape& sh, const RunParams& prm, const RunIO& io, const GridDesc& grid,
-                               const EventDesc& ev, const DeviceBuffers& b, int large_points,
-                               cudaStream_t st) {
+                               const EventDesc& ev, const DeviceBuffers& b, cudaStream_t st) {
   FrontArgs a{};
   for (int d = 0; d < sh.D; ++d) {
     a.x[d] = io.coords[d];
@@ -674,8 +668,6 @@ cudaError_t launch_event_front(const RunShape& sh, const RunParams& prm, const R
   a.sunc = b.sorted_unc;
   a.stag = b.sorted_tag;
   a.rec = sweep_fast_path(prm) ? b.rec_dens : nullptr;
-  a.large_tiles = b.large_tiles;
-  a.large_points = large_points;
   a.event_exact = sh.D == 2 || sh.D == 3 ? b.event_exact : nullptr;
   a.counters = b.counters;
   const auto kernel = sh.D == 2 ? k_event_front<2> : sh.D == 3 ? k_event_front<3> : k_event_front<0>;

@@ -1461,7 +1461,7 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
   const bool event = io.event && event_path(sh);
   if (event) {  // up to and including the gather: one cluster launch
     CLUE_MARK(1);
-    CLUE_CHECK(launch_event_front(sh, prm, io, *io.grid, *io.event, b, kEventLargeTilePoints, st));
+    CLUE_CHECK(launch_event_front(sh, prm, io, *io.grid, *io.event, b, st));
     CLUE_MARK(2);
   } else {
     CLUE_CHECK(launch_front(sh, prm, io, b, st, marks));
@@ -1476,7 +1476,6 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
   a.cls_dens = b.cls_dens;
   a.cls_nh = b.cls_nh;
   a.queue = b.counters + 4;
-  a.large_points = event ? kEventLargeTilePoints : kLargeTilePoints;
   a.large_tiles = b.large_tiles;
   a.large_count = b.counters + 3;
   a.rec_dens = b.rec_dens;
@@ -1511,7 +1510,10 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
     a.rec_cell = b.rec_cell;
     a.event_exact = b.event_exact;
     a.n_events = sh.n_events;
-    a.walk = b.cls_nh;  // k_work_order's scratch, free once it has run
+    if (sweep_tile_blocks(prm, n, sh.n_tiles))
+      a.work_dens = nullptr;
+    else
+      a.walk = b.cls_nh;  // k_work_order's scratch, which the fast path leaves free
   }
   CLUE_CHECK(launch_work_order(D, prm, a, st));
   CLUE_MARK(3);

@@ -31,9 +31,8 @@ struct SweepArgs {
   // each counts the 32-point work items taken so far (k_gather resets
   // both), so warps that finish early take the next item.
   int32_t* queue;
-  // Tiles of more than large_points points (listed by the binning or the tile
-  // sort) and their count: k_cells gives each of them a whole block.
-  int32_t large_points;
+  // Tiles of more than 256 points (listed by the binning or the tile sort) and
+  // their count: k_cells gives each of them a whole block.
   const int32_t* large_tiles;
   const int32_t* large_count;
   // Exact-sum density (flat kernel): the density records again, in cell-layout
@@ -47,7 +46,8 @@ struct SweepArgs {
   // Walk order of the cell layout (k_cells): walk[k] is the layout position
   // visited k-th, tile by tile, cells in strips of 4 rows so that consecutive
   // points are spatial neighbours. Orders the density work and the
-  // nearest-higher threads.
+  // nearest-higher threads. Null, like work_dens, when the sweeps take the points
+  // in layout order (sweep_tile_blocks).
   int32_t* walk;
   // Packed candidate records of the fast path (D = 2 or 3).
   float4* rec_dens;  // {x, y, [z], v}: v = flat * w for the flat kernel, else w
@@ -94,6 +94,12 @@ cudaError_t launch_work_order(int D, const RunParams& p, const SweepArgs& a, cud
 // kGroupPoints points (density_group.cu).
 constexpr int64_t kGroupPoints = 1 << 16;
 cudaError_t launch_density_group(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
+// Runs whose sweeps give every point a group of lanes (n <= kGroupPoints) take the
+// points in layout order, and k_cells_tile lays the cells out with a block per tile;
+// `walk` and `work_dens` are then null. Above kTileBlocks tiles most hold too few
+// points for a block of their own.
+constexpr int64_t kTileBlocks = 4096;
+bool sweep_tile_blocks(const RunParams& p, int64_t n, int64_t n_tiles);
 // The sweeps off the fast path: any number of dimensions, metric, kernel and
 // option (sweep_any.cu).
 cudaError_t launch_density_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
