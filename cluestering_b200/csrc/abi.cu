@@ -507,11 +507,13 @@ RunParams make_run_params(const clue_params* p, const clue_points* pts, const cl
     if (m == 0.5f && e - 1 >= -125 && e - 1 <= 125)
       r.gauss_inv_den = std::ldexp(1.0f, 1 - e);
     // exponents of in-range pairs lie in [-(dc^2/den)(1 + 2^-22), 0]
-    r.exp_in_range = std::isfinite(den) && den > 0.0f &&
-                     (double)p->dc * (double)p->dc / (double)den <= 100.0;
+    const double most = (double)p->dc * (double)p->dc / (double)den;
+    if (std::isfinite(den) && den > 0.0f)
+      r.exp_in_range = most <= 79.0 ? 2 : most <= 100.0 ? 1 : 0;
   } else if (p->kernel_kind == CLUE_KERNEL_EXPONENTIAL) {
     // exponents lie in [-(avg * dc)(1 + 2^-23), 0]
-    r.exp_in_range = (double)p->kernel_params[0] * (double)p->dc <= 100.0;
+    const double most = (double)p->kernel_params[0] * (double)p->dc;
+    r.exp_in_range = most <= 79.0 ? 2 : most <= 100.0 ? 1 : 0;
   }
   return r;
 }

@@ -97,7 +97,8 @@ struct RunParams {
   // so the division can be a multiplication.
   float gauss_inv_den;
   // Nonzero when every exponent the kernel can see for an in-range pair
-  // (distance <= dc) lies where clue_expf needs no special-case branch.
+  // (distance <= dc) lies where clue_expf needs no special-case branch; 2 when it
+  // also lies in [-80, 0] (clue_expf_normal).
   int32_t exp_in_range;
   // Density sweep, warps whose lanes have different search boxes: the warp
   // streams the union of the boxes when the union holds at most
@@ -279,6 +280,24 @@ __device__ __forceinline__ float kernel_value_in_range(const RunParams& p, float
     return __fmul_rn(p.kernel_p1, p.exp_in_range ? clue_expf_core(x) : clue_expf(x));
   }
   return p.kernel_p0;
+}
+
+// kernel_value_in_range decided at compile time: KIND the kernel, and with NORMAL the
+// run's exp_in_range is 2 (and, for the Gaussian kernel, gauss_inv_den not 0). A
+// choice per pair between forms of the exponential is turned into evaluating both:
+// the density of a 262,144-hit 3-D event took 1,608 us with it, 1,379 us without; of
+// 262,144 2-D points with the Gaussian kernel 1,215 and 931 us.
+template <int KIND, bool NORMAL>
+__device__ __forceinline__ float kernel_value_of(const RunParams& p, float dist, bool self) {
+  if (!NORMAL)
+    return kernel_value_in_range(p, dist, self);
+  const float x = KIND == CLUE_KERNEL_GAUSSIAN ? __fmul_rn(__fmul_rn(-dist, dist), p.gauss_inv_den)
+                                               : __fmul_rn(-p.kernel_p0, dist);
+  const float k = __fmul_rn(p.kernel_p1, clue_expf_normal(x));
+  return self ? 1.0f : k;
+}
+inline bool kernel_value_normal(const RunParams& p) {
+  return p.exp_in_range == 2 && (p.kernel_kind != CLUE_KERNEL_GAUSSIAN || p.gauss_inv_den != 0.0f);
 }
 
 // ---------------------------------------------------------------------------

@@ -58,20 +58,7 @@ struct NearGroup {
   uint16_t list[32 * G];  // the set bits of G words, in order
 };
 
-// Distance from x to the slab of cell c along one dimension, less a margin that
-// covers the rounding of cell_coord and of the slab's ends. The first and last
-// cells also hold what lies beyond them.
-__device__ __forceinline__ float slab_gap(float x, int c, int s, float lo, float inv) {
-  if (!(inv > 0.0f))
-    return 0.0f;
-  const float width = __fdividef(1.0f, inv);
-  const float margin = 1e-5f * (fabsf(lo) + (float)s * width);
-  const float below = lo + (float)c * width - x, above = x - (lo + (float)(c + 1) * width);
-  const float gap = fmaxf(c > 0 ? below : 0.0f, c < s - 1 ? above : 0.0f);
-  return fmaxf(gap - margin, 0.0f);
-}
-
-template <int D, int KIND, int G, int NT, int MINB>
+template <int D, int KIND, bool NORMAL, int G, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_density_group(const RunParams p, const SweepArgs a) {
   constexpr int P = 32 / G;  // points of a warp at a time
   constexpr unsigned kGroup = G == 32 ? kFullMask : (1u << G) - 1u;
@@ -206,8 +193,8 @@ __global__ void __launch_bounds__(NT, MINB) k_density_group(const RunParams p, c
             }
             const int c0 = ct.c0 + r;
             // what is left of the reach along the last dimension
-            const float gap0 = slab_gap(xi[0], c0, ct.s, ct.lo[0], ct.inv[0]);
-            const float gap1 = D == 3 ? slab_gap(xi[1], c1, ct.s, ct.lo[1], ct.inv[1]) : 0.0f;
+            const float gap0 = slab_gap(xi[0], xi[0], c0, ct.s, ct.lo[0], ct.inv[0]);
+            const float gap1 = D == 3 ? slab_gap(xi[1], xi[1], c1, ct.s, ct.lo[1], ct.inv[1]) : 0.0f;
             const float left2 = R2 * 1.00001f - gap0 * gap0 - gap1 * gap1;
             // (a NaN coordinate has no gap and no cells but the first)
             const bool here = exact || (ct.bit < b0 + kBits && ct.bit + ct.points > b0);
@@ -305,7 +292,7 @@ __global__ void __launch_bounds__(NT, MINB) k_density_group(const RunParams p, c
               if (KIND == CLUE_KERNEL_FLAT)
                 add = q == s ? wi : v;
               else
-                add = __fmul_rn(kernel_value_in_range(p, __fsqrt_rn(sq_dist<D>(xi, r)), q == s), v);
+                add = __fmul_rn(kernel_value_of<KIND, NORMAL>(p, __fsqrt_rn(sq_dist<D>(xi, r)), q == s), v);
             }
             sh.add[l] = add;
             __syncwarp();
@@ -358,12 +345,12 @@ __global__ void __launch_bounds__(NT, MINB) k_density_group(const RunParams p, c
   }
 }
 
-template <int D, int KIND, int G>
+template <int D, int KIND, bool NORMAL, int G>
 cudaError_t launch(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   constexpr int NT = 128;
   constexpr int smem = (int)sizeof(NearGroup<G>) * (NT / G);
   const int64_t blocks = (a.n * G + NT - 1) / NT;
-  const auto kernel = k_density_group<D, KIND, G, NT, 7>;
+  const auto kernel = k_density_group<D, KIND, NORMAL, G, NT, 7>;
   kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)sm_count() * 16)), NT, smem, st>>>(p, a);
   count_launches(1);
   return cudaGetLastError();
@@ -372,9 +359,13 @@ cudaError_t launch(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
 template <int D, int G>
 cudaError_t launch_kind(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   switch (p.kernel_kind) {
-    case CLUE_KERNEL_FLAT: return launch<D, CLUE_KERNEL_FLAT, G>(p, a, st);
-    case CLUE_KERNEL_GAUSSIAN: return launch<D, CLUE_KERNEL_GAUSSIAN, G>(p, a, st);
-    default: return launch<D, CLUE_KERNEL_EXPONENTIAL, G>(p, a, st);
+    case CLUE_KERNEL_FLAT: return launch<D, CLUE_KERNEL_FLAT, false, G>(p, a, st);
+    case CLUE_KERNEL_GAUSSIAN:
+      return kernel_value_normal(p) ? launch<D, CLUE_KERNEL_GAUSSIAN, true, G>(p, a, st)
+                                    : launch<D, CLUE_KERNEL_GAUSSIAN, false, G>(p, a, st);
+    default:
+      return kernel_value_normal(p) ? launch<D, CLUE_KERNEL_EXPONENTIAL, true, G>(p, a, st)
+                                    : launch<D, CLUE_KERNEL_EXPONENTIAL, false, G>(p, a, st);
   }
 }
 

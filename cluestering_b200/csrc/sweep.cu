@@ -206,7 +206,7 @@ __device__ __forceinline__ void cell_axis(const GridDesc& g, int b, int s, int d
 }
 
 // Contribution of candidate record r (sorted position q) to rho_i.
-template <int D, int KIND>
+template <int D, int KIND, bool NORMAL>
 __device__ __forceinline__ void density_add(const RunParams& p, const float* xi, const float4& r,
                                             bool self, float wi, float& rho) {
   const float d2 = sq_dist<D>(xi, r);
@@ -215,7 +215,7 @@ __device__ __forceinline__ void density_add(const RunParams& p, const float* xi,
     if (KIND == CLUE_KERNEL_FLAT) {
       rho = __fadd_rn(rho, self ? wi : v);
     } else {
-      const float k = kernel_value_in_range(p, __fsqrt_rn(d2), self);
+      const float k = kernel_value_of<KIND, NORMAL>(p, __fsqrt_rn(d2), self);
       rho = __fadd_rn(rho, __fmul_rn(k, v));
     }
   }
@@ -268,7 +268,7 @@ __device__ __forceinline__ void stream_issue(float4 (*ring)[kChunk], const int* 
 // records the lane takes: the lanes of a warp seldom have the same candidates
 // in range, and a kernel evaluated inside the candidate loop would run
 // whenever any lane is in range.
-template <int D, int KIND>
+template <int D, int KIND, bool NORMAL>
 __device__ __forceinline__ void density_chunk_masked(const RunParams& p, unsigned long long xi_xy,
                                                      float zi, const ulonglong2* chunk, int cnt,
                                                      unsigned acc, int jself, float wi,
@@ -300,7 +300,7 @@ __device__ __forceinline__ void density_chunk_masked(const RunParams& p, unsigne
     if (KIND == CLUE_KERNEL_FLAT) {
       rho = __fadd_rn(rho, j == jself ? wi : v);
     } else {
-      const float k = kernel_value_in_range(p, __fsqrt_rn(d2), j == jself);
+      const float k = kernel_value_of<KIND, NORMAL>(p, __fsqrt_rn(d2), j == jself);
       rho = __fadd_rn(rho, __fmul_rn(k, v));
     }
   }
@@ -548,7 +548,7 @@ __device__ bool density_exact(const RunParams& p, const SweepArgs& a, const Even
 // lane reads each record from shared memory. The stream is the box's rows in
 // order, each a contiguous range of sorted positions, i.e. the reference's
 // summation order. Other warps read candidates from global memory.
-template <int D, int KIND, int NT, int MINB>
+template <int D, int KIND, bool NORMAL, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_density_fast(const RunParams p, const SweepArgs a) {
   __shared__ __align__(16) float4 s_ring[NT / 32][kRing][kChunk];
   __shared__ int s_off[NT / 32][kMaxStream + 1];
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(NT, MINB) k_density_fast(const RunParams p, co
         const int jself = p_self - base;  // own record's place in this chunk, if any
         if (uniform) {
           if (KIND != CLUE_KERNEL_FLAT) {
-            density_chunk_masked<D, KIND>(p, xi_xy, xi[2], chunk, cnt, 0xffffffffu, jself, wi, rho);
+            density_chunk_masked<D, KIND, NORMAL>(p, xi_xy, xi[2], chunk, cnt, 0xffffffffu, jself, wi, rho);
           } else if (cnt == kChunk) {
 #pragma unroll 8
             for (int j = 0; j < kChunk; ++j)
@@ -747,7 +747,7 @@ __global__ void __launch_bounds__(NT, MINB) k_density_fast(const RunParams p, co
             }
             lane_part(cb0, cb1, ilo, ihi);
           }
-          density_chunk_masked<D, KIND>(p, xi_xy, xi[2], chunk, cnt, acc, jself, wi, rho);
+          density_chunk_masked<D, KIND, NORMAL>(p, xi_xy, xi[2], chunk, cnt, acc, jself, wi, rho);
         }
         __syncwarp();
       }
@@ -756,7 +756,7 @@ __global__ void __launch_bounds__(NT, MINB) k_density_fast(const RunParams p, co
     }
     if (!streamed && !done)
       for_each_candidate<D>(a, g, ev.tile_base, inf, sup, [&](int q) {
-        density_add<D, KIND>(p, xi, __ldg(&rec[q]), q == s, wi, rho);
+        density_add<D, KIND, NORMAL>(p, xi, __ldg(&rec[q]), q == s, wi, rho);
         ++tested;
       });
     if (a.stats) {  // warp-uniform
@@ -1844,17 +1844,17 @@ int sweep_grid(int64_t n, int nt, int per_sm) {
 
 // Block shapes of the density sweep (clue_tuning::density_shape):
 // 0: 256 threads, 4 blocks per SM; 1: 128 threads, 8 per SM; 2: 256 threads, 3 per SM.
-template <int D, int KIND>
+template <int D, int KIND, bool NORMAL>
 void launch_density_kind(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   switch (p.dens_shape) {
     case 1:
-      k_density_fast<D, KIND, 128, 8><<<sweep_grid(a.n, 128, 32), 128, 0, st>>>(p, a);
+      k_density_fast<D, KIND, NORMAL, 128, 8><<<sweep_grid(a.n, 128, 32), 128, 0, st>>>(p, a);
       break;
     case 2:
-      k_density_fast<D, KIND, 256, 3><<<sweep_grid(a.n, 256, 16), 256, 0, st>>>(p, a);
+      k_density_fast<D, KIND, NORMAL, 256, 3><<<sweep_grid(a.n, 256, 16), 256, 0, st>>>(p, a);
       break;
     default:
-      k_density_fast<D, KIND, 256, 4><<<sweep_grid(a.n, 256, 16), 256, 0, st>>>(p, a);
+      k_density_fast<D, KIND, NORMAL, 256, 4><<<sweep_grid(a.n, 256, 16), 256, 0, st>>>(p, a);
       break;
   }
 }
@@ -1864,13 +1864,15 @@ cudaError_t launch_density_fast(const RunParams& p, const SweepArgs& a, cudaStre
   count_launches(1);  // the density kernel below; k_gather wrote its records
   switch (p.kernel_kind) {
     case CLUE_KERNEL_FLAT:
-      launch_density_kind<D, CLUE_KERNEL_FLAT>(p, a, st);
+      launch_density_kind<D, CLUE_KERNEL_FLAT, false>(p, a, st);
       break;
     case CLUE_KERNEL_GAUSSIAN:
-      launch_density_kind<D, CLUE_KERNEL_GAUSSIAN>(p, a, st);
+      kernel_value_normal(p) ? launch_density_kind<D, CLUE_KERNEL_GAUSSIAN, true>(p, a, st)
+                             : launch_density_kind<D, CLUE_KERNEL_GAUSSIAN, false>(p, a, st);
       break;
     default:
-      launch_density_kind<D, CLUE_KERNEL_EXPONENTIAL>(p, a, st);
+      kernel_value_normal(p) ? launch_density_kind<D, CLUE_KERNEL_EXPONENTIAL, true>(p, a, st)
+                             : launch_density_kind<D, CLUE_KERNEL_EXPONENTIAL, false>(p, a, st);
       break;
   }
   return cudaGetLastError();

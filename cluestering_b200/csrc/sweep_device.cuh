@@ -173,6 +173,19 @@ __device__ __forceinline__ float reach(float bound2) {
   return __fadd_ru(__fmul_ru(__fsqrt_ru(bound2), 1.000001f), 1e-19f);
 }
 
+// Distance from the interval [x_lo, x_hi] to the slab of cell c along one dimension,
+// less a margin that covers the rounding of cell_coord and of the slab's ends. The
+// first and last cells also hold what lies beyond them.
+__device__ __forceinline__ float slab_gap(float x_lo, float x_hi, int c, int s, float lo, float inv) {
+  if (!(inv > 0.0f))
+    return 0.0f;
+  const float width = __fdividef(1.0f, inv);
+  const float margin = 1e-5f * (fabsf(lo) + (float)s * width);
+  const float below = lo + (float)c * width - x_hi, above = x_lo - (lo + (float)(c + 1) * width);
+  const float gap = fmaxf(c > 0 ? below : 0.0f, c < s - 1 ? above : 0.0f);
+  return fmaxf(gap - margin, 0.0f);
+}
+
 // Asynchronous 16-byte global -> shared copies (per thread, completion by
 // commit groups).
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {

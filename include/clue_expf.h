@@ -88,6 +88,45 @@ CLUE_EXPF_QUAL float clue_expf_core(float x) {
   return CLUE_FMUL(CLUE_FMUL(p, clue_pow2i(n1)), clue_pow2i(n2));
 }
 
+/* clue_expf_core for x in [-80, 0], where n = rint(x*log2(e)) lies in [-116, 0] and
+ * every result is a normal number: the same bits with fewer conversions. Adding
+ * 1.5 * 2^23 rounds x*log2(e) to an integer, to nearest even like rint, and leaves n
+ * in the sum's low bits; p * 2^n is exact, so it is an addition to p's exponent. */
+CLUE_EXPF_QUAL float clue_expf_normal(float x) {
+  const float log2e = 1.44269502162933349609375f;
+  const float ln2_hi = 0.693145751953125f;
+  const float ln2_lo = 1.428606765330187e-06f;
+  const float shift = 12582912.0f; /* 1.5 * 2^23 */
+#if defined(__CUDA_ARCH__)
+  const float t = __fadd_rn(__fmul_rn(x, log2e), shift);
+#else
+  const volatile float product = x * log2e; /* rounded on its own, like the device's */
+  const volatile float t = product + shift;
+#endif
+  const float fn = CLUE_FSUB(t, shift);
+  const float r = CLUE_FSUB(CLUE_FSUB(x, CLUE_FMUL(fn, ln2_hi)), CLUE_FMUL(fn, ln2_lo));
+  float p = 1.98412701138295233249664306640625e-04f;
+  uint32_t bits, n;
+  p = CLUE_FMAF(p, r, 1.38888892251998186111450195312e-03f);
+  p = CLUE_FMAF(p, r, 8.33333376795053482055664062500e-03f);
+  p = CLUE_FMAF(p, r, 4.16666679084300994873046875000e-02f);
+  p = CLUE_FMAF(p, r, 1.66666671633720397949218750000e-01f);
+  p = CLUE_FMAF(p, r, 0.5f);
+  p = CLUE_FMAF(p, r, 1.0f);
+  p = CLUE_FMAF(p, r, 1.0f);
+#if defined(__CUDA_ARCH__)
+  bits = __float_as_uint(p);
+  n = __float_as_uint(t);
+#else
+  {
+    const float tt = t;
+    memcpy(&bits, &p, sizeof bits);
+    memcpy(&n, &tt, sizeof n);
+  }
+#endif
+  return clue_bits_to_float(bits + (n << 23));
+}
+
 CLUE_EXPF_QUAL float clue_expf(float x) {
   /* ln(2^128) rounded down to float: above it the result overflows. */
   const float overflow_at = 88.72283935546875f;
