@@ -763,14 +763,17 @@ __global__ void k_events_order_free(const int32_t* event_exact, const EventDesc*
     *some_ordered = 1;
 }
 
-// Orders the ids of every tile ascending. One warp per tile: tiles of up to
-// kWarpSortCap ids are rank-sorted by the warp with no block barrier; larger
-// tiles are listed for k_tile_sort_large (and for k_cells, which gives each a
-// block). Tiles already in order (one warp of the scatter placed all of them)
-// and tiles whose order does not matter (order_free) are left as they are.
+// Orders the ids of every tile ascending. A warp takes `per_warp` tiles at a time,
+// a lane looking at each: tiles of up to kLaneSortCap ids are sorted by their lane
+// in registers, the others of up to kWarpSortCap are rank-sorted by the warp one by
+// one with no block barrier; larger ones are listed for k_tile_sort_large (and for
+// k_cells, which gives each a block). Tiles already in order (one warp of the
+// scatter placed all of them) and tiles whose order does not matter (order_free) are
+// left as they are.
 constexpr int kWarpSortCap = kLargeTilePoints;
+constexpr int kLaneSortCap = 8;
 __global__ void __launch_bounds__(kThreads) k_tile_sort(const int32_t* tile_offset, int64_t n_tiles,
-                                                        int32_t* perm, int32_t* large,
+                                                        int per_warp, int32_t* perm, int32_t* large,
                                                         int32_t* large_count, const int32_t* event_exact,
                                                         const int32_t* point_event,
                                                         const EventDesc* events,
@@ -780,37 +783,59 @@ __global__ void __launch_bounds__(kThreads) k_tile_sort(const int32_t* tile_offs
   int* ids = s_ids[warp];
   // every event order-free: no tile is sorted, only the large ones listed
   const bool all_free = event_exact && *some_ordered == 0;
-  const int64_t stride = (int64_t)gridDim.x * (kThreads / 32);
-  for (int64_t t = (int64_t)blockIdx.x * (kThreads / 32) + warp; t < n_tiles; t += stride) {
-    const int begin = tile_offset[t], end = tile_offset[t + 1];
-    const int m = end - begin;
-    if (m <= 1)
-      continue;
-    if (m > kWarpSortCap) {
-      if (lane == 0)
-        large[atomicAdd(large_count, 1)] = (int32_t)t;
-      continue;
+  const int64_t stride = (int64_t)gridDim.x * (kThreads / 32) * per_warp;
+  for (int64_t t0 = ((int64_t)blockIdx.x * (kThreads / 32) + warp) * per_warp; t0 < n_tiles; t0 += stride) {
+    int my_begin = 0, my_m = 0;
+    if (lane < per_warp && t0 + lane < n_tiles) {
+      my_begin = tile_offset[t0 + lane];
+      my_m = tile_offset[t0 + lane + 1] - my_begin;
+      if (my_m > kWarpSortCap)
+        large[atomicAdd(large_count, 1)] = (int32_t)(t0 + lane);
     }
-    if (all_free || order_free(event_exact, point_event, events, perm, begin))
-      continue;
-    int unsorted = 0;
-    for (int i = lane; i < m; i += 32) {
-      const int v = perm[begin + i];
-      ids[i] = v;
-      if (i + 1 < m)
-        unsorted |= v > perm[begin + i + 1];
+    const bool mine = my_m > 1 && my_m <= kWarpSortCap && !all_free &&
+                      !order_free(event_exact, point_event, events, perm, my_begin);
+    if (mine && my_m <= kLaneSortCap) {
+      int v[kLaneSortCap];
+#pragma unroll
+      for (int k = 0; k < kLaneSortCap; ++k)
+        v[k] = k < my_m ? perm[my_begin + k] : INT_MAX;
+#pragma unroll
+      for (int k = 0; k < kLaneSortCap; ++k)  // odd-even transposition
+#pragma unroll
+        for (int x = k & 1; x + 1 < kLaneSortCap; x += 2) {
+          const int lo = min(v[x], v[x + 1]);
+          v[x + 1] = max(v[x], v[x + 1]);
+          v[x] = lo;
+        }
+#pragma unroll
+      for (int k = 0; k < kLaneSortCap; ++k)
+        if (k < my_m)
+          perm[my_begin + k] = v[k];
     }
-    __syncwarp();
-    if (__any_sync(kFull, unsorted)) {
-      int32_t* seg = perm + begin;
-      if (m <= 64)
-        warp_rank_sort<2>(seg, m, ids, lane);
-      else if (m <= 128)
-        warp_rank_sort<4>(seg, m, ids, lane);
-      else
-        warp_rank_sort<8>(seg, m, ids, lane);
+    unsigned todo = __ballot_sync(kFull, mine && my_m > kLaneSortCap);
+    while (todo) {
+      const int leader = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const int begin = __shfl_sync(kFull, my_begin, leader), m = __shfl_sync(kFull, my_m, leader);
+      int unsorted = 0;
+      for (int i = lane; i < m; i += 32) {
+        const int v = perm[begin + i];
+        ids[i] = v;
+        if (i + 1 < m)
+          unsorted |= v > perm[begin + i + 1];
+      }
+      __syncwarp();
+      if (__any_sync(kFull, unsorted)) {
+        int32_t* seg = perm + begin;
+        if (m <= 64)
+          warp_rank_sort<2>(seg, m, ids, lane);
+        else if (m <= 128)
+          warp_rank_sort<4>(seg, m, ids, lane);
+        else
+          warp_rank_sort<8>(seg, m, ids, lane);
+      }
+      __syncwarp();
     }
-    __syncwarp();
   }
 }
 
@@ -1245,11 +1270,11 @@ cudaError_t sort_segments(const int32_t* offsets, int64_t n_segments, int32_t* i
     k_events_order_free<<<1, 1024, 0, st>>>(event_exact, b.events, n_events, some_ordered);
     count_launches(1);
   }
-  const int64_t warps_per_block = kThreads / 32;
-  const int blocks =
-      (int)std::max<int64_t>(1, std::min<int64_t>((n_segments + warps_per_block - 1) / warps_per_block,
-                                                  (int64_t)sm_count() * 16));
-  k_tile_sort<<<blocks, kThreads, 0, st>>>(offsets, n_segments, ids, b.large_tiles, large_count,
+  const int per_warp = tiles_per_warp(n_segments);
+  const int64_t per_block = (int64_t)(kThreads / 32) * per_warp;
+  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n_segments + per_block - 1) / per_block,
+                                                                 (int64_t)sm_count() * 16));
+  k_tile_sort<<<blocks, kThreads, 0, st>>>(offsets, n_segments, per_warp, ids, b.large_tiles, large_count,
                                            event_exact, b.point_event, b.events, some_ordered);
   k_tile_sort_large<<<sm_count() * 8, kThreads, 0, st>>>(offsets, b.large_tiles, large_count, ids,
                                                   b.oversize, oversize_count, event_exact,
@@ -1301,6 +1326,10 @@ bool local_labels_ready(int32_t points) {
     granted[dev].store(need, std::memory_order_relaxed);
   }
   return true;
+}
+
+int tiles_per_warp(int64_t n_tiles) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(32, n_tiles / ((int64_t)sm_count() * 256)));
 }
 
 int scan_blocks_for(int64_t n) { return (int)std::max<int64_t>(1, (n + kScanTile - 1) / kScanTile); }

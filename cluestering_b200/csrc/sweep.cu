@@ -1094,11 +1094,66 @@ __device__ void tile_cells(const RunParams& p, const SweepArgs& a, int64_t t, in
   }
 }
 
+// Cell layout of a tile that is one cell (fewer points than two cells' worth) by one
+// lane: layout, walk and work order are the sorted order.
+template <int D>
+__device__ void tile_one_cell(const RunParams& p, const SweepArgs& a, int64_t t, int begin, int m) {
+  const EventDesc ev = a.events[a.sevt[begin]];
+  const GridDesc& g = a.grids[ev.grid];
+  float lo[3] = {0.0f, 0.0f, 0.0f}, inv[3] = {0.0f, 0.0f, 0.0f};
+  int local = (int)t - ev.tile_base;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const int b = local / g.stride[d];
+    local -= b * g.stride[d];
+    cell_axis(g, b, 1, d, lo[d], inv[d]);
+  }
+  float mn[3], mx[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    mn[d] = INFINITY;
+    mx[d] = -INFINITY;
+  }
+  for (int q = begin; q < begin + m; ++q) {
+    const float4 r = a.rec_dens[q];
+    const float x[3] = {r.x, r.y, D == 3 ? r.z : 0.0f};
+    a.cell_slot[q] = begin;
+    a.nh_pos[q] = q;
+    a.nh_q[q] = q;
+    a.rec_cell[q] = r;
+    a.walk[q] = q;
+    a.work_dens[q] = q;
+    if (x[0] == x[0] && x[1] == x[1] && x[2] == x[2]) {  // as in tile_cells
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        mn[d] = fminf(mn[d], x[d]);
+        mx[d] = fmaxf(mx[d], x[d]);
+      }
+    }
+  }
+  CellInfo ci;
+  ci.start = begin;
+  ci.end = begin + m;
+  ci.maxkey = 0ull;
+  a.cell_info[begin] = ci;
+  a.cell_s[t] = 1;
+  if (D == 2) {
+    a.cell_geom[t] = make_float4(lo[0], lo[1], inv[0], inv[1]);
+    a.cell_box[begin] = make_float4(mn[0], mn[1], mx[0], mx[1]);
+  } else {
+    a.cell_geom[2 * t] = make_float4(lo[0], lo[1], lo[2], inv[0]);
+    a.cell_geom[2 * t + 1] = make_float4(inv[1], inv[2], 0.0f, 0.0f);
+    a.cell_box[2 * begin] = make_float4(mn[0], mn[1], mn[2], mx[0]);
+    a.cell_box[2 * begin + 1] = make_float4(mx[1], mx[2], 0.0f, 0.0f);
+  }
+}
+
 // Cell layouts of all tiles. Blocks [0, large_blocks) take the tiles of more
 // than kLargeTilePoints points, which the binning listed, one block each, so
 // a dense tile of thousands of points does not hold up the launch on one warp;
 // they come first so that the heaviest tiles do not run as a tail. The other
-// blocks give one warp to each smaller tile. The kernel waits on dependent
+// blocks give warps `per_warp` smaller tiles at a time (tiles_per_warp), tiles of one
+// cell a lane each and the others the warp one by one. The kernel waits on dependent
 // loads, so it trades registers for resident blocks: in 2-D 6 blocks per SM
 // (40 registers, 8 bytes spilled) took 2.2 ms of the 46.5 M-point batch
 // against 2.7 ms at the compiler's 64 registers (4 blocks); the 3-D form keeps
@@ -1106,7 +1161,7 @@ __device__ void tile_cells(const RunParams& p, const SweepArgs& a, int64_t t, in
 constexpr int kWarpCellSlots = kLargeTilePoints;  // s^D <= m <= 256 (at least 1 point per cell)
 template <int D>
 __global__ void __launch_bounds__(kCellWarps * 32, D == 2 ? 6 : 4) k_cells(const RunParams p, const SweepArgs a,
-                                                          int large_blocks) {
+                                                          int large_blocks, int per_warp) {
   constexpr int E = box_classes<D>();
   static_assert(kWarpCellSlots * kCellWarps <= kCellSlots, "warp counters fit the block's");
   __shared__ int s_cnt[kCellSlots];
@@ -1115,12 +1170,26 @@ __global__ void __launch_bounds__(kCellWarps * 32, D == 2 ? 6 : 4) k_cells(const
   const int warp = threadIdx.x >> 5;
   if ((int)blockIdx.x >= large_blocks) {
     const int64_t wb = (int64_t)blockIdx.x - large_blocks;
-    const int64_t stride = ((int64_t)gridDim.x - large_blocks) * kCellWarps;
-    for (int64_t t = wb * kCellWarps + warp; t < a.n_tiles; t += stride) {
-      if (a.tile_offset[t + 1] - a.tile_offset[t] > kLargeTilePoints)
-        continue;
-      tile_cells<D, 32>(p, a, t, s_cnt + warp * kWarpCellSlots, s_cls[warp],
-                        s_cnt2 + warp * kWarpCellSlots);
+    const int64_t stride = ((int64_t)gridDim.x - large_blocks) * kCellWarps * per_warp;
+    const int lane = threadIdx.x & 31;
+    // points of a tile of one cell: fewer than two cells' worth per dimension (and
+    // not too many for a lane)
+    const int one_cell = min(16, p.cell_points * (D == 2 ? 4 : 8));
+    for (int64_t t0 = (wb * kCellWarps + warp) * per_warp; t0 < a.n_tiles; t0 += stride) {
+      int begin = 0, m = 0;
+      if (lane < per_warp && t0 + lane < a.n_tiles) {
+        begin = a.tile_offset[t0 + lane];
+        m = a.tile_offset[t0 + lane + 1] - begin;
+      }
+      if (per_warp > 1 && m > 0 && m < one_cell)
+        tile_one_cell<D>(p, a, t0 + lane, begin, m);
+      unsigned todo =
+          __ballot_sync(kFullMask, m > 0 && m <= kLargeTilePoints && (per_warp == 1 || m >= one_cell));
+      while (todo) {
+        tile_cells<D, 32>(p, a, t0 + __ffs(todo) - 1, s_cnt + warp * kWarpCellSlots, s_cls[warp],
+                          s_cnt2 + warp * kWarpCellSlots);
+        todo &= todo - 1;
+      }
     }
   } else {
     const int n_large = *a.large_count;
@@ -1821,15 +1890,17 @@ cudaError_t launch_work_order(int D, const RunParams& p, const SweepArgs& a, cud
       k_cells_tile<3><<<blocks, kThreads, 0, st>>>(p, a);
     count_launches(1);
   } else if (a.nh_pos) {
+    const int per_warp = tiles_per_warp(a.n_tiles);
+    const int64_t per_block = (int64_t)kCellWarps * per_warp;
     const int warp_blocks =
-        (int)std::max<int64_t>(1, std::min<int64_t>((a.n_tiles + kCellWarps - 1) / kCellWarps, (int64_t)sm_count() * 32));
+        (int)std::max<int64_t>(1, std::min<int64_t>((a.n_tiles + per_block - 1) / per_block, (int64_t)sm_count() * 32));
     // blocks for the large tiles: at most one per tile that can be large
     const int large_blocks =
         (int)std::max<int64_t>(1, std::min<int64_t>(a.n / (kLargeTilePoints + 1), (int64_t)sm_count() * 24));
     if (D == 2)
-      k_cells<2><<<large_blocks + warp_blocks, kCellWarps * 32, 0, st>>>(p, a, large_blocks);
+      k_cells<2><<<large_blocks + warp_blocks, kCellWarps * 32, 0, st>>>(p, a, large_blocks, per_warp);
     else
-      k_cells<3><<<large_blocks + warp_blocks, kCellWarps * 32, 0, st>>>(p, a, large_blocks);
+      k_cells<3><<<large_blocks + warp_blocks, kCellWarps * 32, 0, st>>>(p, a, large_blocks, per_warp);
     count_launches(1);
   }
   return cudaGetLastError();
