@@ -104,6 +104,11 @@ bool sweep_tile_blocks(const RunParams& p, int64_t n, int64_t n_tiles);
 // option (sweep_any.cu).
 cudaError_t launch_density_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 cudaError_t launch_nearest_higher_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
+// The same with a warp per point, for runs of at most kAnyPointWarps points
+// (sweep_any_point.cu); these take the points in sorted order, without a work order.
+constexpr int64_t kAnyPointWarps = 1 << 14;
+cudaError_t launch_density_point(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
+cudaError_t launch_nearest_higher_point(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 cudaError_t launch_density(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 cudaError_t launch_nearest_higher(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 

@@ -1,6 +1,6 @@
 // sweep_any.cu — local density (core/detail/ClusteringKernels.hpp:29-140) and
 // nearest higher (:142-291) off the fast path: any number of dimensions, metric,
-// kernel and option.
+// kernel and option. (Up to kAnyPointWarps points: sweep_any_point.cu.)
 //
 // A block of 8 warps takes 32 points of the work order, lane l of every warp
 // holding the l-th, and passes over those of one tile together. The tiles of the
@@ -28,7 +28,6 @@ namespace clue_impl {
 namespace {
 
 constexpr int kWarps = kThreads / 32;
-constexpr int kAnyMetric = -1;  // the metric of the run, decided per pair
 
 // Floats per record in shared memory: whole vectors.
 template <int D>
@@ -67,26 +66,6 @@ struct NearestStage : Stage<D> {
   uint64_t key[kWarps][32];
   AnyBest best[kWarps][32];
 };
-
-// metric_inner for the metric of the instantiation.
-template <int D, int METRIC>
-__device__ __forceinline__ float inner_distance(const RunParams& p, const float* xi, const float* xj, const float* si,
-                                                const float* sj) {
-  if (METRIC == kAnyMetric)
-    return metric_inner<D>(p, xi, xj, si, sj);
-  float acc = 0.0f;
-#pragma unroll
-  for (int d = D - 1; d >= 0; --d) {
-    float diff = __fsub_rn(xi[d], xj[d]);
-    if (METRIC == CLUE_METRIC_PERIODIC_EUCLIDEAN) {
-      diff = fabsf(diff);
-      diff = std_min(diff, __fsub_rn(p.mparam[d], diff));
-    }
-    // the right fold starts from +0 and a square is never -0: exact
-    acc = d == D - 1 ? __fmul_rn(diff, diff) : __fadd_rn(__fmul_rn(diff, diff), acc);
-  }
-  return acc;
-}
 
 // The points of an item, one per lane, alike in every warp, and the passes over
 // them. A pass takes the lanes of one tile (`in`), whose boxes are intervals of
@@ -570,10 +549,14 @@ cudaError_t launch_sweep(bool density, int D, const RunParams& p, const SweepArg
 }  // namespace
 
 cudaError_t launch_density_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
+  if (a.n <= kAnyPointWarps)
+    return launch_density_point(D, p, a, st);
   return launch_sweep(true, D, p, a, st);
 }
 
 cudaError_t launch_nearest_higher_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
+  if (a.n <= kAnyPointWarps)
+    return launch_nearest_higher_point(D, p, a, st);
   return launch_sweep(false, D, p, a, st);
 }
 

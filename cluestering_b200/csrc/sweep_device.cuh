@@ -67,6 +67,28 @@ __device__ __forceinline__ void load_point(const RunParams& p, const SweepArgs& 
   }
 }
 
+constexpr int kAnyMetric = -1;  // the metric of the run, decided per pair
+
+// metric_inner for the metric of the instantiation.
+template <int D, int METRIC>
+__device__ __forceinline__ float inner_distance(const RunParams& p, const float* xi, const float* xj, const float* si,
+                                                const float* sj) {
+  if (METRIC == kAnyMetric)
+    return metric_inner<D>(p, xi, xj, si, sj);
+  float acc = 0.0f;
+#pragma unroll
+  for (int d = D - 1; d >= 0; --d) {
+    float diff = __fsub_rn(xi[d], xj[d]);
+    if (METRIC == CLUE_METRIC_PERIODIC_EUCLIDEAN) {
+      diff = fabsf(diff);
+      diff = std_min(diff, __fsub_rn(p.mparam[d], diff));
+    }
+    // the right fold starts from +0 and a square is never -0: exact
+    acc = d == D - 1 ? __fmul_rn(diff, diff) : __fadd_rn(__fmul_rn(diff, diff), acc);
+  }
+  return acc;
+}
+
 // Order-preserving image of a density: key(a) > key(b) iff a > b and equal
 // densities give equal keys. NaN maps to 0, below every number, so a NaN
 // density is never "higher" (every comparison with NaN is false). Densities

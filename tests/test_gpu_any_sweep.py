@@ -1,9 +1,10 @@
 """The sweeps off the fast path (csrc/sweep_any.cu: a block per 32 points of one
-tile, walking the union of their search boxes) where that union is unusual, against
-the checker bit for bit: items that span events, boxes that wrap round or cover the
-whole circle, boxes of more tiles than the block stages at a time, boxes that differ
-much in many dimensions, boxes without the point's own tile, and weights or kernels
-whose out-of-range terms are not zero.
+tile, walking the union of their search boxes; csrc/sweep_any_point.cu: a warp per
+point, up to 16,384 points) where the boxes are unusual, against the checker bit for
+bit: items that span events, boxes that wrap round or cover the whole circle, boxes of
+more tiles than are staged at a time, boxes that differ much in many dimensions, boxes
+without the point's own tile, and weights or kernels whose out-of-range terms are not
+zero. Each test runs below and above the line between the two forms.
 """
 
 import math
@@ -19,18 +20,19 @@ from tests.test_gpu_parity import assert_identical, check, run_gpu, run_oracle
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("events", [40, 200])
 @pytest.mark.parametrize("mode", [clue.GRID_PER_EVENT, clue.GRID_SHARED])
-def test_items_across_events(mode):
-    ev, sizes = W.batch_2d(40, 1, 700, seed=31)
+def test_items_across_events(mode, events):
+    ev, sizes = W.batch_2d(events, 1, 700, seed=31)
     w = np.random.default_rng(32).exponential(1.0, ev.n).astype(np.float32)
     check(ev.coords, w, 1.5, 3.0, 2.0, metric="manhattan", sizes=sizes, grid_mode=mode, path="device")
 
 
+@pytest.mark.parametrize("n", [4099, 17001])
 @pytest.mark.parametrize("r", [0.05, 0.7, 2.9, 7.0])
 @pytest.mark.parametrize("wrapped", [[0, 1], [1, 0], [1, 1]])
-def test_wrapped_boxes(r, wrapped):
+def test_wrapped_boxes(r, wrapped, n):
     rng = np.random.default_rng(33)
-    n = 4099
     c = np.mod(np.stack([rng.normal(0.1, 0.8, n), rng.normal(6.2, 0.9, n)]), 2 * math.pi).astype(np.float32)
     w = rng.exponential(1.0, n).astype(np.float32)
     check(c, w, r, 2.0, 1.3 * r, metric="periodic_euclidean", metric_params=(2 * math.pi, 2 * math.pi),
@@ -38,7 +40,8 @@ def test_wrapped_boxes(r, wrapped):
 
 
 @pytest.mark.parametrize("D,n,ppt,r", [(1, 3001, 2, 2.0), (2, 3001, 2, 12.0), (4, 6001, 4, 6.0), (5, 20011, 16, 2.0),
-                                       (6, 5003, 4, 1.0)])
+                                       (6, 5003, 4, 1.0), (1, 17001, 2, 0.5), (2, 17001, 2, 3.0), (4, 17001, 4, 4.0),
+                                       (6, 17001, 4, 1.0), (2, 16384, 128, 1.0), (2, 16385, 128, 1.0)])
 def test_boxes_of_many_tiles(D, n, ppt, r):
     rng = np.random.default_rng(34 + D)
     c = rng.uniform(0.0, 20.0, (D, n)).astype(np.float32)
@@ -49,19 +52,21 @@ def test_boxes_of_many_tiles(D, n, ppt, r):
                                         exp_mode=O.EXP_CLUE, n_threads=8))
 
 
-def test_box_without_the_own_tile():
+@pytest.mark.parametrize("n", [3000, 17000])
+def test_box_without_the_own_tile(n):
     # a radius beyond the int range of get_bin's conversion sends the box's upper
     # end to bin 0 (x86 conversion)
-    ev = W.blobs(3000, 6, 0.0, 30.0, 1.0, 0.1, seed=35, weights="exponential")
+    ev = W.blobs(n, 6, 0.0, 30.0, 1.0, 0.1, seed=35, weights="exponential")
     check(ev.coords, ev.weights, 1.0, 3.0, 1e13, metric="manhattan", path="device")
     check(ev.coords, ev.weights, 3e12, 3.0, 1e13, metric="weighted_euclidean", metric_params=(1.0, 2.0), path="device")
 
 
+@pytest.mark.parametrize("n", [2500, 17000])
 @pytest.mark.parametrize("kernel,params", [("flat", (0.5,)), ("gaussian", (0.8, 2.0)), ("exponential", (1.2, 0.7))])
-def test_infinite_and_nan_weights(kernel, params):
+def test_infinite_and_nan_weights(kernel, params, n):
     # 0 * k * w of a candidate out of range is NaN for such a weight, and so is
     # every density whose search box holds it
-    ev = W.blobs(2500, 5, 0.0, 60.0, 1.0, 0.1, seed=36, weights="exponential")
+    ev = W.blobs(n, 5, 0.0, 60.0, 1.0, 0.1, seed=36, weights="exponential")
     w = ev.weights.copy()
     w[[7, 900]] = np.inf
     w[1400] = np.nan
@@ -76,8 +81,8 @@ def test_infinite_and_nan_weights(kernel, params):
     assert np.array_equal(g["ci"], o.cluster_index)
 
 
-def test_lattice_ties_and_equal_tags_in_four_dimensions():
+@pytest.mark.parametrize("n", [6000, 17000])
+def test_lattice_ties_and_equal_tags_in_four_dimensions(n):
     rng = np.random.default_rng(37)
-    n = 6000
     c = rng.integers(0, 7, (4, n)).astype(np.float32)
     check(c, np.ones(n, np.float32), 1.0, 2.0, 1.5, tags=rng.integers(0, 3, n).astype(np.uint32), path="device")
