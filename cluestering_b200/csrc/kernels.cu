@@ -304,7 +304,11 @@ __device__ __forceinline__ int sort_event_of(const EventDesc* events, int n_even
 
 // Tile ids and per-run tile counts; also the exact-sum bounds of the event
 // (flat kernel, when event_exact is given), as in k_bin. s_col holds one
-// counter per tile of the warp's event (max_tiles per warp).
+// counter per tile of the warp's event (max_tiles per warp). DD: 2 or 3 dimensions, or
+// 0 for any number; the grid is held in registers and the points of kStableAhead rounds
+// are loaded before they are binned (262,144 hits in 3-D: 74 us with neither, 27 us).
+constexpr int kStableAhead = 4;
+template <int DD>
 __global__ void __launch_bounds__(kThreads) k_bin_stable(RunParams p, CoordPtrs x, const EventDesc* events,
                                                          int n_events, int n_warps, const GridDesc* grids,
                                                          int32_t* tile_of, int32_t* point_event,
@@ -319,7 +323,8 @@ __global__ void __launch_bounds__(kThreads) k_bin_stable(RunParams p, CoordPtrs 
   int* col = s_col + (threadIdx.x >> 5) * max_tiles;
   const int e = sort_event_of(events, n_events, w);
   const EventDesc ev = events[e];
-  const GridDesc& g = grids[ev.grid];
+  const GridDesc g = grids[ev.grid];
+  const int D = DD ? DD : p.D;
   const int c = w - ev.sort_first;
   const int T = g.T;
   for (int t = lane; t < T; t += 32)
@@ -330,36 +335,49 @@ __global__ void __launch_bounds__(kThreads) k_bin_stable(RunParams p, CoordPtrs 
   const bool bounds = event_exact && p.kernel_kind == CLUE_KERNEL_FLAT;
   int lsb = INT_MAX, bad = 0;
   uint32_t vb = 0, wb = 0;
-#pragma unroll 4
-  for (int base = begin; base < end; base += 32) {
-    const int i = base + lane;
-    const bool valid = i < end;
-    int t = -1;
-    if (valid) {
-      int b = 0;
-      for (int d = 0; d < p.D; ++d)
-        b += g.stride[d] * get_bin(g, p, x.p[d][i], d);
-      t = b;
-      tile_of[i] = ev.tile_base + t;
-      point_event[i] = e;
-      if (bounds) {
-        const float wt = weight[i];
-        const float v = __fmul_rn(p.kernel_p0, wt);  // a neighbour's fl(flat * w_j)
-        const int bd = !(wt >= 0.0f) || signbit(wt) || isinf(wt) || isinf(v);
-        bad |= bd;
-        if (!bd) {
-          if (v > 0.0f)
-            lsb = min(lsb, lsb_exponent(v));
-          if (wt > 0.0f)
-            lsb = min(lsb, lsb_exponent(wt));
-          vb = max(vb, __float_as_uint(v));
-          wb = max(wb, __float_as_uint(wt));
+  for (int base = begin; base < end; base += 32 * kStableAhead) {
+    float px[kStableAhead][DD ? DD : 1], pw[kStableAhead];
+#pragma unroll
+    for (int u = 0; u < kStableAhead; ++u) {
+      const int i = base + u * 32 + lane;
+#pragma unroll
+      for (int d = 0; d < DD; ++d)
+        px[u][d] = i < end ? x.p[d][i] : 0.0f;
+      pw[u] = bounds && i < end ? weight[i] : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kStableAhead; ++u) {
+      const int i = base + u * 32 + lane;
+      const bool valid = i < end;
+      int t = -1;
+      if (valid) {
+        int b = 0;
+#pragma unroll
+        for (int d = 0; d < (DD ? DD : kMaxDim); ++d)
+          if (d < D)
+            b += g.stride[d] * get_bin(g, p, DD ? px[u][DD ? d : 0] : x.p[d][i], d);
+        t = b;
+        tile_of[i] = ev.tile_base + t;
+        point_event[i] = e;
+        if (bounds) {
+          const float wt = pw[u];
+          const float v = __fmul_rn(p.kernel_p0, wt);  // a neighbour's fl(flat * w_j)
+          const int bd = !(wt >= 0.0f) || signbit(wt) || isinf(wt) || isinf(v);
+          bad |= bd;
+          if (!bd) {
+            if (v > 0.0f)
+              lsb = min(lsb, lsb_exponent(v));
+            if (wt > 0.0f)
+              lsb = min(lsb, lsb_exponent(wt));
+            vb = max(vb, __float_as_uint(v));
+            wb = max(wb, __float_as_uint(wt));
+          }
         }
       }
+      const unsigned mask = __match_any_sync(kFull, t);
+      if (valid && lane == __ffs(mask) - 1)
+        atomicAdd(&col[t], __popc(mask));  // ordered with later rounds' leaders, no barrier
     }
-    const unsigned mask = __match_any_sync(kFull, t);
-    if (valid && lane == __ffs(mask) - 1)
-      atomicAdd(&col[t], __popc(mask));  // ordered with later rounds' leaders, no barrier
   }
   __syncwarp();
   int32_t* row = matrix + (int64_t)ev.sort_base + (int64_t)c * T;
@@ -384,37 +402,66 @@ __global__ void __launch_bounds__(kThreads) k_bin_stable(RunParams p, CoordPtrs 
   }
 }
 
-// One thread per tile: the tile's counts over the runs of its event become
-// exclusive prefixes (in place), and the total goes to tile_count. Threads of
-// consecutive tiles read consecutive entries of each run's row.
+// The counts of every tile over the runs of its event become exclusive prefixes (in
+// place), and the total goes to tile_count. A block takes 32 consecutive tiles: lane l
+// of every warp the l-th, so that a warp reads consecutive entries of a run's row, and
+// warp w the w-th part of the runs, first their sum, then (from the other warps' sums)
+// their prefixes. (One thread per tile over all runs: 87 us for the 2,197 tiles and 256
+// runs of a 262,144-hit event, 10 us here.)
 __global__ void __launch_bounds__(kThreads) k_tile_prefix(const EventDesc* events, const GridDesc* grids,
                                                           int64_t n_tiles, const int32_t* tile_event,
-                                                          int32_t* matrix, int32_t* tile_count) {
-  for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < n_tiles;
-       g += (int64_t)gridDim.x * blockDim.x) {
-    const EventDesc ev = events[tile_event[g]];
-    const int64_t T = grids[ev.grid].T;
-    int32_t* m = matrix + (int64_t)ev.sort_base + (g - ev.tile_base);
-    int run = 0;
+                                                          int32_t* matrix, int32_t* tile_count,
+                                                          int32_t* large, int32_t* large_count) {
+  constexpr int kParts = kThreads / 32;
+  __shared__ int s_sum[kParts][32];
+  const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+  for (int64_t g0 = (int64_t)blockIdx.x * 32; g0 < n_tiles; g0 += (int64_t)gridDim.x * 32) {
+    const int64_t g = g0 + lane;
+    const bool valid = g < n_tiles;
+    int64_t T = 0;
+    int32_t* m = matrix;
+    int c0 = 0, c1 = 0;
+    if (valid) {
+      const EventDesc ev = events[tile_event[g]];
+      T = grids[ev.grid].T;
+      m = matrix + (int64_t)ev.sort_base + (g - ev.tile_base);
+      const int per = (ev.sort_chunks + kParts - 1) / kParts;
+      c0 = min(ev.sort_chunks, part * per);
+      c1 = min(ev.sort_chunks, c0 + per);
+    }
+    int sum = 0;
 #pragma unroll 8
-    for (int c = 0; c < ev.sort_chunks; ++c) {
+    for (int c = c0; c < c1; ++c)
+      sum += m[c * T];
+    s_sum[part][lane] = sum;
+    __syncthreads();
+    int run = 0, all = 0;
+#pragma unroll
+    for (int q = 0; q < kParts; ++q) {
+      run += q < part ? s_sum[q][lane] : 0;
+      all += s_sum[q][lane];
+    }
+#pragma unroll 8
+    for (int c = c0; c < c1; ++c) {
       const int v = m[c * T];
       m[c * T] = run;
       run += v;
     }
-    tile_count[g] = run;
+    if (valid && part == 0) {
+      tile_count[g] = all;
+      if (all > kLargeTilePoints)  // (for k_cells)
+        large[atomicAdd(large_count, 1)] = (int32_t)g;
+    }
+    __syncthreads();  // the sums are rewritten
   }
 }
 
 // Places each run's points at tile offset + the run's prefix in that tile.
-// The first run of each event lists the event's tiles of more than
-// kLargeTilePoints points (for k_cells).
 __global__ void __launch_bounds__(kThreads) k_scatter_stable(const EventDesc* events, int n_events,
                                                              int n_warps, const GridDesc* grids,
                                                              const int32_t* tile_of, const int32_t* matrix,
                                                              int max_tiles, const int32_t* tile_offset,
-                                                             const int32_t* tile_count, int32_t* perm,
-                                                             int32_t* large, int32_t* large_count) {
+                                                             int32_t* perm) {
   extern __shared__ int s_col[];
   const int lane = threadIdx.x & 31;
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -426,33 +473,36 @@ __global__ void __launch_bounds__(kThreads) k_scatter_stable(const EventDesc* ev
   const int c = w - ev.sort_first;
   const int T = grids[ev.grid].T;
   const int32_t* row = matrix + (int64_t)ev.sort_base + (int64_t)c * T;
-  for (int t = lane; t < T; t += 32) {
+#pragma unroll 4
+  for (int t = lane; t < T; t += 32)
     col[t] = tile_offset[ev.tile_base + t] + row[t];
-    if (c == 0 && tile_count[ev.tile_base + t] > kLargeTilePoints)
-      large[atomicAdd(large_count, 1)] = ev.tile_base + t;
-  }
   __syncwarp();
   const int begin = ev.begin + c * ev.sort_len;
   const int end = min(ev.begin + ev.n, begin + ev.sort_len);
-  // Rounds of 32 points in index order; the next round's tile ids are loaded
-  // before this round's cursor updates, so the load latency overlaps them.
-  int t_next = begin + lane < end ? tile_of[begin + lane] - ev.tile_base : -1;
-  for (int base = begin; base < end; base += 32) {
-    const int i = base + lane;
-    const bool valid = i < end;
-    const int t = t_next;
-    t_next = base + 32 + lane < end ? tile_of[base + 32 + lane] - ev.tile_base : -1;
-    const unsigned mask = __match_any_sync(kFull, t);
-    const int leader = __ffs(mask) - 1;
-    int pos = 0;
-    if (valid && lane == leader) {
-      pos = col[t];
-      col[t] = pos + __popc(mask);
+  // Rounds of 32 points in index order; the tile ids of kStableAhead rounds are
+  // loaded before the first one's cursor updates.
+  for (int base = begin; base < end; base += 32 * kStableAhead) {
+    int tile[kStableAhead];
+#pragma unroll
+    for (int u = 0; u < kStableAhead; ++u) {
+      const int i = base + u * 32 + lane;
+      tile[u] = i < end ? tile_of[i] - ev.tile_base : -1;
     }
-    pos = __shfl_sync(kFull, pos, leader);
-    if (valid)
-      perm[pos + __popc(mask & lanemask_lt())] = i;
-    __syncwarp();  // the next round's leaders read these cursors
+#pragma unroll
+    for (int u = 0; u < kStableAhead; ++u) {
+      const int t = tile[u];
+      const unsigned mask = __match_any_sync(kFull, t);
+      const int leader = __ffs(mask) - 1;
+      int pos = 0;
+      if (t >= 0 && lane == leader) {
+        pos = col[t];
+        col[t] = pos + __popc(mask);
+      }
+      pos = __shfl_sync(kFull, pos, leader);
+      if (t >= 0)
+        perm[pos + __popc(mask & lanemask_lt())] = base + u * 32 + lane;
+      __syncwarp();  // the next round's leaders read these cursors
+    }
   }
 }
 
@@ -665,27 +715,70 @@ __global__ void __launch_bounds__(kThreads) k_hist(const int32_t* keys, int64_t 
   }
 }
 
-// Bitonic sort of s[0..P) (P a power of two) by the whole block.
-__device__ void block_bitonic(int* s, int P) {
-  for (int k = 2; k <= P; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = threadIdx.x; i < P; i += blockDim.x) {
-        const int ixj = i ^ j;
-        if (ixj > i) {
-          const int a = s[i], b = s[ixj];
-          const bool up = (i & k) == 0;
-          if ((a > b) == up) {
-            s[i] = b;
-            s[ixj] = a;
-          }
-        }
+// Bitonic sort of a segment of at most E * kThreads ids (ascending) by the block.
+// Thread t holds ids E t .. E t + E - 1: partners less than E apart meet in its
+// registers, less than 32 E apart by shuffles, and only the few stages beyond that (6
+// of the 55 for 1,024 ids) go through shared memory and a barrier. The network it
+// replaces kept every stage in shared memory; the 1,048,576-point event, whose tiles
+// hold up to 2,000 points, spent 76 us in k_tile_sort_large with it and 22 us this way.
+template <int E>
+__device__ void block_bitonic(int32_t* seg, int m, int* s) {
+  const int tid = threadIdx.x;
+  int v[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    v[e] = tid * E + e < m ? seg[tid * E + e] : INT_MAX;
+  __syncthreads();  // every id has been read
+#pragma unroll 1
+  for (int k = 2; k <= E * kThreads; k <<= 1) {
+    int j = k >> 1;
+#pragma unroll 1
+    for (; j >= 32 * E; j >>= 1) {  // partners in other warps
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        s[e * kThreads + tid] = v[e];
+      __syncthreads();
+      const int partner = tid ^ (j / E);
+      const bool keep_min = ((tid * E & j) == 0) == ((tid * E & k) == 0);
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int o = s[e * kThreads + partner];
+        v[e] = keep_min ? min(v[e], o) : max(v[e], o);
       }
       __syncthreads();
     }
+#pragma unroll 1
+    for (; j >= E; j >>= 1) {  // partners in the warp
+      const bool keep_min = ((tid * E & j) == 0) == ((tid * E & k) == 0);
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int o = __shfl_xor_sync(kFull, v[e], j / E);
+        v[e] = keep_min ? min(v[e], o) : max(v[e], o);
+      }
+    }
+    // partners in the thread
+#pragma unroll
+    for (int jj = E / 2; jj > 0; jj >>= 1) {
+      if (jj >= k)
+        continue;
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        if ((e & jj) == 0) {
+          const bool up = ((tid * E + e) & k) == 0;
+          const int lo = min(v[e], v[e | jj]), hi = max(v[e], v[e | jj]);
+          v[e] = up ? lo : hi;
+          v[e | jj] = up ? hi : lo;
+        }
+    }
   }
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if (tid * E + e < m)
+      seg[tid * E + e] = v[e];
+  __syncthreads();
 }
 
-// Sorts a segment of at most kSortCap ids in place (ascending).
+// Sorts a segment of at most kSortCap ids in place (ascending) by the whole block.
 __device__ void sort_segment(int32_t* seg, int m, int* s) {
   // Already ascending? (common when one warp scattered the whole tile)
   int unsorted = 0;
@@ -693,17 +786,16 @@ __device__ void sort_segment(int32_t* seg, int m, int* s) {
     unsorted |= seg[i] > seg[i + 1];
   if (!__syncthreads_or(unsorted))
     return;
-  int P = 1;
-  while (P < m)
-    P <<= 1;
-  for (int i = threadIdx.x; i < P; i += blockDim.x)
-    s[i] = (i < m) ? seg[i] : INT_MAX;
-  __syncthreads();
-  block_bitonic(s, P);
-  for (int i = threadIdx.x; i < m; i += blockDim.x)
-    seg[i] = s[i];
-  __syncthreads();
+  if (m <= 2 * kThreads)
+    block_bitonic<2>(seg, m, s);
+  else if (m <= 4 * kThreads)
+    block_bitonic<4>(seg, m, s);
+  else if (m <= 8 * kThreads)
+    block_bitonic<8>(seg, m, s);
+  else
+    block_bitonic<16>(seg, m, s);
 }
+static_assert(kSortCap == 16 * kThreads, "sort_segment's largest network");
 
 // Rank sort of one segment of m <= 32 * R distinct ids by one warp: lane L
 // holds ids L, L + 32, ... in registers, `ids` holds all of them in shared
@@ -839,63 +931,8 @@ __global__ void __launch_bounds__(kThreads) k_tile_sort(const int32_t* tile_offs
   }
 }
 
-// Ascending bitonic sort of one value per lane across the warp.
-__device__ __forceinline__ int warp_bitonic(int v, int lane) {
-#pragma unroll
-  for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      const int o = __shfl_xor_sync(kFull, v, j);
-      const bool keep_min = ((lane & j) == 0) == ((lane & k) == 0);
-      v = keep_min ? min(v, o) : max(v, o);
-    }
-  }
-  return v;
-}
-
-// Number of entries of the ascending 32-entry run `c` below v.
-__device__ __forceinline__ int count_below(const int* c, int v) {
-  int p = 0;
-#pragma unroll
-  for (int step = 16; step > 0; step >>= 1)
-    p += (c[p + step - 1] < v) ? step : 0;
-  return p + (c[p] < v);
-}
-
-// Segments of kWarpSortCap < m <= kChunkRankCap ids: every warp sorts runs of
-// 32 ids in registers, then each id's position is its place in its own run
-// plus, for every other run, the number of ids below it (ids are distinct).
-constexpr int kChunkRankCap = 1024;
-__device__ void chunk_rank_sort(int32_t* seg, int m, int* s) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int unsorted = 0;
-  for (int i = threadIdx.x; i + 1 < m; i += kThreads)
-    unsorted |= seg[i] > seg[i + 1];
-  if (!__syncthreads_or(unsorted))
-    return;
-  const int runs = (m + 31) >> 5;
-  for (int c = warp; c < runs; c += kThreads / 32) {
-    const int i = c * 32 + lane;
-    s[i] = warp_bitonic(i < m ? seg[i] : INT_MAX, lane);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < runs * 32; i += kThreads) {
-    const int v = s[i];
-    if (v == INT_MAX)
-      continue;
-    const int own = i >> 5;
-    int rank = i & 31;
-    for (int c = 0; c < runs; ++c)
-      if (c != own)
-        rank += count_below(s + c * 32, v);
-    seg[rank] = v;
-  }
-  __syncthreads();
-}
-
 // Tiles listed by k_tile_sort (more than kWarpSortCap ids): one block each.
-// Up to kChunkRankCap ids: chunk_rank_sort; up to kSortCap: a shared-memory
-// bitonic sort; larger tiles become sorted chunks of kSortCap ids, listed for
+// Tiles of more than kSortCap ids become sorted chunks of kSortCap, listed for
 // k_tile_merge.
 __global__ void __launch_bounds__(kThreads) k_tile_sort_large(const int32_t* tile_offset,
                                                               const int32_t* large,
@@ -916,9 +953,7 @@ __global__ void __launch_bounds__(kThreads) k_tile_sort_large(const int32_t* til
     const int m = end - begin;
     if (m <= 1 || order_free(event_exact, point_event, events, perm, begin))
       continue;
-    if (m <= kChunkRankCap) {
-      chunk_rank_sort(perm + begin, m, s);
-    } else if (m <= kSortCap) {
+    if (m <= kSortCap) {
       sort_segment(perm + begin, m, s);
     } else {
       for (int c = begin; c < end; c += kSortCap)
@@ -1438,18 +1473,18 @@ static cudaError_t launch_front(const RunShape& sh, const RunParams& prm, const 
     const int blocks = (sh.sort_warps + wpb - 1) / wpb;
     const size_t smem = (size_t)wpb * sh.max_event_tiles * sizeof(int);
     CLUE_CHECK(fill32(b.counters + 3, 1, 0, st));  // large-tile count
-    k_bin_stable<<<blocks, wpb * 32, smem, st>>>(prm, x, b.events, sh.n_events, sh.sort_warps, b.grids,
-                                                 b.tile_of, b.point_event, matrix,
-                                                 sh.max_event_tiles, io.weight, exact, b.tile_cursor);
+    const auto bin = D == 2 ? k_bin_stable<2> : D == 3 ? k_bin_stable<3> : k_bin_stable<0>;
+    bin<<<blocks, wpb * 32, smem, st>>>(prm, x, b.events, sh.n_events, sh.sort_warps, b.grids, b.tile_of,
+                                        b.point_event, matrix, sh.max_event_tiles, io.weight, exact, b.tile_cursor);
     CLUE_LAUNCHED();
-    k_tile_prefix<<<grid_for(sh.n_tiles), kThreads, 0, st>>>(b.events, b.grids, sh.n_tiles, b.tile_cursor,
-                                                             matrix, b.tile_count);
+    k_tile_prefix<<<grid_for(sh.n_tiles, 32), kThreads, 0, st>>>(b.events, b.grids, sh.n_tiles, b.tile_cursor,
+                                                                 matrix, b.tile_count, b.large_tiles,
+                                                                 b.counters + 3);
     CLUE_LAUNCHED();
     CLUE_CHECK(scan(b.tile_count, b.tile_offset, sh.n_tiles, b.tile_offset + sh.n_tiles, b, st));
     k_scatter_stable<<<blocks, wpb * 32, smem, st>>>(b.events, sh.n_events, sh.sort_warps, b.grids,
                                                      b.tile_of, matrix, sh.max_event_tiles,
-                                                     b.tile_offset, b.tile_count, b.perm,
-                                                     b.large_tiles, b.counters + 3);
+                                                     b.tile_offset, b.perm);
     CLUE_LAUNCHED();
   } else {
     CLUE_CHECK(fill32(b.tile_count, sh.n_tiles, 0, st));

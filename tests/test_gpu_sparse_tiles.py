@@ -36,3 +36,21 @@ def test_shared_grid_of_many_events_3d(binning):
     algo.set_tuning(tile_binning=binning)
     check(c, w, 3.0, 10.0, 4.0, sizes=[e.n for e in evs], grid_mode=clue.GRID_SHARED, kernel="gaussian",
           kernel_params=(1.0, 1.0), clusterer=algo, path="device")
+
+
+# Counting-sort binning puts every tile's ids in order: by a lane, by a warp or by a
+# block's network of 2, 4, 8 or 16 ids a thread, beyond that by merging chunks.
+@pytest.mark.parametrize("m", [2, 8, 9, 33, 129, 256, 257, 511, 512, 513, 1024, 1025, 2048, 2049, 4095, 4096, 4097, 9001])
+def test_ids_of_a_tile_in_order(m):
+    rng = np.random.default_rng(2100 + m)
+    # the first event is one tile of m points in random index order, the second has
+    # several, and the batch keeps the run off the one-cluster form
+    c = rng.normal(0.0, 1.0, (2, m + 777)).astype(np.float32)
+    w = rng.exponential(1.0, m + 777).astype(np.float32)
+    algo = clue.Clusterer(0.3, 2.0, 0.5, points_per_tile=m)
+    algo.set_tuning(tile_binning=0)
+    from oracle import oracle as O
+    from tests.test_gpu_parity import assert_identical, run_gpu
+    g = run_gpu(c, w, 0.3, 2.0, 0.5, sizes=[m, 777], grid_mode=clue.GRID_PER_EVENT, clusterer=algo, path="device")
+    assert_identical(g, O.make_clusters_batched(c, w, [m, 777], 0.3, 2.0, 0.5, shared_grid=False, points_per_tile=m,
+                                                exp_mode=O.EXP_CLUE, n_threads=8))
