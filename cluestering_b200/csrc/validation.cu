@@ -9,12 +9,13 @@
 #include <cfloat>
 
 #include "abi_internal.h"
+#include "sweep_device.cuh"
 
 using namespace clue_impl;
 
-namespace {
+namespace clue_impl {
 
-constexpr int kThreads = 256;
+namespace {
 
 struct CoordTable {
   const float* p[kMaxDim];
@@ -77,7 +78,7 @@ __global__ void __launch_bounds__(kThreads) k_centroids(int D, CoordTable x, con
 // 32 being gathered meanwhile, and every lane adds its distances in the map's
 // order. Bound by the issue of the square roots (about 16 instructions per
 // pair); with one thread per point over all clusters 32,768 points kept 8 warps
-// on each of 128 SMs waiting for their own chains: 4.96 ms, 0.72 ms here.
+// on each of 128 SMs waiting for their own chains: 4.96 ms, 0.69 ms here.
 // DD: the number of dimensions, or 0 for any (D at run time).
 template <int DD>
 __global__ void __launch_bounds__(kThreads) k_silhouette(int D_any, CoordTable x, const int32_t* labels,
@@ -87,7 +88,9 @@ __global__ void __launch_bounds__(kThreads) k_silhouette(int D_any, CoordTable x
   constexpr int kDims = DD ? DD : kMaxDim;
   constexpr int kWarps = kThreads / 32;
   const int D = DD ? DD : D_any;
-  __shared__ float s_x[kWarps][kDims][32];
+  // a point's coordinates together, so that a lane reads them with one or two loads
+  constexpr int kRow = DD == 3 ? 4 : kDims;
+  __shared__ __align__(16) float s_x[kWarps][32][kRow];
   __shared__ int32_t s_m[kWarps][32];
   __shared__ float s_a[kWarps][32], s_b[kWarps][32];
   __shared__ int s_next[kWarps];
@@ -104,15 +107,33 @@ __global__ void __launch_bounds__(kThreads) k_silhouette(int D_any, CoordTable x
 #pragma unroll
   for (int d = 0; d < kDims; ++d)
     xi[d] = (valid && d < D) ? x.p[d][i] : 0.0f;
-  float(*sx)[32] = s_x[warp];
+  float(*sx)[kRow] = s_x[warp];
   int32_t* sm = s_m[warp];
   float b = FLT_MAX;
   const auto distance = [&](int j) {
     float dist = 0.0f;
+    if (DD == 2 || DD == 3) {
+      // the first two dimensions with one packed subtract and multiply (sweep_device.cuh)
+      float x, y, z = 0.0f, sx2, sy2;
+      if (DD == 2) {
+        const float2 v = *reinterpret_cast<const float2*>(sx[j]);
+        x = v.x, y = v.y;
+      } else {
+        const float4 v = *reinterpret_cast<const float4*>(sx[j]);
+        x = v.x, y = v.y, z = v.z;
+      }
+      sq_diff_xy(xi[0], xi[kDims > 1 ? 1 : 0], x, y, sx2, sy2);
+      dist = __fadd_rn(sx2, sy2);
+      if (DD == 3) {
+        const float dz = __fsub_rn(xi[kDims - 1], z);
+        dist = __fadd_rn(dist, __fmul_rn(dz, dz));
+      }
+      return __fsqrt_rn(dist);
+    }
 #pragma unroll
     for (int d = 0; d < kDims; ++d)
       if (d < D) {
-        const float diff = __fsub_rn(xi[d], sx[d][j]);
+        const float diff = __fsub_rn(xi[d], sx[j][d]);
         // the sum starts at +0 and a square is never -0: the first addition is exact
         dist = d == 0 ? __fmul_rn(diff, diff) : __fadd_rn(dist, __fmul_rn(diff, diff));
       }
@@ -145,7 +166,7 @@ __global__ void __launch_bounds__(kThreads) k_silhouette(int D_any, CoordTable x
 #pragma unroll
       for (int d = 0; d < kDims; ++d)
         if (d < D)
-          sx[d][lane] = next[d];
+          sx[lane][d] = next[d];
       __syncwarp();
       if (k + 32 < k1)
         gather(k + 32);
@@ -205,6 +226,8 @@ clue_status check_map(const clue_points* pts, const int32_t* offsets, const int3
 }
 
 }  // namespace
+
+}  // namespace clue_impl
 
 extern "C" {
 
