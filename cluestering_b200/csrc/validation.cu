@@ -71,14 +71,49 @@ __global__ void __launch_bounds__(kThreads) k_centroids(int D, CoordTable x, con
   }
 }
 
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+
+// The square root of a number from kRootLow up to FLT_MAX: g = x y from the
+// approximate y = 1/sqrt(x), corrected once by the residual x - g^2 of a fused
+// multiply-add (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990): g + (x - g^2) y / 2. On sm_100 each of the
+// floats of the range gives the bits of __fsqrt_rn (all were compared); outside
+// it an infinity, a NaN, a subnormal or a zero gives NaN, and another small
+// number may be a unit in the last place off. The caller tests the range once for
+// many, where __fsqrt_rn does for each.
+constexpr float kRootLow = 0x1p-90f;
+__device__ __forceinline__ float sqrt_in_range(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  const float g = __fmul_rn(x, y);
+  return __fmaf_rn(__fmaf_rn(-g, g, x), __fmul_rn(y, 0.5f), g);
+}
+
 // Silhouettes: a warp holds 32 points, one per lane, and the sums of distances
 // to different clusters do not depend on one another, so the W warps of a group
 // share the same 32 points and take the clusters one by one from the group's
 // counter. A cluster's points pass through shared memory 32 at a time, the next
 // 32 being gathered meanwhile, and every lane adds its distances in the map's
-// order. Bound by the issue of the square roots (about 16 instructions per
-// pair); with one thread per point over all clusters 32,768 points kept 8 warps
-// on each of 128 SMs waiting for their own chains: 4.96 ms, 0.69 ms here.
+// order. Bound by the issue of the distances: four at a time, the differences and
+// squares packed (not their sums: packed products and sums would be contracted),
+// the roots by sqrt_in_range. A tile of 32 that is not full, that holds one of the
+// lanes' own points, or that gives a squared distance out of that range is taken
+// (again) one distance at a time. 32,768 points in 40 clusters: 4.96 ms with one
+// thread per point over all clusters, 0.65 ms with __fsqrt_rn, 0.44 ms now.
 // DD: the number of dimensions, or 0 for any (D at run time).
 template <int DD>
 __global__ void __launch_bounds__(kThreads) k_silhouette(int D_any, CoordTable x, const int32_t* labels,
@@ -88,9 +123,7 @@ __global__ void __launch_bounds__(kThreads) k_silhouette(int D_any, CoordTable x
   constexpr int kDims = DD ? DD : kMaxDim;
   constexpr int kWarps = kThreads / 32;
   const int D = DD ? DD : D_any;
-  // a point's coordinates together, so that a lane reads them with one or two loads
-  constexpr int kRow = DD == 3 ? 4 : kDims;
-  __shared__ __align__(16) float s_x[kWarps][32][kRow];
+  __shared__ __align__(16) float s_x[kWarps][kDims][32];
   __shared__ int32_t s_m[kWarps][32];
   __shared__ float s_a[kWarps][32], s_b[kWarps][32];
   __shared__ int s_next[kWarps];
@@ -107,33 +140,15 @@ __global__ void __launch_bounds__(kThreads) k_silhouette(int D_any, CoordTable x
 #pragma unroll
   for (int d = 0; d < kDims; ++d)
     xi[d] = (valid && d < D) ? x.p[d][i] : 0.0f;
-  float(*sx)[kRow] = s_x[warp];
+  float(*sx)[32] = s_x[warp];
   int32_t* sm = s_m[warp];
   float b = FLT_MAX;
   const auto distance = [&](int j) {
     float dist = 0.0f;
-    if (DD == 2 || DD == 3) {
-      // the first two dimensions with one packed subtract and multiply (sweep_device.cuh)
-      float x, y, z = 0.0f, sx2, sy2;
-      if (DD == 2) {
-        const float2 v = *reinterpret_cast<const float2*>(sx[j]);
-        x = v.x, y = v.y;
-      } else {
-        const float4 v = *reinterpret_cast<const float4*>(sx[j]);
-        x = v.x, y = v.y, z = v.z;
-      }
-      sq_diff_xy(xi[0], xi[kDims > 1 ? 1 : 0], x, y, sx2, sy2);
-      dist = __fadd_rn(sx2, sy2);
-      if (DD == 3) {
-        const float dz = __fsub_rn(xi[kDims - 1], z);
-        dist = __fadd_rn(dist, __fmul_rn(dz, dz));
-      }
-      return __fsqrt_rn(dist);
-    }
 #pragma unroll
     for (int d = 0; d < kDims; ++d)
       if (d < D) {
-        const float diff = __fsub_rn(xi[d], sx[j][d]);
+        const float diff = __fsub_rn(xi[d], sx[d][j]);
         // the sum starts at +0 and a square is never -0: the first addition is exact
         dist = d == 0 ? __fmul_rn(diff, diff) : __fadd_rn(dist, __fmul_rn(diff, diff));
       }
@@ -147,7 +162,6 @@ __global__ void __launch_bounds__(kThreads) k_silhouette(int D_any, CoordTable x
     if (c >= n_clusters)
       break;
     const int k0 = offsets[c], k1 = offsets[c + 1];
-    const bool mine = __any_sync(0xffffffffu, own == c);  // some lane's own point is in c
     float sum = 0.0f, next[kDims];
     int next_m = 0;
     auto gather = [&](int k) {
@@ -166,16 +180,38 @@ __global__ void __launch_bounds__(kThreads) k_silhouette(int D_any, CoordTable x
 #pragma unroll
       for (int d = 0; d < kDims; ++d)
         if (d < D)
-          sx[lane][d] = next[d];
+          sx[d][lane] = next[d];
+      // whether one of the lanes' own points is among these 32
+      const bool mine = __any_sync(0xffffffffu, k + lane < k1 && (next_m >> 5) == (int)(i >> 5));
       __syncwarp();
       if (k + 32 < k1)
         gather(k + 32);
       const int cnt = min(32, k1 - k);
-      if (cnt == 32 && !mine) {
-#pragma unroll 8
-        for (int j = 0; j < 32; ++j)
-          sum = __fadd_rn(sum, distance(j));
-      } else {
+      const float before = sum;
+      float least = FLT_MAX;
+      const bool whole = cnt == 32 && !mine;
+      if (whole) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          float2 a, e;
+#pragma unroll
+          for (int d = 0; d < kDims; ++d)
+            if (d < D) {
+              const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(&sx[d][j]);
+              const unsigned long long own_x = pack2(xi[d], xi[d]);
+              const unsigned long long dl = sub2(own_x, v.x), dh = sub2(own_x, v.y);
+              const float2 sl = unpack2(mul2(dl, dl)), sh = unpack2(mul2(dh, dh));
+              a = d == 0 ? sl : make_float2(__fadd_rn(a.x, sl.x), __fadd_rn(a.y, sl.y));
+              e = d == 0 ? sh : make_float2(__fadd_rn(e.x, sh.x), __fadd_rn(e.y, sh.y));
+            }
+          least = fminf(fminf(least, fminf(a.x, a.y)), fminf(e.x, e.y));
+          sum = __fadd_rn(__fadd_rn(sum, sqrt_in_range(a.x)), sqrt_in_range(a.y));
+          sum = __fadd_rn(__fadd_rn(sum, sqrt_in_range(e.x)), sqrt_in_range(e.y));
+        }
+      }
+      // not (whole and in range): a zero or an infinity gave NaN
+      if (!whole || !(least >= kRootLow) || sum != sum) {
+        sum = before;
         for (int j = 0; j < cnt; ++j) {
           const float dist = distance(j);
           if (sm[j] != (int)i)

@@ -151,3 +151,36 @@ def test_device_scores_of_given_clusters(ndim, sizes):
     for weighted in (False, True) if k else ():
         cen = clue.cluster_centroids(pts, Given(), weighted=weighted)
         assert np.array_equal(cen.view(np.int32), O.centroids(c, w, lab, k, weighted=weighted).view(np.int32))
+
+
+# Tiles of 32 whose distances leave the range of the short square root: points that
+# coincide (in one cluster and across clusters), squared distances below the
+# smallest it takes, subnormal ones and ones that overflow, in whole tiles and ragged.
+@pytest.mark.gpu
+@pytest.mark.parametrize("ndim", [1, 2, 3, 5])
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -46, 2.0 ** -60, 2.0 ** -74, 2.0 ** 62, 2.0 ** 64])
+def test_device_silhouettes_at_the_ends_of_the_range(ndim, scale):
+    import torch
+    rng = np.random.default_rng(17 + ndim)
+    lab = np.repeat(np.arange(5, dtype=np.int32), [96, 70, 64, 33, 200])
+    c = (rng.normal(0.0, 1.0, (ndim, lab.size)) + 3.0 * lab).astype(np.float32)
+    c[:, 96:166] = c[:, :70]  # two clusters at the same places
+    c[:, 230:263] = c[:, 230:231]  # one cluster at one place
+    c = (c * np.float32(scale)).astype(np.float32)
+    order = rng.permutation(lab.size)
+    lab, c = lab[order], np.ascontiguousarray(c[:, order])
+    dev = torch.device("cuda", 0)
+    pts = clue.PointsDevice(torch.from_numpy(c).to(dev), torch.ones(lab.size, device=dev))
+    pts.cluster_index = torch.from_numpy(lab).to(dev)
+    offsets, members = clue.api.clusters_csr(lab)
+
+    class Given:
+        def getClustersDevice(self, stream=None):  # noqa: N802
+            return torch.from_numpy(offsets).to(dev), torch.from_numpy(members).to(dev)
+
+    pts.clustered = True
+    got = clue.silhouette_scores(pts, Given())
+    ref = O.silhouette(c, lab, 5)
+    assert np.array_equal(np.isnan(got), np.isnan(ref))
+    keep = ~np.isnan(ref)
+    assert np.array_equal(got[keep].view(np.int32), ref[keep].view(np.int32))
