@@ -1205,13 +1205,24 @@ __global__ void __launch_bounds__(kCellWarps * 32, D == 2 ? 6 : 4) k_cells(const
 // k_cells goes through ten dependent passes over global memory. Tiles of more than
 // kTilePoints points go through their scratch arrays instead. k_cells took 25 us of a
 // 1,024-point event, 23 us of 16,384 points and 16 us of 10,000 3-D hits (a block per
-// tile of more than 32 points), 14, 10 and 8 us this way.
+// tile of more than 32 points), 7, 7 and 6 us this way.
+// The members' boxes of up to kBoxSlots cells grow by shared-memory atomics, on integers
+// in the order of the floats, while the points are counted: one thread per cell
+// going through the members took 14 us instead of 7 where 1,024 points crowd a few
+// cells. Tiles of more cells still do.
+constexpr int kBoxSlots = 1024;
+__device__ __forceinline__ int ordered_int(float x) {
+  const int b = __float_as_int(x);
+  return b ^ ((b >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float ordered_float(int b) { return __int_as_float(b ^ ((b >> 31) & 0x7fffffff)); }
 constexpr int kTileRounds = 8;
 constexpr int kTilePoints = kTileRounds * kThreads;
 template <int D>
 __global__ void __launch_bounds__(kThreads) k_cells_tile(const RunParams p, const SweepArgs a) {
   __shared__ int s_cnt[kCellSlots + 1];
   __shared__ int s_warp[kThreads / 32];
+  __shared__ int s_box[2 * D][kBoxSlots];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int64_t t = blockIdx.x; t < a.n_tiles; t += gridDim.x) {
     const int begin = a.tile_offset[t];
@@ -1252,9 +1263,18 @@ __global__ void __launch_bounds__(kThreads) k_cells_tile(const RunParams p, cons
       c = c * s + cell_coord(r.y, lo[1], inv[1], s);
       return D == 2 ? c : c * s + cell_coord(r.z, lo[D - 1], inv[D - 1], s);
     };
-    __syncthreads();  // the previous tile's counters have been read
-    for (int c = tid; c < S; c += kThreads)
+    __syncthreads();  // the previous tile's counters and boxes have been read
+    const bool boxed = kept && S <= kBoxSlots;
+    for (int c = tid; c < S; c += kThreads) {
       s_cnt[c] = 0;
+      if (boxed) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          s_box[d][c] = ordered_int(INFINITY);
+          s_box[D + d][c] = ordered_int(-INFINITY);
+        }
+      }
+    }
     __syncthreads();
     int cell[kTileRounds], rank[kTileRounds];
     if (kept) {
@@ -1263,6 +1283,14 @@ __global__ void __launch_bounds__(kThreads) k_cells_tile(const RunParams p, cons
         if (tid + k * kThreads < m) {
           cell[k] = cell_of(rec[k]);
           rank[k] = atomicAdd(&s_cnt[cell[k]], 1);
+          const float x[3] = {rec[k].x, rec[k].y, D == 3 ? rec[k].z : 0.0f};
+          if (boxed && x[0] == x[0] && x[1] == x[1] && x[2] == x[2]) {  // as in tile_cells
+#pragma unroll
+            for (int d = 0; d < D; ++d) {
+              atomicMin(&s_box[d][cell[k]], ordered_int(x[d]));
+              atomicMax(&s_box[D + d][cell[k]], ordered_int(x[d]));
+            }
+          }
         }
     } else {
       for (int i = tid; i < m; i += kThreads) {
@@ -1325,7 +1353,8 @@ __global__ void __launch_bounds__(kThreads) k_cells_tile(const RunParams p, cons
         a.rec_cell[pos] = a.rec_dens[q];
       }
     }
-    __syncthreads();
+    if (!boxed)
+      __syncthreads();  // the records in layout order are read below
     // Member ranges and boxes, as in tile_cells.
     for (int c = tid; c < S; c += kThreads) {
       CellInfo ci;
@@ -1339,7 +1368,13 @@ __global__ void __launch_bounds__(kThreads) k_cells_tile(const RunParams p, cons
         mn[d] = INFINITY;
         mx[d] = -INFINITY;
       }
-      for (int q = ci.start; q < ci.end; ++q) {
+#pragma unroll
+      for (int d = 0; d < D; ++d)
+        if (boxed) {
+          mn[d] = ordered_float(s_box[d][c]);
+          mx[d] = ordered_float(s_box[D + d][c]);
+        }
+      for (int q = boxed ? ci.end : ci.start; q < ci.end; ++q) {
         const float4 r = a.rec_cell[q];
         const float x[3] = {r.x, r.y, D == 3 ? r.z : 0.0f};
         if (x[0] == x[0] && x[1] == x[1] && x[2] == x[2]) {

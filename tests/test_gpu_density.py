@@ -84,3 +84,22 @@ def test_points_on_a_line_and_coincident_points(kernel, params, weights):
     check(c, w, 0.3, 3.0, 0.5, kernel=kernel, kernel_params=params, path="device")
     c = np.repeat(rng.uniform(0.0, 5.0, (2, 12)), n // 12, axis=1).astype(np.float32)
     check(c, w, 0.3, 3.0, 0.5, kernel=kernel, kernel_params=params, path="device")
+
+
+# One block lays out a tile: few cells (boxes grown by atomics), more cells than it keeps
+# boxes for, more points than it keeps; coordinates of both signs, zeros of both signs
+# and all points of a cell at one place.
+@pytest.mark.parametrize("cell_points", [1, 2, 8])
+@pytest.mark.parametrize("n", [3, 1023, 1100, 2047, 2049, 5000])
+@pytest.mark.parametrize("D", [2, 3])
+def test_cell_boxes_of_one_tile(D, n, cell_points):
+    rng = np.random.default_rng(n + D)
+    c = rng.uniform(-4.0, 4.0, (D, n)).astype(np.float32)
+    c[:, rng.random(n) < 0.2] = np.float32(-1.25)
+    c[0, ::7] = np.float32(0.0)
+    c[1, ::11] = np.float32(-0.0)
+    w = rng.exponential(1.0, n).astype(np.float32)
+    clusterer = clue.Clusterer(0.3, 2.0, 0.9, points_per_tile=2 * n)
+    clusterer.set_tuning(cell_points=cell_points)
+    g = run_gpu(c, w, 0.3, 2.0, 0.9, path="device", clusterer=clusterer)
+    assert_identical(g, O.make_clusters(c, w, 0.3, 2.0, 0.9, points_per_tile=2 * n, exp_mode=O.EXP_CLUE, n_threads=8))
