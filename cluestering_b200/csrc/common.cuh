@@ -343,7 +343,6 @@ enum : uint32_t {
   kStatusScanTimeout = 1u << 0,
   kStatusSortOverflow = 1u << 1,
   kStatusLabelTimeout = 1u << 2,
-  kStatusCopyTimeout = 1u << 3,
   kStatusLabelRange = 1u << 4,  // a nearest-higher chain left its event
 };
 

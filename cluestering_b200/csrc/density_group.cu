@@ -61,7 +61,6 @@ struct NearGroup {
 template <int D, int KIND, bool NORMAL, int G, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) k_density_group(const RunParams p, const SweepArgs a) {
   constexpr int P = 32 / G;  // points of a warp at a time
-  constexpr unsigned kGroup = G == 32 ? kFullMask : (1u << G) - 1u;
   constexpr int kBits = NearGroup<G>::kBits;
   extern __shared__ __align__(16) unsigned char s_dyn[];
   const int64_t n = a.n;

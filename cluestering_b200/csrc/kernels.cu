@@ -13,6 +13,8 @@
 //                   index order gets cluster id k), roots by pointer jumping
 //                   (per event in shared memory when every event has its own
 //                   grid and at most 65,536 points; else over the whole run).
+// A single event of at most 65,536 points and 2,560 tiles takes everything before
+// the cell layout, and everything after the sweeps, in one launch each (event.cu).
 #include <atomic>
 #include <cfloat>
 #include <cuda/atomic>

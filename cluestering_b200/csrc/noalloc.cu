@@ -1,6 +1,7 @@
 // noalloc.cu — clue_make_clusters_device_noalloc: the single-event run with
 // every scratch buffer carved from one file-scope device array instead of a
-// workspace allocation. The launch sequence is the library's usual one.
+// workspace allocation. The launch sequence is the library's usual one (event.cu
+// before and after the sweeps, where the device takes its clusters).
 
 #include "abi_internal.h"
 

@@ -24,11 +24,6 @@ namespace clue_impl {
 
 namespace {
 
-int grid_for(int64_t n) {
-  const int64_t b = (n + kThreads - 1) / kThreads;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(b, (int64_t)sm_count() * 16));
-}
-
 // ---------------------------------------------------------------------------
 // Work order: within each tile, points grouped by search-box class
 // ---------------------------------------------------------------------------

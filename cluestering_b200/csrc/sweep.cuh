@@ -28,8 +28,8 @@ struct SweepArgs {
   int32_t* cls_dens;  // scratch: box class per sorted position
   int32_t* cls_nh;
   // Work queues of the fast-path sweeps: [0] density, [1] nearest higher;
-  // each counts the 32-point work items taken so far (k_gather resets
-  // both), so warps that finish early take the next item.
+  // each counts the points or work items taken so far (k_gather, or the front of
+  // a single event, resets both), so warps that finish early take the next.
   int32_t* queue;
   // Tiles of more than 256 points (listed by the binning or the tile sort) and
   // their count: k_cells gives each of them a whole block.

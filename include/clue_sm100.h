@@ -155,15 +155,15 @@ clue_status clue_workspace_stage_ms(clue_workspace* ws, float* stage_ms, int32_t
  * tests (one point tested against one candidate record), [1] density work
  * items of 32 points, [2] nearest-higher candidate members tested, [3] cells
  * checked by the nearest-higher search, [4] cells whose members it tested.
- * The nearest-higher counters cover the cell search (2-D and 3-D Euclidean runs
- * without user tags); other paths leave them at 0. Waits for the run. */
+ * The nearest-higher counters cover the cell search (2-D and 3-D Euclidean
+ * runs); other paths leave them at 0. Waits for the run. */
 #define CLUE_N_SWEEP_STATS 5
 clue_status clue_workspace_sweep_stats(clue_workspace* ws, int64_t* stats, int32_t capacity);
 /* CUDA-graph replay (off by default; no reference counterpart). When on, a
  * device run on a non-default stream (without stage timing) is captured into a
  * CUDA graph, and a later run with identical arguments — the same pointers,
  * event sizes, parameters, grid mode and tuning — replays it: no host-side
- * table building and one graph launch instead of ~20 kernel launches. The
+ * table building and one graph launch instead of 5 to ~20 kernel launches. The
  * inputs' contents may change between replays. Any other run replaces the
  * graph. Turning it off releases the graph. */
 clue_status clue_workspace_set_graphs(clue_workspace* ws, int32_t enable);
@@ -207,18 +207,20 @@ typedef struct {
    * default 2). The tile grid itself stays the reference's (128 points per
    * tile): it decides the search boxes and the order of the density sums. */
   int32_t cell_points;
-  /* Block shape of the density sweep: 0 = 256 threads with 4 blocks per SM,
-   * 1 = 128 threads with 8, 2 = 256 threads with 3. */
+  /* Block shape of the density sweep of runs above 65,536 points (smaller ones
+   * have one shape): 0 = 256 threads with 4 blocks per SM, 1 = 128 threads with
+   * 8, 2 = 256 threads with 3. */
   int32_t density_shape;
-  /* Block shape of the nearest-higher cell search: 0 = 256 threads with 8
-   * blocks per SM in 2-D (4 in 3-D), 1 = 256 threads with 6, 2 = 128 threads
-   * with 16 in 2-D (8 in 3-D). */
+  /* Block shape of the nearest-higher cell search with one lane per point (2-D
+   * runs above 262,144 points; other runs have one shape): 0 = 256 threads with
+   * 8 blocks per SM, 1 = 256 threads with 6, 2 = 128 threads with 16. */
   int32_t nh_shape;
   /* Tile binning: 0 = counting sort by atomics, then each tile's points put
    * in ascending index; 1 = stable runs (one warp per run of consecutive
    * points, per-event count matrices), used when every event of the run has at
    * most 4,096 tiles (else 0). Both give every tile its points in ascending
-   * index. */
+   * index. A single event of at most 65,536 points and 2,560 tiles is binned in
+   * a stable way of its own whatever this says. */
   int32_t tile_binning;
 } clue_tuning;
 
