@@ -21,6 +21,7 @@
 // 65,536: 131 / 137 / 125, 131,072: 181 / 283 / 260; with the Gaussian kernel 8,192:
 // 406 / 53 / 74, 16,384: 348 / 86 / 86; 3-D showers 1,024: 31 / 12 / 12, 16,384: 121 /
 // 47 / 41, 65,536: 359 / 248 / 229. (8 lanes per point lost to 16 up to 16,384.)
+// (Measured with 7 blocks per SM; 16 lanes in 2-D are 5 to 9 % faster now, see launch.)
 // (The lines between the forms: launch_density_group and kGroupPoints.)
 // The warp stays converged: groups that are done wait for the others, and every
 // shuffle and vote is reached by all 32 lanes.
@@ -349,7 +350,11 @@ cudaError_t launch(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   constexpr int NT = 128;
   constexpr int smem = (int)sizeof(NearGroup<G>) * (NT / G);
   const int64_t blocks = (a.n * G + NT - 1) / NT;
-  const auto kernel = k_density_group<D, KIND, NORMAL, G, NT, 7>;
+  // Blocks per SM: in 2-D 9 (56 registers) took 39 and 90 us of 16,384 and 50,021
+  // points against 41 and 99 with 7, and 44 and 100 with 10, which spills; in 3-D 7
+  // took 27 us of 10,000 points and 225 of 65,536 against 33 and 252 with 9.
+  constexpr int kMinBlocks = D == 2 ? 9 : 7;
+  const auto kernel = k_density_group<D, KIND, NORMAL, G, NT, kMinBlocks>;
   kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)sm_count() * 16)), NT, smem, st>>>(p, a);
   count_launches(1);
   return cudaGetLastError();
