@@ -351,7 +351,7 @@ cudaError_t launch(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   constexpr int smem = (int)sizeof(NearGroup<G>) * (NT / G);
   const int64_t blocks = (a.n * G + NT - 1) / NT;
   // Blocks per SM: in 2-D 9 (56 registers) took 39 and 90 us of 16,384 and 50,021
-  // points against 41 and 99 with 7, and 44 and 100 with 10, which spills; in 3-D 7
+  // points against 41 and 99 with 7, and 44 and 100 with 10; in 3-D 7
   // took 27 us of 10,000 points and 225 of 65,536 against 33 and 252 with 9.
   constexpr int kMinBlocks = D == 2 ? 9 : 7;
   const auto kernel = k_density_group<D, KIND, NORMAL, G, NT, kMinBlocks>;

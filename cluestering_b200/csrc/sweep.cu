@@ -1442,8 +1442,7 @@ __device__ __forceinline__ void visit_cell(const SweepArgs& a, int slot, const f
 // The search is bound by the latency of its dependent loads (cell info, box,
 // members), so the 2-D form trades registers for resident warps: 8 blocks of
 // 256 threads per SM measured 8.3 ms on the 46.5 M-point batch against 9.4 ms
-// at 5 and 10.8 ms at 4, small spills included. The 3-D form, with more state
-// per lane, stays at 4.
+// at 5 and 10.8 ms at 4, small spills included.
 // STATS: the profiling instantiation, which also counts the candidates tested
 // (SweepArgs::stats); the counters cost registers, so timed runs go without.
 template <int D, int NT, int MINB, bool TAGS, bool STATS>
@@ -1997,7 +1996,10 @@ int nh_lanes(int D, int64_t n) {
 
 template <int D, bool TAGS, bool STATS>
 void launch_nh_group(const RunParams& p, const SweepArgs& a, int G, cudaStream_t st) {
-  constexpr int kMinBlocks = D == 2 ? 5 : 4;
+  // Blocks per SM that the registers leave room for, us: 2-D 3 / 4 / 5 / 6: 51 / 54 / 57 /
+  // 60 at 50,021 points, 212 / 189 / 198 / 203 at 262,144; 3-D 4 / 5 / 6: 252 / 246 /
+  // 242 at 262,144 hits, 67 / 66 / 68 at 65,536.
+  constexpr int kMinBlocks = D == 2 ? 4 : 5;
   const int blocks = sweep_grid(a.n * G, 256, 16);
   if (G == 32)
     k_nearest_higher_group<D, 32, 256, kMinBlocks, TAGS, STATS><<<blocks, 256, 0, st>>>(p, a);
