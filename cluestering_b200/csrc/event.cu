@@ -407,7 +407,9 @@ __global__ void __launch_bounds__(kBlock, 1) k_event_front(const RunParams p, co
 }
 
 // Cluster -> points map (utils/detail/get_clusters.hpp:24-49): a stable counting
-// sort of the points by label, outliers (-1) left out. One launch for the nine
+// sort of the points by label. Outliers (-1) are left out, and so is any label that is
+// not below n_clusters: the labels are the caller's memory, which may have been written
+// since the run, and here they index shared memory. One launch for the nine
 // of the general form (histogram, scan, scatter and the ordering of each
 // cluster's ids): 45 -> 7 us for 32,768 points in 40 clusters.
 __global__ void __launch_bounds__(kBlock, 1) k_event_map(int n, const int32_t* labels, int n_clusters,
@@ -424,7 +426,8 @@ __global__ void __launch_bounds__(kBlock, 1) k_event_map(int n, const int32_t* l
 #pragma unroll
   for (int k = 0; k < kRounds; ++k) {
     const int i = begin + k * 32 + lane;
-    label[k] = i < end ? labels[i] : -1;
+    const int l = i < end ? labels[i] : -1;
+    label[k] = (unsigned)l < (unsigned)n_clusters ? l : -1;
   }
   sort.clear();
   __syncthreads();

@@ -685,14 +685,14 @@ __global__ void __launch_bounds__(kThreads) k_scan(const int32_t* in, int32_t* o
 // Scatter and per-tile ordering
 // ---------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(kThreads) k_scatter(const int32_t* tile_of, int64_t n,
+__global__ void __launch_bounds__(kThreads) k_scatter(const int32_t* keys, int64_t n, int32_t n_keys,
                                                       int32_t* cursor, int32_t* perm) {
   const int lane = threadIdx.x & 31;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n;
        base += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = base + threadIdx.x;
-    const int t = i < n ? tile_of[i] : -1;
-    const bool valid = t >= 0;  // negative keys (outliers) are not placed
+    const int t = i < n ? keys[i] : -1;
+    const bool valid = (unsigned)t < (unsigned)n_keys;  // others (outliers) are not placed
     const unsigned mask = __match_any_sync(kFull, t);
     const int leader = __ffs(mask) - 1;
     int pos = 0;
@@ -704,15 +704,15 @@ __global__ void __launch_bounds__(kThreads) k_scatter(const int32_t* tile_of, in
   }
 }
 
-// Histogram of non-negative keys (warp-aggregated atomics).
-__global__ void __launch_bounds__(kThreads) k_hist(const int32_t* keys, int64_t n, int32_t* count) {
+// Histogram of the keys in [0, n_keys) (warp-aggregated atomics).
+__global__ void __launch_bounds__(kThreads) k_hist(const int32_t* keys, int64_t n, int32_t n_keys, int32_t* count) {
   const int lane = threadIdx.x & 31;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n;
        base += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = base + threadIdx.x;
     const int t = i < n ? keys[i] : -1;
     const unsigned mask = __match_any_sync(kFull, t);
-    if (t >= 0 && lane == __ffs(mask) - 1)
+    if ((unsigned)t < (unsigned)n_keys && lane == __ffs(mask) - 1)
       atomicAdd(&count[t], __popc(mask));
   }
 }
@@ -1387,7 +1387,8 @@ cudaError_t launch_wait_probe(unsigned long long* desc, uint32_t* status, cudaSt
 // utils/detail/get_clusters.hpp:24-49 on the device: cluster -> points as CSR,
 // point ids ascending within a cluster (the order the reference's serial
 // make_associator produces). The same stable counting sort as the tile
-// binning, keyed by cluster id; outliers (-1) are left out.
+// binning, keyed by cluster id; outliers (-1) and labels of no cluster of the run
+// are left out.
 cudaError_t launch_clusters_csr(const DeviceBuffers& b, int64_t n, const int32_t* labels,
                                 int32_t n_clusters, int32_t* offsets, int32_t* points,
                                 cudaStream_t st) {
@@ -1400,7 +1401,7 @@ cudaError_t launch_clusters_csr(const DeviceBuffers& b, int64_t n, const int32_t
     return launch_event_map(n, labels, n_clusters, offsets, points, st);
   if ((e = cudaMemsetAsync(count, 0, sizeof(int32_t) * n_clusters, st)))
     return e;
-  k_hist<<<grid_for(n), kThreads, 0, st>>>(labels, n, count);
+  k_hist<<<grid_for(n), kThreads, 0, st>>>(labels, n, n_clusters, count);
   count_launches(1);
   if ((e = cudaGetLastError()))
     return e;
@@ -1408,7 +1409,7 @@ cudaError_t launch_clusters_csr(const DeviceBuffers& b, int64_t n, const int32_t
     return e;
   if ((e = cudaMemcpyAsync(cursor, offsets, sizeof(int32_t) * n_clusters, cudaMemcpyDeviceToDevice, st)))
     return e;
-  k_scatter<<<grid_for(n), kThreads, 0, st>>>(labels, n, cursor, points);
+  k_scatter<<<grid_for(n), kThreads, 0, st>>>(labels, n, n_clusters, cursor, points);
   count_launches(1);
   if ((e = cudaGetLastError()))
     return e;
@@ -1497,7 +1498,7 @@ static cudaError_t launch_front(const RunShape& sh, const RunParams& prm, const 
     k_copy32<<<grid_for(sh.n_tiles), kThreads, 0, st>>>((uint32_t*)b.tile_cursor,
                                                        (const uint32_t*)b.tile_offset, sh.n_tiles);
     CLUE_LAUNCHED();
-    k_scatter<<<grid_for(n), kThreads, 0, st>>>(b.tile_of, n, b.tile_cursor, b.perm);
+    k_scatter<<<grid_for(n), kThreads, 0, st>>>(b.tile_of, n, (int32_t)sh.n_tiles, b.tile_cursor, b.perm);
     CLUE_LAUNCHED();
     // Exact-sum events need no ascending order within their tiles when nothing
     // else on this run reads it (flat kernel; user tags break ties by it).
