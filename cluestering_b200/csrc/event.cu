@@ -53,6 +53,7 @@ struct FrontArgs {
   float4* rec;  // density records of the fast sweeps, or null
   int32_t* event_exact;  // or null
   int32_t* counters;
+  int32_t* large_count;  // tiles of more than kLargeTilePoints points (any_form), or null
 };
 
 __device__ __forceinline__ unsigned lanemask_lt() {
@@ -137,7 +138,7 @@ struct ClusterSort {
     }
   }
   // Bases of this block's elements, from the totals of every block, and the
-  // first position of every key, which block 0 hands to emit(key, first).
+  // first position of every key, which block 0 hands to emit(key, first, elements).
   // Returns the number of elements. The others' shared memory has been read
   // when it returns.
   template <typename Emit>
@@ -170,7 +171,7 @@ struct ClusterSort {
       if (k0 + j < k1) {
         base[k0 + j] += block_first;
         if (rank == 0)
-          emit(k0 + j, first);
+          emit(k0 + j, first, counts[j]);
         first += counts[j];
       }
     return total;
@@ -219,6 +220,8 @@ __global__ void __launch_bounds__(kBlock, 1) k_event_front(const RunParams p, co
     s_sum[threadIdx.x] = threadIdx.x == 0 ? INT_MAX : 0;
   if (threadIdx.x == 0)
     sg = a.grid;
+  if (a.large_count && rank == 0 && threadIdx.x == 0)
+    *a.large_count = 0;
   float x[kRounds][DD ? DD : 1], w[kRounds];
 #pragma unroll
   for (int k = 0; k < kRounds; ++k) {
@@ -359,7 +362,11 @@ __global__ void __launch_bounds__(kBlock, 1) k_event_front(const RunParams p, co
     }
     a.counters[4] = a.counters[5] = 0;  // the sweeps' work queues
   }
-  sort.bases(cluster, T, s_warp, [&](int t, int first) { a.tile_offset[t] = first; });
+  sort.bases(cluster, T, s_warp, [&](int t, int first, int count) {
+    a.tile_offset[t] = first;
+    if (a.large_count && count > kLargeTilePoints)
+      atomicAdd(a.large_count, 1);
+  });
   // the others' shared memory has been read: after the matching wait at the
   // end every block may exit
   __syncwarp();
@@ -438,7 +445,7 @@ __global__ void __launch_bounds__(kBlock, 1) k_event_map(int n, const int32_t* l
   __syncthreads();
   sort.block_prefix(n_clusters);
   cluster.sync();
-  const int total = sort.bases(cluster, n_clusters, s_warp, [&](int c, int first) { offsets[c] = first; });
+  const int total = sort.bases(cluster, n_clusters, s_warp, [&](int c, int first, int) { offsets[c] = first; });
   __syncwarp();
   cluster.barrier_arrive();
   __syncthreads();
@@ -673,6 +680,7 @@ cudaError_t launch_event_front(const RunShape& sh, const RunParams& prm, const R
   a.rec = sweep_fast_path(prm) ? b.rec_dens : nullptr;
   a.event_exact = sh.D == 2 || sh.D == 3 ? b.event_exact : nullptr;
   a.counters = b.counters;
+  a.large_count = sweep_fast_path(prm) ? nullptr : b.counters + 3;
   const auto kernel = sh.D == 2 ? k_event_front<2> : sh.D == 3 ? k_event_front<3> : k_event_front<0>;
   return launch_cluster(kernel, cluster_blocks(sh.n), ClusterSort::bytes((int)sh.n_tiles), st, prm, a);
 }

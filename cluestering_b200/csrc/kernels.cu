@@ -1545,6 +1545,8 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
   a.queue = b.counters + 4;
   a.large_tiles = b.large_tiles;
   a.large_count = b.counters + 3;
+  a.n_events = sh.n_events;
+  a.max_event_points = sh.max_event_points;
   a.rec_dens = b.rec_dens;
   a.rec_nh = b.rec_nh;
   a.rec_tag = b.rec_tag;
@@ -1576,11 +1578,12 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
     a.cell_box = b.cell_box;
     a.rec_cell = b.rec_cell;
     a.event_exact = b.event_exact;
-    a.n_events = sh.n_events;
     if (sweep_tile_blocks(prm, n, sh.n_tiles))
       a.work_dens = nullptr;
     else
       a.walk = b.cls_nh;  // k_work_order's scratch, which the fast path leaves free
+  } else if (!any_form(D, a).work_order) {
+    a.work_dens = a.work_nh = nullptr;
   }
   CLUE_CHECK(launch_work_order(D, prm, a, st));
   CLUE_MARK(3);

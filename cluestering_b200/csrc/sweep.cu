@@ -1906,7 +1906,7 @@ cudaError_t launch_work_order(int D, const RunParams& p, const SweepArgs& a, cud
   if (a.n == 0)
     return cudaSuccess;
   // On the fast path k_cells writes the density work order.
-  if (!sweep_fast_path(p) && a.n > kAnyPointWarps) {
+  if (!sweep_fast_path(p) && any_form(D, a).work_order) {
     const int blocks = (int)std::min<int64_t>(a.n_tiles, (int64_t)sm_count() * 16);
     CLUE_DISPATCH_D(D, k_work_order, blocks, kThreads, 0, st)
     count_launches(1);

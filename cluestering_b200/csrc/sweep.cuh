@@ -32,7 +32,8 @@ struct SweepArgs {
   // a single event, resets both), so warps that finish early take the next.
   int32_t* queue;
   // Tiles of more than 256 points (listed by the binning or the tile sort) and
-  // their count: k_cells gives each of them a whole block.
+  // their count: k_cells gives each of them a whole block. (The one-cluster form of a
+  // single event only counts them, and only off the fast path: any_form.)
   const int32_t* large_tiles;
   const int32_t* large_count;
   // Exact-sum density (flat kernel): the density records again, in cell-layout
@@ -43,6 +44,7 @@ struct SweepArgs {
   float4* rec_cell;
   int32_t* event_exact;
   int32_t n_events;
+  int32_t max_event_points;
   // Walk order of the cell layout (k_cells): walk[k] is the layout position
   // visited k-th, tile by tile, cells in strips of 4 rows so that consecutive
   // points are spatial neighbours. Orders the density work and the
@@ -101,14 +103,25 @@ cudaError_t launch_density_group(int D, const RunParams& p, const SweepArgs& a, 
 constexpr int64_t kTileBlocks = 4096;
 bool sweep_tile_blocks(const RunParams& p, int64_t n, int64_t n_tiles);
 // The sweeps off the fast path: any number of dimensions, metric, kernel and
-// option (sweep_any.cu).
+// option. Three forms, chosen by any_form (sweep_any.cu): a warp per point
+// (sweep_any_point.cu), a block of 8 warps per 32 points (sweep_any.cu) and a thread
+// per point (sweep_any_thread.cu).
+enum AnyWhen { kAnyNever, kAnyAlways, kAnyLargeTiles, kAnyNoLargeTiles };
+struct AnyForm {
+  AnyWhen point = kAnyNever, block = kAnyNever, thread = kAnyNever;
+  bool work_order = false;  // k_work_order runs first
+};
+AnyForm any_form(int D, const SweepArgs& a);
+// Whether a kernel launched for the case `when` has the run: some choices depend on
+// the tiles of more than kLargeTilePoints points, which the host does not know.
+__device__ __forceinline__ bool any_form_runs(const SweepArgs& a, int when) {
+  return when == kAnyAlways || (*a.large_count > 0) == (when == kAnyLargeTiles);
+}
 cudaError_t launch_density_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 cudaError_t launch_nearest_higher_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
-// The same with a warp per point, for runs of at most kAnyPointWarps points
-// (sweep_any_point.cu); these take the points in sorted order, without a work order.
-constexpr int64_t kAnyPointWarps = 1 << 14;
-cudaError_t launch_density_point(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
-cudaError_t launch_nearest_higher_point(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
+cudaError_t launch_sweep_point(bool density, int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
+cudaError_t launch_sweep_thread(bool density, int D, const RunParams& p, const SweepArgs& a, int when,
+                                cudaStream_t st);
 cudaError_t launch_density(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 cudaError_t launch_nearest_higher(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 

@@ -1,6 +1,6 @@
 // sweep_any.cu — local density (core/detail/ClusteringKernels.hpp:29-140) and
 // nearest higher (:142-291) off the fast path: any number of dimensions, metric,
-// kernel and option. (Up to kAnyPointWarps points: sweep_any_point.cu.)
+// kernel and option, and the choice between the three forms they come in (any_form).
 //
 // A block of 8 warps takes 32 points of the work order, lane l of every warp
 // holding the l-th, and passes over those of one tile together. The tiles of the
@@ -12,11 +12,10 @@
 // chain. For the nearest higher each warp keeps its best, and the best of the
 // warps is the answer: the comparisons are a strict order on (distance, density,
 // tag, visiting order).
-// With one thread per point over its whole box, as these kernels had it before, an
-// event of 16,384 or 32,768 points filled 8 warps on each of half the SMs, all
+// With one thread per point over its whole box (sweep_any_thread.cu) an event of
+// 32,768 points fills 8 warps on each of the SMs, all
 // waiting for their own loads and additions: density and nearest higher took 1.32 +
-// 1.42 ms for 32,768 points in 2-D with the periodic metric and 1.45 + 1.38 ms for
-// 16,384 in 4-D; 0.17 + 0.14 ms and 0.11 + 0.12 ms here.
+// 1.42 ms for 32,768 points in 2-D with the periodic metric, 0.17 + 0.14 ms here.
 #include <cfloat>
 #include <climits>
 
@@ -310,8 +309,11 @@ __device__ __forceinline__ float pair_inner(const RunParams& p, const Item<D>& i
 }
 
 template <int D, int METRIC>
-__global__ void __launch_bounds__(kThreads, D <= 4 ? 3 : 2) k_density_any(const RunParams p, const SweepArgs a) {
+__global__ void __launch_bounds__(kThreads, D <= 4 ? 3 : 2) k_density_any(const RunParams p, const SweepArgs a,
+                                                                             const int when) {
   extern __shared__ __align__(16) unsigned char s_dyn[];
+  if (!any_form_runs(a, when))
+    return;
   DensityStage<D>& sh = *reinterpret_cast<DensityStage<D>*>(s_dyn);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t n_items = (a.n + 31) / 32;
@@ -392,8 +394,11 @@ __global__ void __launch_bounds__(kThreads, D <= 4 ? 3 : 2) k_density_any(const 
 }
 
 template <int D, int METRIC>
-__global__ void __launch_bounds__(kThreads, D <= 4 ? 3 : 2) k_nearest_higher_any(const RunParams p, const SweepArgs a) {
+__global__ void __launch_bounds__(kThreads, D <= 4 ? 3 : 2) k_nearest_higher_any(const RunParams p, const SweepArgs a,
+                                                                                    const int when) {
   extern __shared__ __align__(16) unsigned char s_dyn[];
+  if (!any_form_runs(a, when))
+    return;
   NearestStage<D>& sh = *reinterpret_cast<NearestStage<D>*>(s_dyn);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t n_items = (a.n + 31) / 32;
@@ -498,7 +503,7 @@ __global__ void __launch_bounds__(kThreads, D <= 4 ? 3 : 2) k_nearest_higher_any
 }
 
 template <int D, int METRIC>
-cudaError_t launch_any(bool density, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
+cudaError_t launch_any(bool density, const RunParams& p, const SweepArgs& a, int when, cudaStream_t st) {
   const int64_t items = (a.n + 31) / 32;
   const int blocks = (int)std::min<int64_t>(items, (int64_t)sm_count() * 64);
   // up to 70 KB: above the default 48 KB they need the opt-in, a function
@@ -508,56 +513,103 @@ cudaError_t launch_any(bool density, const RunParams& p, const SweepArgs& a, cud
     const cudaError_t e = cudaFuncSetAttribute(k_density_any<D, METRIC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess)
       return e;
-    k_density_any<D, METRIC><<<blocks, kThreads, smem, st>>>(p, a);
+    k_density_any<D, METRIC><<<blocks, kThreads, smem, st>>>(p, a, when);
   } else {
     constexpr int smem = (int)sizeof(NearestStage<D>);
     const cudaError_t e =
         cudaFuncSetAttribute(k_nearest_higher_any<D, METRIC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess)
       return e;
-    k_nearest_higher_any<D, METRIC><<<blocks, kThreads, smem, st>>>(p, a);
+    k_nearest_higher_any<D, METRIC><<<blocks, kThreads, smem, st>>>(p, a, when);
   }
   count_launches(1);
   return cudaGetLastError();
 }
 
 template <int D>
-cudaError_t launch_dim(bool density, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
+cudaError_t launch_dim(bool density, const RunParams& p, const SweepArgs& a, int when, cudaStream_t st) {
   switch (p.metric_kind) {
-    case CLUE_METRIC_EUCLIDEAN: return launch_any<D, CLUE_METRIC_EUCLIDEAN>(density, p, a, st);
-    case CLUE_METRIC_PERIODIC_EUCLIDEAN: return launch_any<D, CLUE_METRIC_PERIODIC_EUCLIDEAN>(density, p, a, st);
-    default: return launch_any<D, kAnyMetric>(density, p, a, st);
+    case CLUE_METRIC_EUCLIDEAN: return launch_any<D, CLUE_METRIC_EUCLIDEAN>(density, p, a, when, st);
+    case CLUE_METRIC_PERIODIC_EUCLIDEAN: return launch_any<D, CLUE_METRIC_PERIODIC_EUCLIDEAN>(density, p, a, when, st);
+    default: return launch_any<D, kAnyMetric>(density, p, a, when, st);
   }
 }
 
-cudaError_t launch_sweep(bool density, int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
+cudaError_t launch_sweep_block(bool density, int D, const RunParams& p, const SweepArgs& a, int when,
+                               cudaStream_t st) {
   switch (D) {
-    case 1: return launch_dim<1>(density, p, a, st);
-    case 2: return launch_dim<2>(density, p, a, st);
-    case 3: return launch_dim<3>(density, p, a, st);
-    case 4: return launch_dim<4>(density, p, a, st);
-    case 5: return launch_dim<5>(density, p, a, st);
-    case 6: return launch_dim<6>(density, p, a, st);
-    case 7: return launch_dim<7>(density, p, a, st);
-    case 8: return launch_dim<8>(density, p, a, st);
-    case 9: return launch_dim<9>(density, p, a, st);
-    case 10: return launch_dim<10>(density, p, a, st);
+    case 1: return launch_dim<1>(density, p, a, when, st);
+    case 2: return launch_dim<2>(density, p, a, when, st);
+    case 3: return launch_dim<3>(density, p, a, when, st);
+    case 4: return launch_dim<4>(density, p, a, when, st);
+    case 5: return launch_dim<5>(density, p, a, when, st);
+    case 6: return launch_dim<6>(density, p, a, when, st);
+    case 7: return launch_dim<7>(density, p, a, when, st);
+    case 8: return launch_dim<8>(density, p, a, when, st);
+    case 9: return launch_dim<9>(density, p, a, when, st);
+    case 10: return launch_dim<10>(density, p, a, when, st);
     default: return cudaErrorInvalidValue;
   }
 }
 
+cudaError_t launch_forms(bool density, int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
+  const AnyForm f = any_form(D, a);
+  cudaError_t e = cudaSuccess;
+  if (f.point)
+    e = launch_sweep_point(density, D, p, a, st);
+  if (e == cudaSuccess && f.block)
+    e = launch_sweep_block(density, D, p, a, f.block, st);
+  if (e == cudaSuccess && f.thread)
+    e = launch_sweep_thread(density, D, p, a, f.thread, st);
+  return e;
+}
+
 }  // namespace
 
+// The form of a run's sweeps. A thread per point takes as long as its longest chain of
+// candidates, about 0.35 us each, until the points fill the GPU; the other forms take
+// a time that grows with the number of points (a block of 32 points of one tile about
+// 0.75 ns a point and more where a tile holds fewer) and little with the candidates.
+// Few candidates: events of few points. Density + nearest higher, us, thread / warp
+// per point, 16,384 points in events of 16: 22 / 40, 32: 33 / 38, 64: 49 / 42, 256:
+// 174 / 54; thread / block, 32,768 points in events of 64: 49 / 66, 128: 84 / 67;
+// 65,536 in events of 128: 90 / 104, 256: 186 / 141; 131,072 in events of 256: 217 / 250.
+// Tiles of few points: one grid for a batch, 65,536 points in 32 events of 2,048 (4
+// points a tile) 184 / 592, in 4-D 274 / 606; per event, 65,536 in 4-D events of 256 (16
+// points a tile) 172 / 317, of 512 (32) 289 / 300.
+// Beyond 65,536 points it depends on the points: even ones (no tile of more than 256
+// points) of 131,072 in 4-D 1,665 / 2,232 and 262,144 in 1-D 401 / 580; clustered ones
+// 3,546 / 1,153 and 1,852 / 1,612; 1,048,576 clustered ones in 2-D 8,149 / 6,860, in
+// 3-D 8,784 / 7,120, but in 1-D 4,717 / 6,147. So both kernels are launched there, and
+// in smaller runs of sparse tiles, and one of them returns at once (about 4 us).
+AnyForm any_form(int D, const SweepArgs& a) {
+  constexpr int64_t kPointWarps = 1 << 14, kBlocks = 1 << 16;
+  const int64_t most_blocks = D == 1 ? 1 << 18 : 1 << 20;
+  AnyForm f;
+  const int64_t event = std::min<int64_t>(a.n / std::max(1, a.n_events), 512);  // points, at most 512
+  const bool few = a.n > 256 * event, sparse = a.n < 32 * a.n_tiles;
+  if (a.n <= kPointWarps) {
+    (few ? f.thread : f.point) = kAnyAlways;
+    return f;
+  }
+  f.work_order = true;
+  if (a.n <= kBlocks && !few && !sparse) {
+    f.block = kAnyAlways;
+  } else if (a.n <= most_blocks && a.max_event_points > kLargeTilePoints) {
+    f.block = kAnyLargeTiles;
+    f.thread = kAnyNoLargeTiles;
+  } else {  // (no tile can hold more than 256 points, or the points fill the GPU)
+    f.thread = kAnyAlways;
+  }
+  return f;
+}
+
 cudaError_t launch_density_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
-  if (a.n <= kAnyPointWarps)
-    return launch_density_point(D, p, a, st);
-  return launch_sweep(true, D, p, a, st);
+  return launch_forms(true, D, p, a, st);
 }
 
 cudaError_t launch_nearest_higher_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
-  if (a.n <= kAnyPointWarps)
-    return launch_nearest_higher_point(D, p, a, st);
-  return launch_sweep(false, D, p, a, st);
+  return launch_forms(false, D, p, a, st);
 }
 
 }  // namespace clue_impl

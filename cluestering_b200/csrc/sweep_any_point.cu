@@ -1,6 +1,6 @@
 // sweep_any_point.cu — local density (core/detail/ClusteringKernels.hpp:29-140) and
 // nearest higher (:142-291) off the fast path, with a warp per point: runs of at most
-// kAnyPointWarps points.
+// 16,384 points (any_form).
 //
 // The lanes find the tiles of the point's search box, 32 at a time in the reference's
 // order, and test their points 32 at a time in that order. For the density the lanes
@@ -298,7 +298,9 @@ cudaError_t launch_dim(bool density, const RunParams& p, const SweepArgs& a, cud
   }
 }
 
-cudaError_t launch_sweep(bool density, int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
+}  // namespace
+
+cudaError_t launch_sweep_point(bool density, int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   switch (D) {
     case 1: return launch_dim<1>(density, p, a, st);
     case 2: return launch_dim<2>(density, p, a, st);
@@ -312,16 +314,6 @@ cudaError_t launch_sweep(bool density, int D, const RunParams& p, const SweepArg
     case 10: return launch_dim<10>(density, p, a, st);
     default: return cudaErrorInvalidValue;
   }
-}
-
-}  // namespace
-
-cudaError_t launch_density_point(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
-  return launch_sweep(true, D, p, a, st);
-}
-
-cudaError_t launch_nearest_higher_point(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
-  return launch_sweep(false, D, p, a, st);
 }
 
 }  // namespace clue_impl

@@ -86,3 +86,42 @@ def test_lattice_ties_and_equal_tags_in_four_dimensions(n):
     rng = np.random.default_rng(37)
     c = rng.integers(0, 7, (4, n)).astype(np.float32)
     check(c, np.ones(n, np.float32), 1.0, 2.0, 1.5, tags=rng.integers(0, 3, n).astype(np.uint32), path="device")
+
+
+# The three forms and the lines between them: events of few points (a thread per point,
+# in the sorted order up to 16,384 points), tiles of few points (one grid for a batch,
+# many tiles per event), and runs beyond 65,536 points with and without tiles of more
+# than 256, up to and past the form's largest run.
+def _crowded(c, n, share, seed):
+    """The last `share` of n points drawn together into one place."""
+    k = int(n * share)
+    c[:, n - k:] = 10.0 + 0.05 * np.random.default_rng(seed).normal(0.0, 1.0, (c.shape[0], k))
+    return c.astype(np.float32)
+
+
+@pytest.mark.parametrize("D,n,m,mode", [
+    (2, 1600, 5, clue.GRID_PER_EVENT), (4, 16384, 16, clue.GRID_SHARED), (2, 16384, 64, clue.GRID_PER_EVENT),
+    (3, 16385, 63, clue.GRID_PER_EVENT), (2, 32768, 127, clue.GRID_PER_EVENT), (2, 32768, 128, clue.GRID_PER_EVENT),
+    (4, 40000, 200, clue.GRID_PER_EVENT), (2, 20000, 60, clue.GRID_SHARED), (1, 70000, 7000, clue.GRID_PER_EVENT),
+    (3, 131072, 32768, clue.GRID_PER_EVENT)])
+@pytest.mark.parametrize("crowd", [0.0, 0.02])  # none or the tile of the last events holds many points
+def test_lines_between_the_forms(D, n, m, mode, crowd):
+    rng = np.random.default_rng(n + m)
+    c = rng.uniform(0.0, 20.0, (D, n)) * (1.0 if D > 1 else n / 2000.0)
+    c = _crowded(c, n, crowd, n)
+    w = rng.exponential(1.0, n).astype(np.float32)
+    sizes = [m] * (n // m) + ([n % m] if n % m else [])
+    if crowd and m < 1000:  # one larger event at the end
+        k = -(-int(n * crowd) // m)
+        sizes = sizes[:len(sizes) - k] + [sum(sizes[len(sizes) - k:])]
+    check(c, w, 0.4, 2.0, 0.9, metric="manhattan", kernel="exponential", kernel_params=(1.2, 0.7), sizes=sizes,
+          grid_mode=mode, tags=rng.integers(0, 50, n).astype(np.uint32), path="device")
+
+
+@pytest.mark.parametrize("n", [65536, 65537, 1 << 20, (1 << 20) + 1])
+@pytest.mark.parametrize("crowd", [0, 700])
+def test_large_runs_off_the_fast_path(n, crowd):
+    rng = np.random.default_rng(n)
+    c = _crowded(rng.uniform(0.0, n / 100.0, (1, n)), n, crowd / n, 3)
+    w = rng.exponential(1.0, n).astype(np.float32)
+    check(c, w, 0.2, 2.0, 0.4, metric="manhattan", path="device")
