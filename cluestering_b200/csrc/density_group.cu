@@ -22,7 +22,8 @@
 // 406 / 53 / 74, 16,384: 348 / 86 / 86; 3-D showers 1,024: 31 / 12 / 12, 16,384: 121 /
 // 47 / 41, 65,536: 359 / 248 / 229. (8 lanes per point lost to 16 up to 16,384.)
 // (Measured with 7 blocks per SM; 16 lanes in 2-D are 5 to 9 % faster now, see launch.)
-// (The lines between the forms: launch_density_group and kGroupPoints.)
+// Those are blobs and showers of a few hundred candidates per point. Crowded tiles make
+// the lanes lose, so the cell layout estimates both forms (density_by_load, add_load).
 // The warp stays converged: groups that are done wait for the others, and every
 // shuffle and vote is reached by all 32 lanes.
 #include <climits>
@@ -71,6 +72,8 @@ __global__ void __launch_bounds__(NT, MINB) k_density_group(const RunParams p, c
   const float4* __restrict__ rec_cell = a.rec_cell;
   const float R = reach(p.dc2);
   const float R2 = __fmul_ru(R, R);
+  if (G < 32 && density_streams(a))
+    return;
   for (;;) {
     int64_t w0 = 0;
     if (lane == 0)
@@ -375,8 +378,23 @@ cudaError_t launch_kind(const RunParams& p, const SweepArgs& a, cudaStream_t st)
 
 }  // namespace
 
+// From kGroupWide points on a tile can fill several windows of the bitmap, and the flat
+// kernel's ordered sums, which a group adds one hit after another, can lose to 32 points
+// per warp; the smooth kernels, which those evaluate for all their points, can where n x
+// windows is above 46,000. Below, one launch is the better: the second takes 3 us.
+// Density, us, lanes per point / 32 points per warp, 65,536 points: ordered flat sums of
+// 2-D blobs of 800 points 250 / 138, of 6,400 1,645 / 482, of 16,384 9,554 / 1,435, in 3-D
+// of 1,600 344 / 237; Gaussian of 16,384 8,724 / 3,309 and of 6,400 1,602 / 1,950 (lanes
+// taken), in 3-D 8,663 / 1,834; exact sums in 3-D of 6,400 479 / 353, but in 2-D 448 / 469
+// (lanes taken). All points in one cell (an outlier at 10,000 times the extent), whole
+// call: 176 ms / 12.5 ms.
+bool density_by_load(const RunParams& p, int64_t n) {
+  return n > kGroupWide && n <= kGroupPoints &&
+         (p.kernel_kind == CLUE_KERNEL_FLAT || n * ((n + 4095) / 4096) > 46000);
+}
+
 cudaError_t launch_density_group(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
-  const bool wide = a.n <= 8192;
+  const bool wide = a.n <= kGroupWide;
   if (D == 2)
     return wide ? launch_kind<2, 32>(p, a, st) : launch_kind<2, 16>(p, a, st);
   return wide ? launch_kind<3, 32>(p, a, st) : launch_kind<3, 16>(p, a, st);

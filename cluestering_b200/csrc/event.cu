@@ -360,7 +360,8 @@ __global__ void __launch_bounds__(kBlock, 1) k_event_front(const RunParams p, co
       }
       reinterpret_cast<int4*>(a.event_exact)[0] = st;
     }
-    a.counters[4] = a.counters[5] = 0;  // the sweeps' work queues
+    a.counters[4] = a.counters[5] = 0;   // the sweeps' work queues
+    a.counters[9] = a.counters[10] = 0;  // SweepArgs::load
   }
   sort.bases(cluster, T, s_warp, [&](int t, int first, int count) {
     a.tile_offset[t] = first;

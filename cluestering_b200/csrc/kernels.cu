@@ -1024,9 +1024,9 @@ __global__ void __launch_bounds__(kThreads) k_gather(int D, int64_t n, const int
   // The density records of the fast sweeps (rec, D = 2: {x, y, v, w}; D = 3:
   // {x, y, z, v}, v = fl(flat * w) for the flat kernel, ConvolutionalKernel.hpp:
   // 24-27, else w) come from the same loads, and the sweeps' work queues start
-  // empty (queue[0], queue[1]).
-  if (queue && blockIdx.x == 0 && threadIdx.x < 2)
-    queue[threadIdx.x] = 0;
+  // empty (queue[0], queue[1], and SweepArgs::load, queue[5] and queue[6]).
+  if (queue && blockIdx.x == 0 && threadIdx.x < 4)
+    queue[threadIdx.x < 2 ? threadIdx.x : threadIdx.x + 3] = 0;
   auto record = [&](int64_t s, float x0, float x1, float x2, float wt) {
     const float v = flat ? __fmul_rn(flat_p0, wt) : wt;
     rec[s] = D == 2 ? make_float4(x0, x1, v, wt) : make_float4(x0, x1, x2, v);
@@ -1578,6 +1578,8 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
     a.cell_box = b.cell_box;
     a.rec_cell = b.rec_cell;
     a.event_exact = b.event_exact;
+    if (density_by_load(prm, n))
+      a.load = reinterpret_cast<float*>(b.counters + 9);
     if (sweep_tile_blocks(prm, n, sh.n_tiles))
       a.work_dens = nullptr;
     else

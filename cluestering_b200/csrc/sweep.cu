@@ -543,8 +543,15 @@ __device__ bool density_exact(const RunParams& p, const SweepArgs& a, const Even
 // lane reads each record from shared memory. The stream is the box's rows in
 // order, each a contiguous range of sorted positions, i.e. the reference's
 // summation order. Other warps read candidates from global memory.
-template <int D, int KIND, bool NORMAL, int NT, int MINB>
+// BY_LOAD: only if density_streams says so, and in layout order where there is no
+// work order.
+template <int D, int KIND, bool NORMAL, int NT, int MINB, bool BY_LOAD = false>
 __global__ void __launch_bounds__(NT, MINB) k_density_fast(const RunParams p, const SweepArgs a) {
+  if (BY_LOAD) {
+    cudaGridDependencySynchronize();  // (launch_density_by_load)
+    if (!density_streams(a))
+      return;
+  }
   __shared__ __align__(16) float4 s_ring[NT / 32][kRing][kChunk];
   __shared__ int s_off[NT / 32][kMaxStream + 1];
   __shared__ int s_qa[NT / 32][kMaxStream];
@@ -566,7 +573,7 @@ __global__ void __launch_bounds__(NT, MINB) k_density_fast(const RunParams p, co
       break;
     const int64_t w = item * 32 + lane;
     const bool active = w < n;
-    int s = active ? a.work_dens[w] : 0;
+    int s = !active ? 0 : BY_LOAD && !a.work_dens ? a.nh_q[w] : a.work_dens[w];
     // idle lanes shadow lane 0 (the shuffle runs on every lane: a full-mask
     // shuffle that only some lanes reach never completes)
     const int s_lane0 = __shfl_sync(kFullMask, s, 0);
@@ -913,6 +920,37 @@ __device__ __forceinline__ int strip_position(int c, int s) {
   return D == 2 ? p2 : z * s * s + p2;
 }
 
+// Whether an event's tiles count as exact sums in SweepArgs::load.
+__device__ __forceinline__ bool load_exact(const RunParams& p, const SweepArgs& a, int event, int event_n) {
+  return a.load && p.kernel_kind == CLUE_KERNEL_FLAT && event_sums_exact(a.event_exact, event, event_n);
+}
+
+// Adds a tile of m points to the estimated times of the density (SweepArgs::load);
+// `squares` is the sum of the squares of its cells' members. A point is taken to have as
+// many points around it as its tile has on average, and as many candidates as its cell
+// suggests. Lanes per point test candidates one by one, and where sums are ordered once
+// for each window of 4,096 points that their tile meets (6 ps of the whole GPU a test;
+// exact sums 3 ps). With 32 points per warp the longest item bounds the kernel: 30 ns for
+// each record of its box, with the smooth kernels 90 ns and 160 ns for each that is a
+// candidate, with exact sums 60 ns.
+template <int D>
+__device__ __forceinline__ void add_load(const RunParams& p, const SweepArgs& a, const GridDesc& g, bool exact,
+                                         int event_n, int m, const float* inv, float squares) {
+  const float R = reach(p.dc2);
+  float box = (float)m, near = 0.6f * squares / (float)m;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    box *= g.tile[d] > 0.0f ? 1.0f + 2.0f * R / g.tile[d] : 1.0f;
+    near *= 1.0f + 2.0f * R * inv[d];
+  }
+  box = fminf(box, (float)event_n);
+  near = fminf(near, box);
+  const float tests = (float)m * near * (exact ? 1.0f : (float)((m + 4095) / 4096));
+  atomicAdd(&a.load[0], tests * (exact ? 3e-6f : 6e-6f));
+  const float stream = p.kernel_kind == CLUE_KERNEL_FLAT ? (exact ? 0.06f : 0.03f) * box : 0.09f * box + 0.16f * near;
+  atomicMax(reinterpret_cast<int*>(&a.load[1]), __float_as_int(stream));  // positive floats order like ints
+}
+
 // Cell layout of tile t by a group of NT threads (one warp, or the whole block
 // for a large tile): cell of every point, the layout positions (a counting
 // sort by cell inside the tile's range), cell ranges and member boxes, the
@@ -1087,6 +1125,22 @@ __device__ void tile_cells(const RunParams& p, const SweepArgs& a, int64_t t, in
     if (valid)
       a.work_dens[begin + first + __popc(grp & lane_mask_lt())] = a.nh_q[a.walk[begin + i]];
   }
+  if (NT > 32 && a.load) {  // (tiles of up to kLargeTilePoints points weigh little)
+    float* sum = reinterpret_cast<float*>(cnt2);
+    float squares = 0.0f;
+    for (int c = tid; c < S; c += NT) {
+      const float members = (float)((c + 1 < S ? cnt[c] : m) - (c > 0 ? cnt[c - 1] : 0));
+      squares += members * members;
+    }
+    group_sync<NT>();  // the walk positions have been read
+    if (tid == 0)
+      *sum = 0.0f;
+    group_sync<NT>();
+    atomicAdd(sum, squares);
+    group_sync<NT>();
+    if (tid == 0)
+      add_load<D>(p, a, g, load_exact(p, a, a.sevt[begin], ev.n), ev.n, m, inv, *sum);
+  }
 }
 
 // Cell layout of a tile that is one cell (fewer points than two cells' worth) by one
@@ -1214,10 +1268,11 @@ __device__ __forceinline__ float ordered_float(int b) { return __int_as_float(b 
 constexpr int kTileRounds = 8;
 constexpr int kTilePoints = kTileRounds * kThreads;
 template <int D>
-__global__ void __launch_bounds__(kThreads) k_cells_tile(const RunParams p, const SweepArgs a) {
+__global__ void __launch_bounds__(kThreads, 3) k_cells_tile(const RunParams p, const SweepArgs a) {
   __shared__ int s_cnt[kCellSlots + 1];
   __shared__ int s_warp[kThreads / 32];
   __shared__ int s_box[2 * D][kBoxSlots];
+  __shared__ float s_squares[kThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int64_t t = blockIdx.x; t < a.n_tiles; t += gridDim.x) {
     const int begin = a.tile_offset[t];
@@ -1230,7 +1285,9 @@ __global__ void __launch_bounds__(kThreads) k_cells_tile(const RunParams p, cons
     for (int k = 0; k < kTileRounds; ++k)
       if (kept && tid + k * kThreads < m)
         rec[k] = a.rec_dens[begin + tid + k * kThreads];
-    const EventDesc ev = a.events[a.sevt[begin]];
+    const int event = a.sevt[begin];
+    const EventDesc ev = a.events[event];
+    const bool exact = load_exact(p, a, event, ev.n);
     const GridDesc& g = a.grids[ev.grid];
     const int s = cells_per_dim<D>(m, p.cell_points);
     const int S = D == 2 ? s * s : s * s * s;
@@ -1299,11 +1356,20 @@ __global__ void __launch_bounds__(kThreads) k_cells_tile(const RunParams p, cons
     {
       constexpr int kPer = kCellSlots / kThreads;
       int v[kPer], sum = 0;
+      float squares = 0.0f;  // of the members (add_load)
 #pragma unroll
       for (int j = 0; j < kPer; ++j) {
         const int c = tid * kPer + j;
         v[j] = c < S ? s_cnt[c] : 0;
         sum += v[j];
+        squares += (float)v[j] * (float)v[j];
+      }
+      if (a.load) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+          squares += __shfl_xor_sync(kFullMask, squares, o);
+        if (lane == 0)
+          s_squares[warp] = squares;
       }
       int incl = sum;
 #pragma unroll
@@ -1328,6 +1394,12 @@ __global__ void __launch_bounds__(kThreads) k_cells_tile(const RunParams p, cons
       }
       if (tid == 0)
         s_cnt[S] = m;
+      if (a.load && tid == 0) {  // (written before the scan's barrier)
+        squares = 0.0f;
+        for (int w = 0; w < kThreads / 32; ++w)
+          squares += s_squares[w];
+        add_load<D>(p, a, g, exact, ev.n, m, inv, squares);
+      }
     }
     __syncthreads();
     if (kept) {
@@ -1959,23 +2031,40 @@ void launch_density_kind(const RunParams& p, const SweepArgs& a, cudaStream_t st
   }
 }
 
+// Behind k_density_group, which leaves the run to this kernel or has done it all (then
+// every block returns at once): launched early, it waits for that kernel itself.
+template <int D, int KIND, bool NORMAL>
+cudaError_t launch_density_by_load(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(sweep_grid(a.n, 256, 16));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cfg.attrs = &early;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_density_fast<D, KIND, NORMAL, 256, 4, true>, p, a);
+}
+
+template <int D, int KIND>
+cudaError_t launch_density_fast_kind(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
+  constexpr bool kSmooth = KIND != CLUE_KERNEL_FLAT;
+  const bool normal = kSmooth && kernel_value_normal(p);
+  if (a.load)
+    return normal ? launch_density_by_load<D, KIND, kSmooth>(p, a, st) : launch_density_by_load<D, KIND, false>(p, a, st);
+  normal ? launch_density_kind<D, KIND, kSmooth>(p, a, st) : launch_density_kind<D, KIND, false>(p, a, st);
+  return cudaGetLastError();
+}
+
 template <int D>
 cudaError_t launch_density_fast(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   count_launches(1);  // the density kernel below; k_gather wrote its records
   switch (p.kernel_kind) {
-    case CLUE_KERNEL_FLAT:
-      launch_density_kind<D, CLUE_KERNEL_FLAT, false>(p, a, st);
-      break;
-    case CLUE_KERNEL_GAUSSIAN:
-      kernel_value_normal(p) ? launch_density_kind<D, CLUE_KERNEL_GAUSSIAN, true>(p, a, st)
-                             : launch_density_kind<D, CLUE_KERNEL_GAUSSIAN, false>(p, a, st);
-      break;
-    default:
-      kernel_value_normal(p) ? launch_density_kind<D, CLUE_KERNEL_EXPONENTIAL, true>(p, a, st)
-                             : launch_density_kind<D, CLUE_KERNEL_EXPONENTIAL, false>(p, a, st);
-      break;
+    case CLUE_KERNEL_FLAT: return launch_density_fast_kind<D, CLUE_KERNEL_FLAT>(p, a, st);
+    case CLUE_KERNEL_GAUSSIAN: return launch_density_fast_kind<D, CLUE_KERNEL_GAUSSIAN>(p, a, st);
+    default: return launch_density_fast_kind<D, CLUE_KERNEL_EXPONENTIAL>(p, a, st);
   }
-  return cudaGetLastError();
 }
 
 // Lanes per point of the nearest-higher search. One lane per point is the least
@@ -2041,11 +2130,14 @@ void launch_nh(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
 cudaError_t launch_density(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   if (a.n == 0)
     return cudaSuccess;
-  if (sweep_fast_path(p) && a.n <= kGroupPoints)
-    return launch_density_group(D, p, a, st);
-  if (sweep_fast_path(p))
-    return D == 2 ? launch_density_fast<2>(p, a, st) : launch_density_fast<3>(p, a, st);
-  return launch_density_any(D, p, a, st);
+  if (!sweep_fast_path(p))
+    return launch_density_any(D, p, a, st);
+  if (a.n <= kGroupPoints) {
+    const cudaError_t e = launch_density_group(D, p, a, st);
+    if (e != cudaSuccess || !a.load)
+      return e;
+  }
+  return D == 2 ? launch_density_fast<2>(p, a, st) : launch_density_fast<3>(p, a, st);
 }
 
 cudaError_t launch_nearest_higher(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {

@@ -31,6 +31,10 @@ struct SweepArgs {
   // each counts the points or work items taken so far (k_gather, or the front of
   // a single event, resets both), so warps that finish early take the next.
   int32_t* queue;
+  // Estimated times of the density, us, added up by the cell layout from its tiles: [0]
+  // with lanes per point, [1] with 32 points per warp; density_streams compares them.
+  // Null where lanes per point always do (density_by_load).
+  float* load;
   // Tiles of more than 256 points (listed by the binning or the tile sort) and
   // their count: k_cells gives each of them a whole block. (The one-cluster form of a
   // single event only counts them, and only off the fast path: any_form.)
@@ -94,8 +98,14 @@ bool sweep_fast_path(const RunParams& p);
 cudaError_t launch_work_order(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 // The density with 16 or 32 lanes per point, for fast-path runs of at most
 // kGroupPoints points (density_group.cu).
-constexpr int64_t kGroupPoints = 1 << 16;
+constexpr int64_t kGroupPoints = 1 << 16, kGroupWide = 1 << 13;  // 32 lanes up to the latter
 cudaError_t launch_density_group(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
+// Whether such a run may take 32 points per warp all the same (density_streams), and
+// both kernels are launched.
+bool density_by_load(const RunParams& p, int64_t n);
+__device__ __forceinline__ bool density_streams(const SweepArgs& a) {
+  return a.load && a.load[0] > a.load[1] + 50.0f;
+}
 // Runs whose sweeps give every point a group of lanes (n <= kGroupPoints) take the
 // points in layout order, and k_cells_tile lays the cells out with a block per tile;
 // `walk` and `work_dens` are then null. Above kTileBlocks tiles most hold too few

@@ -103,3 +103,40 @@ def test_cell_boxes_of_one_tile(D, n, cell_points):
     clusterer.set_tuning(cell_points=cell_points)
     g = run_gpu(c, w, 0.3, 2.0, 0.9, path="device", clusterer=clusterer)
     assert_identical(g, O.make_clusters(c, w, 0.3, 2.0, 0.9, points_per_tile=2 * n, exp_mode=O.EXP_CLUE, n_threads=8))
+
+
+# Crowded tiles, where the density takes 32 points per warp below 65,537 points too: an
+# outlier that leaves all other points one tile or one cell, and a radius over the whole
+# extent; sizes on both sides of the lines (8,192 points; 12,288 with the smooth kernels),
+# and a batch of as many tiles as k_cells lays out.
+@pytest.mark.parametrize("kernel,params,weights", KERNELS + [("gaussian", (1.0, 1.0), "exponential")])
+@pytest.mark.parametrize("D,n,outlier,r", [(2, 8192, 3e3, 1.2), (2, 8193, 3e5, 1.2), (2, 12288, 3e5, 1.2),
+                                           (3, 12289, 3e4, 1.5), (2, 20011, 3e3, 1.2), (3, 20011, 3e5, 1.5),
+                                           (2, 20011, None, 90.0), (3, 9001, None, 25.0), (2, 65536, 3e5, 1.2)])
+def test_crowded_tiles(D, n, outlier, r, kernel, params, weights):
+    if n == 65536 and kernel != "flat":
+        pytest.skip("the checker's time")
+    c, w = event(D, n, weights, 1600 + D)
+    if outlier:
+        c[:, n // 2] = outlier
+    check(c, w, r, 3.0, r if r < 20.0 else 1.0, kernel=kernel, kernel_params=params, path="device")
+
+
+@pytest.mark.parametrize("weights", ["unit", "exponential"])
+def test_largest_crowded_tile(weights):
+    c, w = event(2, 65536, weights, 1650)
+    c[:, 7] = 3e5
+    check(c, w, 1.2, 3.0, 1.2, path="device")
+
+
+@pytest.mark.parametrize("kernel,params,weights", KERNELS)
+@pytest.mark.parametrize("mode", [clue.GRID_PER_EVENT, clue.GRID_SHARED])
+def test_crowded_tiles_in_a_batch(mode, kernel, params, weights):
+    sizes = [4000, 9000, 300, 12000, 1, 2500]
+    c, w = event(2, sum(sizes), weights, 1700)
+    c[:, 10], c[:, 5000] = 2e4, -2e4
+    g = run_gpu(c, w, 1.2, 3.0, 1.5, kernel=kernel, kernel_params=params, sizes=sizes, grid_mode=mode, path="device",
+                clusterer=clue.Clusterer(1.2, 3.0, 1.5, points_per_tile=96))
+    assert_identical(g, O.make_clusters_batched(c, w, sizes, 1.2, 3.0, 1.5, shared_grid=mode == clue.GRID_SHARED,
+                                                points_per_tile=96, kernel=kernel, kernel_params=params,
+                                                exp_mode=O.EXP_CLUE, n_threads=8))
