@@ -2074,13 +2074,15 @@ cudaError_t launch_density_fast(const RunParams& p, const SweepArgs& a, cudaStre
 // 18 / 16 / 16; 16,384: 84 / 25 / 25 / 35; 65,536: 199 / 59 / 68 / 98; 262,144:
 // 240 / 162 / 201 / 322 (and 115 / 113 with 31 blobs per 16,384 points); 524,288:
 // 364 / 358 (168 / 201). In 3-D, where a point has 27 neighbour cells: 16,384
-// hits 113 / 27 / 27 / 39; 262,144: 378 / 219 / 257 / 404; 524,288: 835 / 512.
+// hits 113 / 27 / 27 / 39; 262,144: 378 / 219 / 257 / 404; 524,288: 835 / 512; blobs and
+// evenly spread points of 524,288: 762 / 617 and 215 / 283, of 1,048,576: 1,259 /
+// 1,197 and 403 / 549, of 2,097,152: 2,278 / 2,377 and 777 / 1,519.
 int nh_lanes(int D, int64_t n) {
   if (n <= 4096)
     return 32;
   if (n <= 16384)
     return 16;
-  return D == 3 || n <= (int64_t)1 << 18 ? 8 : 1;
+  return n <= (int64_t)1 << (D == 3 ? 19 : 18) ? 8 : 1;
 }
 
 template <int D, bool TAGS, bool STATS>
@@ -2099,32 +2101,35 @@ void launch_nh_group(const RunParams& p, const SweepArgs& a, int G, cudaStream_t
 }
 
 // Block shapes of the nearest-higher search with one lane per point
-// (clue_tuning::nh_shape): 0: 256 threads with 8 blocks per SM; 1: 256 threads, 6
-// per SM; 2: 128 threads with 16 blocks per SM. (2-D only: nh_lanes.)
-template <bool TAGS, bool STATS>
+// (clue_tuning::nh_shape): 0: 256 threads with 8 blocks per SM in 2-D, 4 in 3-D; 1: 256
+// threads, 6 per SM; 2: 128 threads with 16 blocks per SM in 2-D, 8 in 3-D.
+template <int D, bool TAGS, bool STATS>
 void launch_nh_cells(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   switch (p.nh_shape) {
     case 1:
-      k_nearest_higher_cells<2, 256, 6, TAGS, STATS><<<sweep_grid(a.n, 256, 16), 256, 0, st>>>(p, a);
+      k_nearest_higher_cells<D, 256, 6, TAGS, STATS><<<sweep_grid(a.n, 256, 16), 256, 0, st>>>(p, a);
       break;
     case 2:
-      k_nearest_higher_cells<2, 128, 16, TAGS, STATS><<<sweep_grid(a.n, 128, 32), 128, 0, st>>>(p, a);
+      k_nearest_higher_cells<D, 128, D == 2 ? 16 : 8, TAGS, STATS><<<sweep_grid(a.n, 128, 32), 128, 0, st>>>(p, a);
       break;
     default:
-      k_nearest_higher_cells<2, 256, 8, TAGS, STATS><<<sweep_grid(a.n, 256, 16), 256, 0, st>>>(p, a);
+      k_nearest_higher_cells<D, 256, D == 2 ? 8 : 4, TAGS, STATS><<<sweep_grid(a.n, 256, 16), 256, 0, st>>>(p, a);
       break;
   }
 }
 
-template <bool TAGS, bool STATS>
-void launch_nh(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
+template <int D, bool TAGS, bool STATS>
+void launch_nh_dim(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
   const int G = nh_lanes(D, a.n);
   if (G == 1)
-    launch_nh_cells<TAGS, STATS>(p, a, st);
-  else if (D == 2)
-    launch_nh_group<2, TAGS, STATS>(p, a, G, st);
+    launch_nh_cells<D, TAGS, STATS>(p, a, st);
   else
-    launch_nh_group<3, TAGS, STATS>(p, a, G, st);
+    launch_nh_group<D, TAGS, STATS>(p, a, G, st);
+}
+
+template <bool TAGS, bool STATS>
+void launch_nh(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {
+  D == 2 ? launch_nh_dim<2, TAGS, STATS>(p, a, st) : launch_nh_dim<3, TAGS, STATS>(p, a, st);
 }
 
 cudaError_t launch_density(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st) {

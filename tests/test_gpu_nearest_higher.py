@@ -43,3 +43,20 @@ def test_search_box_of_many_tiles(D, n):
     w = rng.exponential(1.0, n).astype(np.float32)
     g = run_gpu(c, w, 1.0, 2.0, 2.5, path="device", clusterer=clue.Clusterer(1.0, 2.0, 2.5, points_per_tile=4))
     assert_identical(g, O.make_clusters(c, w, 1.0, 2.0, 2.5, points_per_tile=4, exp_mode=O.EXP_CLUE, n_threads=8))
+
+
+# One lane per point in 3-D, and the largest run with eight, every block shape: ties
+# on a lattice, real weights, with and without tags.
+@pytest.mark.parametrize("tags", [False, True])
+@pytest.mark.parametrize("n,shape", [(524288, 0), (524289, 0), (600001, 1), (600001, 2)])
+def test_large_runs_in_three_dimensions(n, shape, tags):
+    import cluestering_b200 as clue
+    rng = np.random.default_rng(n + shape)
+    c = rng.uniform(0.0, 100.0, (3, n)).astype(np.float32)
+    half = rng.random(n) < 0.5
+    c[:, half] = np.round(c[:, half])
+    w = np.where(half, 1.0, rng.exponential(1.0, n)).astype(np.float32)
+    algo = clue.Clusterer(1.0, 2.0, 1.5)
+    algo.set_tuning(nh_shape=shape)
+    check(c, w, 1.0, 2.0, 1.5, path="device", clusterer=algo,
+          tags=rng.integers(0, 3, n).astype(np.uint32) if tags else None)
