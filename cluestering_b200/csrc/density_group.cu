@@ -388,8 +388,8 @@ cudaError_t launch_kind(const RunParams& p, const SweepArgs& a, cudaStream_t st)
 // taken), in 3-D 8,663 / 1,834; exact sums in 3-D of 6,400 479 / 353, but in 2-D 448 / 469
 // (lanes taken). All points in one cell (an outlier at 10,000 times the extent), whole
 // call: 176 ms / 12.5 ms.
-bool density_by_load(const RunParams& p, int64_t n) {
-  return n > kGroupWide && n <= kGroupPoints &&
+bool density_by_load(const RunParams& p, int64_t n, int32_t n_events) {
+  return sweep_groups(p, n, n_events) && n > kGroupWide &&
          (p.kernel_kind == CLUE_KERNEL_FLAT || n * ((n + 4095) / 4096) > 46000);
 }
 

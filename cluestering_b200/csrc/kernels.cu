@@ -1578,9 +1578,10 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
     a.cell_box = b.cell_box;
     a.rec_cell = b.rec_cell;
     a.event_exact = b.event_exact;
-    if (density_by_load(prm, n))
+    if (density_by_load(prm, n, sh.n_events))
       a.load = reinterpret_cast<float*>(b.counters + 9);
-    if (sweep_tile_blocks(prm, n, sh.n_tiles))
+    a.tile_blocks = sweep_tile_blocks(prm, n, sh.n_tiles, sh.n_events, event);
+    if (a.tile_blocks)
       a.work_dens = nullptr;
     else
       a.walk = b.cls_nh;  // k_work_order's scratch, which the fast path leaves free

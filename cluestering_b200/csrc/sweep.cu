@@ -1955,8 +1955,12 @@ bool sweep_fast_path(const RunParams& p) {
   return true;
 }
 
-bool sweep_tile_blocks(const RunParams& p, int64_t n, int64_t n_tiles) {
-  return sweep_fast_path(p) && n <= kGroupPoints && n_tiles <= kTileBlocks;
+bool sweep_groups(const RunParams& p, int64_t n, int32_t n_events) {
+  return sweep_fast_path(p) && n <= kGroupPoints && n_events <= kGroupEvents;
+}
+
+bool sweep_tile_blocks(const RunParams& p, int64_t n, int64_t n_tiles, int32_t n_events, bool one_cluster) {
+  return sweep_groups(p, n, n_events) && (one_cluster || n_tiles <= kTileBlocks);
 }
 
 #define CLUE_DISPATCH_D(D, KERNEL, ...)                \
@@ -1983,7 +1987,7 @@ cudaError_t launch_work_order(int D, const RunParams& p, const SweepArgs& a, cud
     CLUE_DISPATCH_D(D, k_work_order, blocks, kThreads, 0, st)
     count_launches(1);
   }
-  if (a.nh_pos && sweep_tile_blocks(p, a.n, a.n_tiles)) {
+  if (a.nh_pos && a.tile_blocks) {
     const int blocks = (int)std::min<int64_t>(a.n_tiles, (int64_t)sm_count() * 8);
     if (D == 2)
       k_cells_tile<2><<<blocks, kThreads, 0, st>>>(p, a);
@@ -2077,7 +2081,13 @@ cudaError_t launch_density_fast(const RunParams& p, const SweepArgs& a, cudaStre
 // hits 113 / 27 / 27 / 39; 262,144: 378 / 219 / 257 / 404; 524,288: 835 / 512; blobs and
 // evenly spread points of 524,288: 762 / 617 and 215 / 283, of 1,048,576: 1,259 /
 // 1,197 and 403 / 549, of 2,097,152: 2,278 / 2,377 and 777 / 1,519.
-int nh_lanes(int D, int64_t n) {
+// Small events have few cells to look at: 65,536 points in 2-D events of 16 18 / 43, of
+// 512 35 / 45, of 1,024 39 / 46, 16,384 in events of 128 24 / 28, of 256 32 / 30; 65,536 in
+// 3-D events of 128 32 / 47, of 512 49 / 49; 250,000 in 2-D events of 1,024 54 / 136, of
+// 4,096 65 / 136 (the call 314 / 357), 500,000 in 3-D events of 4,096 169 / 267.
+int nh_lanes(int D, int64_t n, int32_t n_events) {
+  if (n_events > (D == 2 ? 32 : 64) * (n <= kGroupPoints ? 2 : 1))
+    return 1;
   if (n <= 4096)
     return 32;
   if (n <= 16384)
@@ -2120,7 +2130,7 @@ void launch_nh_cells(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
 
 template <int D, bool TAGS, bool STATS>
 void launch_nh_dim(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
-  const int G = nh_lanes(D, a.n);
+  const int G = nh_lanes(D, a.n, a.n_events);
   if (G == 1)
     launch_nh_cells<D, TAGS, STATS>(p, a, st);
   else
@@ -2137,7 +2147,7 @@ cudaError_t launch_density(int D, const RunParams& p, const SweepArgs& a, cudaSt
     return cudaSuccess;
   if (!sweep_fast_path(p))
     return launch_density_any(D, p, a, st);
-  if (a.n <= kGroupPoints) {
+  if (sweep_groups(p, a.n, a.n_events)) {
     const cudaError_t e = launch_density_group(D, p, a, st);
     if (e != cudaSuccess || !a.load)
       return e;

@@ -55,6 +55,7 @@ struct SweepArgs {
   // nearest-higher threads. Null, like work_dens, when the sweeps take the points
   // in layout order (sweep_tile_blocks).
   int32_t* walk;
+  bool tile_blocks;
   // Packed candidate records of the fast path (D = 2 or 3).
   float4* rec_dens;  // {x, y, [z], v}: v = flat * w for the flat kernel, else w
   float4* rec_nh;    // D = 2: {x, y, rho, tag bits}; D = 3: {x, y, z, rho}
@@ -96,22 +97,29 @@ struct SweepArgs {
 bool sweep_fast_path(const RunParams& p);
 
 cudaError_t launch_work_order(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
-// The density with 16 or 32 lanes per point, for fast-path runs of at most
-// kGroupPoints points (density_group.cu).
+// The density with 16 or 32 lanes per point (density_group.cu), for fast-path runs of
+// at most kGroupPoints points in at most kGroupEvents events. Small events have few
+// candidates to share among lanes: density, us, 32 points per warp / lanes, 65,536 points
+// in events of 16 12 / 48, of 256 23 / 49, of 512 29 / 49, of 1,024 40 / 50 (Gaussian 47 / 49
+// at 256, 113 / 54 at 1,024); 16,384 in events of 64 12 / 21, of 256 20 / 21, of 512 24 / 21.
 constexpr int64_t kGroupPoints = 1 << 16, kGroupWide = 1 << 13;  // 32 lanes up to the latter
+constexpr int32_t kGroupEvents = 64;
+bool sweep_groups(const RunParams& p, int64_t n, int32_t n_events);
 cudaError_t launch_density_group(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 // Whether such a run may take 32 points per warp all the same (density_streams), and
 // both kernels are launched.
-bool density_by_load(const RunParams& p, int64_t n);
+bool density_by_load(const RunParams& p, int64_t n, int32_t n_events);
 __device__ __forceinline__ bool density_streams(const SweepArgs& a) {
   return a.load && a.load[0] > a.load[1] + 50.0f;
 }
-// Runs whose sweeps give every point a group of lanes (n <= kGroupPoints) take the
+// Runs whose sweeps give every point a group of lanes (sweep_groups) take the
 // points in layout order, and k_cells_tile lays the cells out with a block per tile;
-// `walk` and `work_dens` are then null. Above kTileBlocks tiles most hold too few
-// points for a block of their own.
-constexpr int64_t kTileBlocks = 4096;
-bool sweep_tile_blocks(const RunParams& p, int64_t n, int64_t n_tiles);
+// `walk` and `work_dens` are then null. Above kTileBlocks tiles (about what the GPU
+// holds at once) most hold too few points for a block of their own: 16,384 points in
+// 2,304 tiles 17 us without, 22 with it; 65,536 in 512 23 and 17. The one-cluster form of
+// a single event (up to 2,560 tiles) always takes it: it leaves no coordinate planes.
+constexpr int64_t kTileBlocks = 1024;
+bool sweep_tile_blocks(const RunParams& p, int64_t n, int64_t n_tiles, int32_t n_events, bool one_cluster);
 // The sweeps off the fast path: any number of dimensions, metric, kernel and
 // option. Three forms, chosen by any_form (sweep_any.cu): a warp per point
 // (sweep_any_point.cu), a block of 8 warps per 32 points (sweep_any.cu) and a thread

@@ -140,3 +140,19 @@ def test_crowded_tiles_in_a_batch(mode, kernel, params, weights):
     assert_identical(g, O.make_clusters_batched(c, w, sizes, 1.2, 3.0, 1.5, shared_grid=mode == clue.GRID_SHARED,
                                                 points_per_tile=96, kernel=kernel, kernel_params=params,
                                                 exp_mode=O.EXP_CLUE, n_threads=8))
+
+
+# Small events: lanes per point up to 64 events (nearest higher 64 in 2-D, 128 in 3-D,
+# half of that above 65,536 points), one lane per point beyond.
+@pytest.mark.parametrize("kernel,params,weights", KERNELS[1:3])
+@pytest.mark.parametrize("D,events,m", [(2, 63, 90), (2, 64, 90), (2, 65, 90), (3, 65, 40), (3, 128, 40), (3, 129, 40),
+                                        (2, 32, 2049), (2, 33, 2049), (3, 64, 1025), (3, 65, 1025)])
+def test_batches_of_small_events(D, events, m, kernel, params, weights):
+    rng = np.random.default_rng(1800 + events)
+    sizes = rng.integers(1, 2 * m, events)
+    sizes[-1] += max(0, m * events - sizes.sum())
+    c = rng.uniform(0.0, 6.0, (D, int(sizes.sum()))).astype(np.float32)
+    w = rng.exponential(1.0, c.shape[1]).astype(np.float32)
+    tags = rng.integers(0, 9, c.shape[1]).astype(np.uint32) if kernel == "flat" else None
+    check(c, w, 0.8, 2.0, 1.1, kernel=kernel, kernel_params=params, sizes=sizes, tags=tags,
+          grid_mode=clue.GRID_PER_EVENT, path="device")
