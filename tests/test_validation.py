@@ -184,3 +184,31 @@ def test_device_silhouettes_at_the_ends_of_the_range(ndim, scale):
     assert np.array_equal(np.isnan(got), np.isnan(ref))
     keep = ~np.isnan(ref)
     assert np.array_equal(got[keep].view(np.int32), ref[keep].view(np.int32))
+
+
+# Both forms of the centroids: a block per cluster below 4,096 clusters, a thread per
+# cluster and dimension from there on; sizes from one point to many rounds of a block.
+@pytest.mark.gpu
+@pytest.mark.parametrize("ndim", [1, 3, 10])
+@pytest.mark.parametrize("k", [4095, 4096, 5000])
+def test_device_centroids_of_many_clusters(ndim, k):
+    import torch
+    rng = np.random.default_rng(85 + k)
+    sizes = rng.integers(1, 6, k)
+    sizes[[0, k // 2, k - 1]] = [257, 256, 700]
+    lab = np.concatenate([np.repeat(np.arange(k), sizes), np.full(17, -1)]).astype(np.int32)
+    lab = lab[rng.permutation(lab.size)]
+    c = rng.normal(0.0, 50.0, (ndim, lab.size)).astype(np.float32)
+    w = rng.exponential(1.0, lab.size).astype(np.float32)
+    dev = torch.device("cuda", 0)
+    pts = clue.PointsDevice(torch.from_numpy(c).to(dev), torch.from_numpy(w).to(dev))
+    offsets, members = clue.api.clusters_csr(lab)
+
+    class Given:
+        def getClustersDevice(self, stream=None):  # noqa: N802
+            return torch.from_numpy(offsets).to(dev), torch.from_numpy(members).to(dev)
+
+    pts.clustered = True
+    for weighted in (False, True):
+        got = clue.cluster_centroids(pts, Given(), weighted=weighted)
+        assert np.array_equal(got.view(np.int32), O.centroids(c, w, lab, k, weighted=weighted).view(np.int32))
