@@ -1440,19 +1440,23 @@ clue_status clue_workspace_autotune(clue_workspace* ws, const clue_params* param
       }
     }
   };
-  // The union threshold, the cell size and the sweeps' block shapes matter on
-  // the packed 2-D/3-D path only.
-  if (points->ndim == 2)
+  // Only choices that this run obeys: another's candidates would all be the same run,
+  // and the fastest of them, by chance, would stay for the runs that do obey it.
+  const TuningUse use = tuning_use(ws->tables.shape, make_run_params(params, points, best));
+  if (use.density && points->ndim == 2)
     try_field(&clue_tuning::density_union_x16_2d, {0, 12, 16, 20, 24, 32, 48, 1 << 20});
-  else if (points->ndim == 3)
+  else if (use.density)
     try_field(&clue_tuning::density_union_x16_3d, {0, 16, 24, 32, 48, 64, 1 << 20});
-  if (points->ndim == 2 || points->ndim == 3) {
+  if (use.cells)
     try_field(&clue_tuning::cell_points, {1, 2, 3, 4});
+  if (use.density)
     try_field(&clue_tuning::density_shape, {0, 1, 2});
+  if (use.nearest)
     try_field(&clue_tuning::nh_shape, {0, 1, 2});
-  }
-  try_field(&clue_tuning::tile_binning, {0, 1});
-  try_field(&clue_tuning::label_jump_rounds, {0, 1, 2, 3, 4});
+  if (use.binning)
+    try_field(&clue_tuning::tile_binning, {0, 1});
+  if (use.labels)
+    try_field(&clue_tuning::label_jump_rounds, {0, 1, 2, 3, 4});
   for (auto& x : ev)
     cudaEventDestroy(x);
   ws->tuning = s == CLUE_OK ? best : start;

@@ -186,6 +186,12 @@ cudaError_t launch_run(const RunShape& shape, const RunParams& prm, const RunIO&
                        const DeviceBuffers& b, cudaStream_t stream,
                        cudaEvent_t* marks = nullptr);
 
+// Which choices of clue_tuning a run of this shape obeys; the others change nothing.
+struct TuningUse {
+  bool density, cells, nearest, binning, labels;
+};
+TuningUse tuning_use(const RunShape& shape, const RunParams& prm);
+
 // The stages of an event_path run before and after the sweeps.
 cudaError_t launch_event_front(const RunShape& shape, const RunParams& prm, const RunIO& io, const GridDesc& grid,
                                const EventDesc& ev, const DeviceBuffers& b, cudaStream_t stream);

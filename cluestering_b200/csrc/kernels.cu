@@ -1518,6 +1518,24 @@ static cudaError_t launch_front(const RunShape& sh, const RunParams& prm, const 
   return cudaSuccess;
 }
 
+// One grid per event keeps every event in its own range of the layout: the chains of
+// followers are then walked per event in shared memory.
+static bool local_labels(const RunShape& sh) {
+  return sh.n_grids == sh.n_events && sh.max_event_points <= kLocalLabelPoints &&
+         local_labels_ready(sh.max_event_points);
+}
+
+TuningUse tuning_use(const RunShape& sh, const RunParams& prm) {
+  const bool fast = sweep_fast_path(prm), event = event_path(sh);
+  TuningUse u;
+  u.density = fast && !sweep_groups(prm, sh.n, sh.n_events);
+  u.cells = fast;
+  u.nearest = fast && nh_lanes(sh.D, sh.n, sh.n_events) == 1;
+  u.binning = !event && sh.stable;
+  u.labels = !event && !local_labels(sh);
+  return u;
+}
+
 cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io,
                        const DeviceBuffers& b, cudaStream_t st, cudaEvent_t* marks) {
   const int D = sh.D;
@@ -1604,11 +1622,7 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
   CLUE_CHECK(scan(b.seed_flag, b.seed_rank, n, b.counters + 1, b, st));
   const bool piece = io.piece_base != nullptr;
   int32_t* nh_shift = piece && io.point_base ? io.nh : nullptr;
-  // One grid per event keeps every event in its own range of the layout: the
-  // chains are walked per event in shared memory.
-  const bool local_labels = sh.n_grids == sh.n_events && sh.max_event_points <= kLocalLabelPoints &&
-                            local_labels_ready(sh.max_event_points);
-  if (local_labels) {
+  if (local_labels(sh)) {
     const size_t smem = ((size_t)std::max(sh.max_event_points, 1) * sizeof(uint16_t) + 15) & ~(size_t)15;
     const int blocks = std::max(1, std::min(sh.n_events, sm_count() * (smem <= (96u << 10) ? 2 : 1)));
     CLUE_CHECK(fill32(b.counters + 6, 1, 0, st));

@@ -120,6 +120,8 @@ __device__ __forceinline__ bool density_streams(const SweepArgs& a) {
 // a single event (up to 2,560 tiles) always takes it: it leaves no coordinate planes.
 constexpr int64_t kTileBlocks = 1024;
 bool sweep_tile_blocks(const RunParams& p, int64_t n, int64_t n_tiles, int32_t n_events, bool one_cluster);
+// Lanes per point of the nearest-higher search on the fast path.
+int nh_lanes(int D, int64_t n, int32_t n_events);
 // The sweeps off the fast path: any number of dimensions, metric, kernel and
 // option. Three forms, chosen by any_form (sweep_any.cu): a warp per point
 // (sweep_any_point.cu), a block of 8 warps per 32 points (sweep_any.cu) and a thread

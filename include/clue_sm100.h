@@ -190,7 +190,8 @@ clue_status clue_workspace_kernel_launches(const clue_workspace* ws, int64_t* la
  * division is fixed at compile time). None of these choices changes a result:
  * they decide only how the work is spread over the GPU. ------------------- */
 typedef struct {
-  /* Density sweep, 2-D and 3-D Euclidean runs: a warp whose 32 points have
+  /* Density sweep, 2-D and 3-D Euclidean runs above 65,536 points or of more
+   * than 64 events (and smaller ones with crowded tiles): a warp whose 32 points have
    * different search boxes streams the union of their boxes through shared
    * memory when the union holds at most (threshold / 16) times the
    * candidates of the warp's largest own box; otherwise each point reads its
@@ -200,19 +201,21 @@ typedef struct {
   int32_t density_union_x16_3d;
   /* Labels: whole-array pointer-jumping rounds over the follower tree before
    * each point walks to its seed (0..4); -1 picks by size (none below 2^18
-   * points, 2 below 2^22, else 3). */
+   * points, 2 below 2^22, else 3). Runs with one grid per event and at most 65,536
+   * points in each take their chains event by event and ignore it. */
   int32_t label_jump_rounds;
   /* Sweeps of 2-D and 3-D Euclidean runs: average points per cell of the cell
    * layout that orders and prunes the candidates inside each tile (1..8;
    * default 2). The tile grid itself stays the reference's (128 points per
    * tile): it decides the search boxes and the order of the density sums. */
   int32_t cell_points;
-  /* Block shape of the density sweep of runs above 65,536 points (smaller ones
-   * have one shape): 0 = 256 threads with 4 blocks per SM, 1 = 128 threads with
+  /* Block shape of the density sweep of runs above 65,536 points or of more than
+   * 64 events (others have one shape): 0 = 256 threads with 4 blocks per SM, 1 = 128 threads with
    * 8, 2 = 256 threads with 3. */
   int32_t density_shape;
   /* Block shape of the nearest-higher cell search with one lane per point (2-D
-   * runs above 262,144 points, 3-D runs above 524,288; other runs have
+   * runs above 262,144 points, 3-D runs above 524,288, and batches of more than 64
+   * events in 2-D and 128 in 3-D, half of that above 65,536 points; other runs have
    * one shape): 0 = 256 threads with 8 blocks per SM in 2-D (4 in 3-D), 1 = 256
    * threads with 6, 2 = 128 threads with 16 in 2-D (8 in 3-D). */
   int32_t nh_shape;
@@ -235,7 +238,8 @@ clue_status clue_workspace_get_tuning(const clue_workspace* ws, clue_tuning* out
 clue_status clue_workspace_set_tuning(clue_workspace* ws, const clue_tuning* tuning);
 /* Autotuner: runs make_clusters on these device points (the single-event form
  * when event_sizes is NULL, else the batched form with grid_mode) under
- * candidate tunings, one field at a time, times each candidate with CUDA events
+ * candidate tunings, one field at a time and only the fields that such a run obeys
+ * (the others stay as they are), times each candidate with CUDA events
  * on `stream` (median of `reps` runs after one warm-up run), keeps the fastest
  * in the workspace and returns it in *chosen (may be NULL). The points' outputs
  * are written by every run and hold the (unchanged) result at the end. Blocks
