@@ -119,17 +119,42 @@ __device__ __forceinline__ float2 unpack2(unsigned long long v) {
 // The square root of a number from kRootLow up to FLT_MAX: g = x y from the
 // approximate y = 1/sqrt(x), corrected once by the residual x - g^2 of a fused
 // multiply-add (Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", 1990): g + (x - g^2) y / 2. On sm_100 each of the
-// floats of the range gives the bits of __fsqrt_rn (all were compared); outside
-// it an infinity, a NaN, a subnormal or a zero gives NaN, and another small
-// number may be a unit in the last place off. The caller tests the range once for
-// many, where __fsqrt_rn does for each.
+// System/6000 processor", 1990): g + (x - g^2) y / 2. That it is the correctly rounded
+// root on sm_100 is checked on every float of the range (clue_selftest_math); outside
+// it an infinity, a NaN, a subnormal or a zero gives NaN, and another small number may
+// be a unit in the last place off. The caller tests the range once for 32 of them.
 constexpr float kRootLow = 0x1p-90f;
 __device__ __forceinline__ float sqrt_in_range(float x) {
   float y;
   asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   const float g = __fmul_rn(x, y);
   return __fmaf_rn(__fmaf_rn(-g, g, x), __fmul_rn(y, 0.5f), g);
+}
+
+// Counts of floats: [0] from kRootLow to FLT_MAX with sqrt_in_range other than __fsqrt_rn,
+// [1] from -80 to 0 with clue_expf_normal other than clue_expf, [2] zero, subnormal or
+// not finite with a sqrt_in_range that is a number.
+__global__ void __launch_bounds__(kThreads) k_math_selftest(unsigned long long* differing) {
+  unsigned bad[3] = {0, 0, 0};
+  const uint32_t root_low = __float_as_uint(kRootLow), infinite = 0x7f800000u;
+  const uint32_t last = __float_as_uint(80.0f) | 0x80000000u;
+  for (uint64_t b = (uint64_t)blockIdx.x * kThreads + threadIdx.x; b <= last; b += (uint64_t)gridDim.x * kThreads) {
+    const uint32_t bits = (uint32_t)b;
+    const float x = __uint_as_float(bits);
+    if (bits >= 0x80000000u) {
+      bad[1] += __float_as_uint(clue_expf_normal(x)) != __float_as_uint(clue_expf(x));
+    } else {
+      const float root = sqrt_in_range(x);
+      if (bits >= root_low && bits < infinite)
+        bad[0] += __float_as_uint(root) != __float_as_uint(__fsqrt_rn(x));
+      else if (bits < 0x00800000u || bits >= infinite)
+        bad[2] += root == root;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (bad[k])
+      atomicAdd(&differing[k], (unsigned long long)bad[k]);
 }
 
 // Silhouettes: a warp holds 32 points, one per lane, and the sums of distances
@@ -352,6 +377,27 @@ clue_status clue_silhouette_device(const clue_points* points, const int32_t* clu
   }
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? CLUE_OK : fail_cuda(e, "silhouette kernel launch");
+}
+
+clue_status clue_selftest_math(int32_t device, void* stream, int64_t* differing) {
+  if (!differing)
+    return fail(CLUE_ERR_INVALID_ARGUMENT, "the counts are required");
+  cudaError_t e = cudaSetDevice(device);
+  if (e != cudaSuccess)
+    return fail_cuda(e, "cudaSetDevice");
+  constexpr size_t kBytes = 3 * sizeof(unsigned long long);
+  unsigned long long* counts = nullptr;
+  if ((e = cudaMalloc(&counts, kBytes)) != cudaSuccess)
+    return fail_cuda(e, "self-test allocation");
+  const cudaStream_t st = (cudaStream_t)stream;
+  if ((e = cudaMemsetAsync(counts, 0, kBytes, st)) == cudaSuccess) {
+    k_math_selftest<<<sm_count() * 16, kThreads, 0, st>>>(counts);
+    if ((e = cudaGetLastError()) == cudaSuccess &&
+        (e = cudaMemcpyAsync(differing, counts, kBytes, cudaMemcpyDeviceToHost, st)) == cudaSuccess)
+      e = cudaStreamSynchronize(st);
+  }
+  cudaFree(counts);
+  return e == cudaSuccess ? CLUE_OK : fail_cuda(e, "math self-test");
 }
 
 }  // extern "C"

@@ -175,6 +175,12 @@ clue_status clue_workspace_set_graphs(clue_workspace* ws, int32_t enable);
  * up. The GPU stays usable afterwards. CLUE_ERR_RUNTIME means the wait did not
  * report. Blocks until done. */
 clue_status clue_selftest_bounded_wait(int32_t device, void* stream);
+/* Self-test of the kernels' own arithmetic (no reference counterpart): on `device`, over
+ * every float of their ranges, the number at which [0] the silhouettes' short square
+ * root is not the correctly rounded one, [1] clue_expf_normal is not clue_expf, [2] the
+ * short root of a zero, a subnormal, an infinity or a NaN is a number. All are 0.
+ * Blocks until done. */
+clue_status clue_selftest_math(int32_t device, void* stream, int64_t* differing);
 /* 1 when the workspace's last run was a graph replay, else 0. */
 clue_status clue_workspace_graph_replayed(const clue_workspace* ws, int32_t* replayed);
 /* Pieces the last host-buffer run on this workspace was split into: a batch of

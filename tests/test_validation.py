@@ -212,3 +212,14 @@ def test_device_centroids_of_many_clusters(ndim, k):
     for weighted in (False, True):
         got = clue.cluster_centroids(pts, Given(), weighted=weighted)
         assert np.array_equal(got.view(np.int32), O.centroids(c, w, lab, k, weighted=weighted).view(np.int32))
+
+
+# Every float of the range of the silhouettes' short square root against __fsqrt_rn, and
+# of clue_expf_normal on the device against clue_expf.
+@pytest.mark.gpu
+def test_device_arithmetic_over_whole_ranges():
+    import ctypes as C
+    from cluestering_b200 import _lib as L
+    differing = (C.c_int64 * 3)(-1, -1, -1)
+    L.check(L.load().clue_selftest_math(0, None, differing))
+    assert list(differing) == [0, 0, 0]
