@@ -14,9 +14,9 @@ device->host copy of the cluster ids. Extra keys report the plain per-event GPU
 form (one make_clusters call per event with a host sync per event, the
 reference's usage pattern), the 1,048,576-point single event and the serving
 loop. With --impl reference the reference's own make_clusters (oracle/_ref:
-its serial CPU backend compiled from its unmodified headers; the CPU
-restatement in oracle/ where that build is absent) runs a bounded sample of
-the same workload on all host cores, one share of the events per thread.
+its serial CPU backend compiled from its unmodified headers) runs a bounded
+sample of the same workload on all host cores, one share of the events per
+thread; where that build is absent the line says `unavailable`.
 
 Under torchrun every rank clusters its own batch (events are independent: no
 collective on the data path); time is the max over ranks and `value` the points
@@ -227,18 +227,19 @@ def parity_sample(algo, coords_d, weights_d, sizes, stream, timed_labels, ref, n
 
 def run_reference(args, world, rank):
     from cluestering_b200 import workloads as W
+    from oracle import ref as Rf
     if rank != 0:
+        return 0
+    if not Rf.available():  # nothing else stands in for the reference's own code
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "the reference's own make_clusters is not built (oracle/_ref)"}), flush=True)
         return 0
     ev, sizes = W.batch_2d(n_events=args.events)
     threads = os.cpu_count() or 1
     budget = args.cpu_sample_points
-    from oracle import ref as Rf
-    kind = "reference" if Rf.available() else "port"
 
     def one(budget_points):
-        if kind == "reference":
-            return reference_cpu(ev, sizes, budget_points, threads)[:3]
-        return cpu_reference(ev, sizes, budget_points, threads)[:3]
+        return reference_cpu(ev, sizes, budget_points, threads)[:3]
 
     for _ in range(args.warmup):
         one(budget // 4)
@@ -252,7 +253,7 @@ def run_reference(args, world, rank):
         "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": pts / value * 1e3, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f32", "data": "synthetic", "config": CONFIG,
-        "cpu_baseline": {"value": value, "unit": "points/s", "cores": threads, "kind": kind,
+        "cpu_baseline": {"value": value, "unit": "points/s", "cores": threads, "kind": "reference",
                          "sample": sample},
         "e2e": {"value": value, "unit": "points/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
     }
@@ -753,7 +754,7 @@ def main():
     if args.case == "large-2d":
         return run_large_2d(args)
     if args.impl == "reference":
-        # CPU arm: rank 0 times the CPU restatement; other ranks have no work.
+        # CPU arm: rank 0 times the reference's own code; other ranks have no work.
         return run_reference(args, int(os.environ.get("WORLD_SIZE", "1")),
                              int(os.environ.get("RANK", "0")))
     world, rank, local = dist_setup()
