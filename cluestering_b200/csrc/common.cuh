@@ -328,14 +328,16 @@ __device__ __forceinline__ int lsb_exponent(float x) {
 // The bound is checked in double: the true bound n * max_v + max_w and 2^24 u
 // are multiples of u, so a true bound above 2^24 u is at least (2^24 + 1) u,
 // which the double product cannot round down to 2^24 u.
-__device__ __forceinline__ bool event_sums_exact(const int32_t* event_exact, int e, int n_points) {
-  const int4 st = reinterpret_cast<const int4*>(event_exact)[e];
+__device__ __forceinline__ bool bounds_exact(const int4& st, int n_points) {
   if (st.w != 0)
     return false;
   if (st.x == INT_MAX)
     return true;  // every contribution is zero
   const double bound = (double)n_points * (double)__int_as_float(st.y) + (double)__int_as_float(st.z);
   return bound <= ldexp(1.0, 24 + st.x);
+}
+__device__ __forceinline__ bool event_sums_exact(const int32_t* event_exact, int e, int n_points) {
+  return bounds_exact(reinterpret_cast<const int4*>(event_exact)[e], n_points);
 }
 
 // Status word bits written by kernels whose waits are bounded.

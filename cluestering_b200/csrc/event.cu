@@ -678,6 +678,7 @@ cudaError_t launch_event_front(const RunShape& sh, const RunParams& prm, const R
   a.ssig = b.sorted_sigma;
   a.sunc = b.sorted_unc;
   a.stag = b.sorted_tag;
+  static_assert(kEventTiles <= kTileBlocks, "the cell layout of such an event reads records, not coordinate planes");
   a.rec = sweep_fast_path(prm) ? b.rec_dens : nullptr;
   a.event_exact = sh.D == 2 || sh.D == 3 ? b.event_exact : nullptr;
   a.counters = b.counters;

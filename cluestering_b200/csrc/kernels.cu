@@ -1530,7 +1530,8 @@ TuningUse tuning_use(const RunShape& sh, const RunParams& prm) {
   TuningUse u;
   u.density = fast && !sweep_groups(prm, sh.n, sh.n_events);
   u.cells = fast;
-  u.nearest = fast && nh_lanes(sh.D, sh.n, sh.n_events) == 1;
+  const NearestForm near = nearest_form(sh.D, sh.n, sh.n_events, sh.max_event_points);
+  u.nearest = fast && (near.lanes == 1 || near.when != kAlways);
   u.binning = !event && sh.stable;
   u.labels = !event && !local_labels(sh);
   return u;
@@ -1598,7 +1599,7 @@ cudaError_t launch_run(const RunShape& sh, const RunParams& prm, const RunIO& io
     a.event_exact = b.event_exact;
     if (density_by_load(prm, n, sh.n_events))
       a.load = reinterpret_cast<float*>(b.counters + 9);
-    a.tile_blocks = sweep_tile_blocks(prm, n, sh.n_tiles, sh.n_events, event);
+    a.tile_blocks = sweep_tile_blocks(prm, n, sh.n_tiles, sh.n_events);
     if (a.tile_blocks)
       a.work_dens = nullptr;
     else

@@ -216,20 +216,15 @@ __device__ __forceinline__ void density_add(const RunParams& p, const float* xi,
   }
 }
 
-// Streamed form of density_add (same arithmetic).
-template <int D, int KIND>
+// Streamed form of density_add for the flat kernel (same arithmetic).
+template <int D>
 __device__ __forceinline__ void density_add_packed(const RunParams& p, unsigned long long xi_xy,
                                                    float zi, const ulonglong2& r, bool self,
                                                    float wi, float& rho) {
   float v;
   const float d2 = packed_d2<D>(xi_xy, zi, r, v);
-  if (KIND == CLUE_KERNEL_FLAT) {
-    if (d2 <= p.dc2)
-      rho = __fadd_rn(rho, self ? wi : v);
-  } else if (d2 <= p.dc2) {
-    const float k = kernel_value_in_range(p, __fsqrt_rn(d2), self);
-    rho = __fadd_rn(rho, __fmul_rn(k, v));
-  }
+  if (d2 <= p.dc2)
+    rho = __fadd_rn(rho, self ? wi : v);
 }
 
 constexpr int kRing = 4;       // chunks of candidate records in flight per warp
@@ -721,10 +716,10 @@ __global__ void __launch_bounds__(NT, MINB) k_density_fast(const RunParams p, co
           } else if (cnt == kChunk) {
 #pragma unroll 8
             for (int j = 0; j < kChunk; ++j)
-              density_add_packed<D, KIND>(p, xi_xy, xi[2], chunk[j], j == jself, wi, rho);
+              density_add_packed<D>(p, xi_xy, xi[2], chunk[j], j == jself, wi, rho);
           } else {
             for (int j = 0; j < cnt; ++j)
-              density_add_packed<D, KIND>(p, xi_xy, xi[2], chunk[j], j == jself, wi, rho);
+              density_add_packed<D>(p, xi_xy, xi[2], chunk[j], j == jself, wi, rho);
           }
         } else {
           // positions of this chunk inside this lane's box
@@ -920,11 +915,6 @@ __device__ __forceinline__ int strip_position(int c, int s) {
   return D == 2 ? p2 : z * s * s + p2;
 }
 
-// Whether an event's tiles count as exact sums in SweepArgs::load.
-__device__ __forceinline__ bool load_exact(const RunParams& p, const SweepArgs& a, int event, int event_n) {
-  return a.load && p.kernel_kind == CLUE_KERNEL_FLAT && event_sums_exact(a.event_exact, event, event_n);
-}
-
 // Adds a tile of m points to the estimated times of the density (SweepArgs::load);
 // `squares` is the sum of the squares of its cells' members. A point is taken to have as
 // many points around it as its tile has on average, and as many candidates as its cell
@@ -934,8 +924,9 @@ __device__ __forceinline__ bool load_exact(const RunParams& p, const SweepArgs& 
 // each record of its box, with the smooth kernels 90 ns and 160 ns for each that is a
 // candidate, with exact sums 60 ns.
 template <int D>
-__device__ __forceinline__ void add_load(const RunParams& p, const SweepArgs& a, const GridDesc& g, bool exact,
-                                         int event_n, int m, const float* inv, float squares) {
+__device__ __forceinline__ void add_load(const RunParams& p, const SweepArgs& a, const GridDesc& g,
+                                         const int4& bounds, int event_n, int m, const float* inv, float squares) {
+  const bool flat = p.kernel_kind == CLUE_KERNEL_FLAT, exact = flat && bounds_exact(bounds, event_n);
   const float R = reach(p.dc2);
   float box = (float)m, near = 0.6f * squares / (float)m;
 #pragma unroll
@@ -947,7 +938,7 @@ __device__ __forceinline__ void add_load(const RunParams& p, const SweepArgs& a,
   near = fminf(near, box);
   const float tests = (float)m * near * (exact ? 1.0f : (float)((m + 4095) / 4096));
   atomicAdd(&a.load[0], tests * (exact ? 3e-6f : 6e-6f));
-  const float stream = p.kernel_kind == CLUE_KERNEL_FLAT ? (exact ? 0.06f : 0.03f) * box : 0.09f * box + 0.16f * near;
+  const float stream = flat ? (exact ? 0.06f : 0.03f) * box : 0.09f * box + 0.16f * near;
   atomicMax(reinterpret_cast<int*>(&a.load[1]), __float_as_int(stream));  // positive floats order like ints
 }
 
@@ -1139,7 +1130,7 @@ __device__ void tile_cells(const RunParams& p, const SweepArgs& a, int64_t t, in
     atomicAdd(sum, squares);
     group_sync<NT>();
     if (tid == 0)
-      add_load<D>(p, a, g, load_exact(p, a, a.sevt[begin], ev.n), ev.n, m, inv, *sum);
+      add_load<D>(p, a, g, reinterpret_cast<const int4*>(a.event_exact)[a.sevt[begin]], ev.n, m, inv, *sum);
   }
 }
 
@@ -1287,7 +1278,9 @@ __global__ void __launch_bounds__(kThreads, 3) k_cells_tile(const RunParams p, c
         rec[k] = a.rec_dens[begin + tid + k * kThreads];
     const int event = a.sevt[begin];
     const EventDesc ev = a.events[event];
-    const bool exact = load_exact(p, a, event, ev.n);
+    int4 bounds = make_int4(0, 0, 0, 1);  // (add_load, by one thread)
+    if (a.load && tid == 0)
+      bounds = reinterpret_cast<const int4*>(a.event_exact)[event];
     const GridDesc& g = a.grids[ev.grid];
     const int s = cells_per_dim<D>(m, p.cell_points);
     const int S = D == 2 ? s * s : s * s * s;
@@ -1398,7 +1391,7 @@ __global__ void __launch_bounds__(kThreads, 3) k_cells_tile(const RunParams p, c
         squares = 0.0f;
         for (int w = 0; w < kThreads / 32; ++w)
           squares += s_squares[w];
-        add_load<D>(p, a, g, exact, ev.n, m, inv, squares);
+        add_load<D>(p, a, g, bounds, ev.n, m, inv, squares);
       }
     }
     __syncthreads();
@@ -1462,14 +1455,10 @@ __global__ void __launch_bounds__(kThreads, 3) k_cells_tile(const RunParams p, c
   }
 }
 
-// Nearest higher with (density, tag) as one ordered 64-bit key and distances
-// compared as squared distances. A candidate j of point i is eligible when it is
-// "higher" (key_j > key_i, which is rho_j > rho_i, or equal densities above zero
-// and tag_j > tag_i) and sqrt(d2) <= the effective distance (d2 <= eff2). Against
-// the current best (distance delta) it wins when sqrt(d2) < delta, or when
-// sqrt(d2) == delta and key_j > key_best (ClusteringKernels.hpp:195-202). The
-// bracket decides all but the candidates whose squared distance falls in
-// (lo, hi); those take the exact square root.
+// Nearest higher with (density, tag) as one ordered 64-bit key and distances compared as
+// squared distances: a candidate j of point i is eligible when it is "higher" (key_j >
+// key_i: rho_j > rho_i, or equal densities above zero and tag_j > tag_i) and d2 <=
+// eff2, the effective distance; nh_consider compares it with the current best.
 
 // Tests the members of one cell unless the cell is empty, holds no higher
 // key, or its box is out of reach.
@@ -1504,7 +1493,7 @@ __device__ __forceinline__ void visit_cell(const SweepArgs& a, int slot, const f
 }
 
 // Nearest higher over the cell layout, one point per lane, for runs whose points
-// fill the GPU that way (nh_lanes). Thread w takes the w-th point of the
+// fill the GPU that way (nearest_form). Thread w takes the w-th point of the
 // walk order, so a warp holds neighbouring points. The own cell and its neighbours in the own
 // tile come first, which usually fixes a small delta; then every tile of the
 // reference's search box is visited, but only its cells that can hold a point
@@ -1519,6 +1508,8 @@ __device__ __forceinline__ void visit_cell(const SweepArgs& a, int slot, const f
 // (SweepArgs::stats); the counters cost registers, so timed runs go without.
 template <int D, int NT, int MINB, bool TAGS, bool STATS>
 __global__ void __launch_bounds__(NT, MINB) k_nearest_higher_cells(const RunParams p, const SweepArgs a) {
+  if (!runs_when(a, a.nh_when))
+    return;
   const int64_t n = a.n;
   const float4* __restrict__ rec = a.rec_nh;
   const int lane = threadIdx.x & 31;
@@ -1660,7 +1651,7 @@ __global__ void __launch_bounds__(NT, MINB) k_nearest_higher_cells(const RunPara
 // small bound. Phase 1: the tiles of the reference's search box, G at a time,
 // one per lane, each with its range of cells within the bound; these ranges are
 // laid end to end and dealt to the lanes. Bound by the latency of dependent loads
-// (tile, cell info, box, members), which G lanes pay once; nh_lanes has the figures.
+// (tile, cell info, box, members), which G lanes pay once; nearest_form has the figures.
 // The warp stays converged: groups that are done wait for the others, and every
 // shuffle and vote is reached by all 32 lanes.
 // STATS: the profiling instantiation, which also counts the candidates tested
@@ -1675,6 +1666,8 @@ struct NhTile {
 
 template <int D, int G, int NT, int MINB, bool TAGS, bool STATS>
 __global__ void __launch_bounds__(NT, MINB) k_nearest_higher_group(const RunParams p, const SweepArgs a) {
+  if (!runs_when(a, a.nh_when))
+    return;
   constexpr int P = 32 / G;  // points of a warp at a time
   constexpr unsigned kGroup = G == 32 ? kFullMask : (1u << G) - 1u;
   // cells of phase 0: one per lane, the own cell and its nearest neighbours
@@ -1956,11 +1949,11 @@ bool sweep_fast_path(const RunParams& p) {
 }
 
 bool sweep_groups(const RunParams& p, int64_t n, int32_t n_events) {
-  return sweep_fast_path(p) && n <= kGroupPoints && n_events <= kGroupEvents;
+  return sweep_fast_path(p) && n <= kGroupPoints && n_events <= (n <= 49152 ? 64 : 32);
 }
 
-bool sweep_tile_blocks(const RunParams& p, int64_t n, int64_t n_tiles, int32_t n_events, bool one_cluster) {
-  return sweep_groups(p, n, n_events) && (one_cluster || n_tiles <= kTileBlocks);
+bool sweep_tile_blocks(const RunParams& p, int64_t n, int64_t n_tiles, int32_t n_events) {
+  return sweep_groups(p, n, n_events) && n_tiles <= kTileBlocks;
 }
 
 #define CLUE_DISPATCH_D(D, KERNEL, ...)                \
@@ -2081,18 +2074,20 @@ cudaError_t launch_density_fast(const RunParams& p, const SweepArgs& a, cudaStre
 // hits 113 / 27 / 27 / 39; 262,144: 378 / 219 / 257 / 404; 524,288: 835 / 512; blobs and
 // evenly spread points of 524,288: 762 / 617 and 215 / 283, of 1,048,576: 1,259 /
 // 1,197 and 403 / 549, of 2,097,152: 2,278 / 2,377 and 777 / 1,519.
-// Small events have few cells to look at: 65,536 points in 2-D events of 16 18 / 43, of
-// 512 35 / 45, of 1,024 39 / 46, 16,384 in events of 128 24 / 28, of 256 32 / 30; 65,536 in
-// 3-D events of 128 32 / 47, of 512 49 / 49; 250,000 in 2-D events of 1,024 54 / 136, of
-// 4,096 65 / 136 (the call 314 / 357), 500,000 in 3-D events of 4,096 169 / 267.
-int nh_lanes(int D, int64_t n, int32_t n_events) {
-  if (n_events > (D == 2 ? 32 : 64) * (n <= kGroupPoints ? 2 : 1))
-    return 1;
-  if (n <= 4096)
-    return 32;
-  if (n <= 16384)
-    return 16;
-  return n <= (int64_t)1 << (D == 3 ? 19 : 18) ? 8 : 1;
+// Small events of even points have few cells to look at: 65,536 points in 2-D events of 16
+// 18 / 43, of 512 35 / 45, of 1,024 39 / 46, 16,384 in events of 128 24 / 28, of 256 32 / 30;
+// 65,536 in 3-D events of 128 32 / 47, of 512 49 / 49; 250,000 in 2-D events of 1,024 54 /
+// 136, of 4,096 65 / 136, 500,000 in 3-D events of 4,096 169 / 267. But where a tile
+// holds a blob its points are the longest chains: 24,850 points in 66 events of 256 to 512
+// 125 / 35, 85,884 in 100 of up to 2,048 159 / 77, 127,362 in 64 of up to 8,192 134 / 87.
+NearestForm nearest_form(int D, int64_t n, int32_t n_events, int32_t max_event_points) {
+  const int lanes = n <= 4096 ? 32 : n <= 16384 ? 16 : n <= (int64_t)1 << (D == 3 ? 19 : 18) ? 8 : 1;
+  const bool small_events = n_events > (D == 2 ? 32 : 64) * (n <= kGroupPoints ? 2 : 1);
+  if (lanes == 1 || !small_events)
+    return {lanes, kAlways};
+  if (max_event_points <= kLargeTilePoints)  // no tile can hold more
+    return {1, kAlways};
+  return {lanes, kLargeTiles};
 }
 
 template <int D, bool TAGS, bool STATS>
@@ -2129,12 +2124,18 @@ void launch_nh_cells(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
 }
 
 template <int D, bool TAGS, bool STATS>
-void launch_nh_dim(const RunParams& p, const SweepArgs& a, cudaStream_t st) {
-  const int G = nh_lanes(D, a.n, a.n_events);
-  if (G == 1)
-    launch_nh_cells<D, TAGS, STATS>(p, a, st);
-  else
-    launch_nh_group<D, TAGS, STATS>(p, a, G, st);
+void launch_nh_dim(const RunParams& p, SweepArgs a, cudaStream_t st) {
+  const NearestForm f = nearest_form(D, a.n, a.n_events, a.max_event_points);
+  a.nh_when = f.when;
+  if (f.lanes > 1) {
+    launch_nh_group<D, TAGS, STATS>(p, a, f.lanes, st);
+    count_launches(1);
+  }
+  if (f.lanes > 1 && f.when == kAlways)
+    return;
+  a.nh_when = f.lanes > 1 ? kNoLargeTiles : kAlways;
+  launch_nh_cells<D, TAGS, STATS>(p, a, st);
+  count_launches(1);
 }
 
 template <bool TAGS, bool STATS>
@@ -2159,7 +2160,6 @@ cudaError_t launch_nearest_higher(int D, const RunParams& p, const SweepArgs& a,
   if (a.n == 0)
     return cudaSuccess;
   if (sweep_fast_path(p)) {
-    count_launches(1);
     if (p.has_tags)
       a.stats ? launch_nh<true, true>(D, p, a, st) : launch_nh<true, false>(D, p, a, st);
     else

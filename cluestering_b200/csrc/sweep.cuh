@@ -5,6 +5,10 @@
 
 namespace clue_impl {
 
+// Some choices depend on whether a tile holds more than kLargeTilePoints points, which
+// the host does not know: the kernels of both are launched, and one returns at once.
+enum RunWhen { kNever, kAlways, kLargeTiles, kNoLargeTiles };
+
 // Inputs and outputs of the two sweeps. Arrays prefixed with `s` are in
 // tile-contiguous (sorted) order; plane d of sx/ssig starts at d * n.
 struct SweepArgs {
@@ -56,6 +60,7 @@ struct SweepArgs {
   // in layout order (sweep_tile_blocks).
   int32_t* walk;
   bool tile_blocks;
+  RunWhen nh_when;  // whether a launch of the nearest-higher search has the run
   // Packed candidate records of the fast path (D = 2 or 3).
   float4* rec_dens;  // {x, y, [z], v}: v = flat * w for the flat kernel, else w
   float4* rec_nh;    // D = 2: {x, y, rho, tag bits}; D = 3: {x, y, z, rho}
@@ -92,18 +97,24 @@ struct SweepArgs {
   uint32_t* status;
 };
 
+// Whether a kernel launched for the case `when` has the run.
+__device__ __forceinline__ bool runs_when(const SweepArgs& a, RunWhen when) {
+  return when == kAlways || (*a.large_count > 0) == (when == kLargeTiles);
+}
+
 // True when the packed fast path applies: D = 2 or 3, Euclidean metric, no
 // per-point sigma and no wrapped coordinate.
 bool sweep_fast_path(const RunParams& p);
 
 cudaError_t launch_work_order(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 // The density with 16 or 32 lanes per point (density_group.cu), for fast-path runs of
-// at most kGroupPoints points in at most kGroupEvents events. Small events have few
-// candidates to share among lanes: density, us, 32 points per warp / lanes, 65,536 points
-// in events of 16 12 / 48, of 256 23 / 49, of 512 29 / 49, of 1,024 40 / 50 (Gaussian 47 / 49
-// at 256, 113 / 54 at 1,024); 16,384 in events of 64 12 / 21, of 256 20 / 21, of 512 24 / 21.
+// at most kGroupPoints points in at most 64 events, 32 above 49,152 points. Small events
+// have few candidates to share among lanes: density, us, 32 points per warp / lanes, 65,536
+// points in events of 16 12 / 48, of 256 23 / 49, of 512 29 / 49, of 1,024 40 / 50 (Gaussian
+// 47 / 49 at 256, 113 / 54 at 1,024); 16,384 in events of 64 12 / 21, of 256 20 / 21, of 512
+// 24 / 21; blobs, 22,742 points in 64 events 44 / 39, 33,129 in 40 74 / 68, 59,757 in 64 76 /
+// 105 (ordered sums, one grid: 73 / 189).
 constexpr int64_t kGroupPoints = 1 << 16, kGroupWide = 1 << 13;  // 32 lanes up to the latter
-constexpr int32_t kGroupEvents = 64;
 bool sweep_groups(const RunParams& p, int64_t n, int32_t n_events);
 cudaError_t launch_density_group(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 // Whether such a run may take 32 points per warp all the same (density_streams), and
@@ -114,33 +125,33 @@ __device__ __forceinline__ bool density_streams(const SweepArgs& a) {
 }
 // Runs whose sweeps give every point a group of lanes (sweep_groups) take the
 // points in layout order, and k_cells_tile lays the cells out with a block per tile;
-// `walk` and `work_dens` are then null. Above kTileBlocks tiles (about what the GPU
-// holds at once) most hold too few points for a block of their own: 16,384 points in
-// 2,304 tiles 17 us without, 22 with it; 65,536 in 512 23 and 17. The one-cluster form of
-// a single event (up to 2,560 tiles) always takes it: it leaves no coordinate planes.
-constexpr int64_t kTileBlocks = 1024;
-bool sweep_tile_blocks(const RunParams& p, int64_t n, int64_t n_tiles, int32_t n_events, bool one_cluster);
-// Lanes per point of the nearest-higher search on the fast path.
-int nh_lanes(int D, int64_t n, int32_t n_events);
+// `walk` and `work_dens` are then null. Above kTileBlocks tiles (twice what the GPU holds
+// at once) most hold too few points for a block of their own: gather, us, tile by warps /
+// blocks, 16 events with one grid, 2,304 tiles: even points 17 / 22, blobs 28 / 17; 4,096
+// tiles of 16 points 20 / 36. The one-cluster form of a single event, which leaves no
+// coordinate planes, has no more than that.
+constexpr int64_t kTileBlocks = 2560;
+bool sweep_tile_blocks(const RunParams& p, int64_t n, int64_t n_tiles, int32_t n_events);
+// Lanes per point of the nearest-higher search on the fast path: `lanes` where tiles hold
+// more than kLargeTilePoints points or always (when), else one.
+struct NearestForm {
+  int lanes;
+  RunWhen when;
+};
+NearestForm nearest_form(int D, int64_t n, int32_t n_events, int32_t max_event_points);
 // The sweeps off the fast path: any number of dimensions, metric, kernel and
 // option. Three forms, chosen by any_form (sweep_any.cu): a warp per point
 // (sweep_any_point.cu), a block of 8 warps per 32 points (sweep_any.cu) and a thread
 // per point (sweep_any_thread.cu).
-enum AnyWhen { kAnyNever, kAnyAlways, kAnyLargeTiles, kAnyNoLargeTiles };
 struct AnyForm {
-  AnyWhen point = kAnyNever, block = kAnyNever, thread = kAnyNever;
+  RunWhen point = kNever, block = kNever, thread = kNever;
   bool work_order = false;  // k_work_order runs first
 };
 AnyForm any_form(int D, const SweepArgs& a);
-// Whether a kernel launched for the case `when` has the run: some choices depend on
-// the tiles of more than kLargeTilePoints points, which the host does not know.
-__device__ __forceinline__ bool any_form_runs(const SweepArgs& a, int when) {
-  return when == kAnyAlways || (*a.large_count > 0) == (when == kAnyLargeTiles);
-}
 cudaError_t launch_density_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 cudaError_t launch_nearest_higher_any(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 cudaError_t launch_sweep_point(bool density, int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
-cudaError_t launch_sweep_thread(bool density, int D, const RunParams& p, const SweepArgs& a, int when,
+cudaError_t launch_sweep_thread(bool density, int D, const RunParams& p, const SweepArgs& a, RunWhen when,
                                 cudaStream_t st);
 cudaError_t launch_density(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);
 cudaError_t launch_nearest_higher(int D, const RunParams& p, const SweepArgs& a, cudaStream_t st);

@@ -310,9 +310,9 @@ __device__ __forceinline__ float pair_inner(const RunParams& p, const Item<D>& i
 
 template <int D, int METRIC>
 __global__ void __launch_bounds__(kThreads, D <= 4 ? 3 : 2) k_density_any(const RunParams p, const SweepArgs a,
-                                                                             const int when) {
+                                                                             const RunWhen when) {
   extern __shared__ __align__(16) unsigned char s_dyn[];
-  if (!any_form_runs(a, when))
+  if (!runs_when(a, when))
     return;
   DensityStage<D>& sh = *reinterpret_cast<DensityStage<D>*>(s_dyn);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -395,9 +395,9 @@ __global__ void __launch_bounds__(kThreads, D <= 4 ? 3 : 2) k_density_any(const 
 
 template <int D, int METRIC>
 __global__ void __launch_bounds__(kThreads, D <= 4 ? 3 : 2) k_nearest_higher_any(const RunParams p, const SweepArgs a,
-                                                                                    const int when) {
+                                                                                    const RunWhen when) {
   extern __shared__ __align__(16) unsigned char s_dyn[];
-  if (!any_form_runs(a, when))
+  if (!runs_when(a, when))
     return;
   NearestStage<D>& sh = *reinterpret_cast<NearestStage<D>*>(s_dyn);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(kThreads, D <= 4 ? 3 : 2) k_nearest_higher_any
 }
 
 template <int D, int METRIC>
-cudaError_t launch_any(bool density, const RunParams& p, const SweepArgs& a, int when, cudaStream_t st) {
+cudaError_t launch_any(bool density, const RunParams& p, const SweepArgs& a, RunWhen when, cudaStream_t st) {
   const int64_t items = (a.n + 31) / 32;
   const int blocks = (int)std::min<int64_t>(items, (int64_t)sm_count() * 64);
   // up to 70 KB: above the default 48 KB they need the opt-in, a function
@@ -527,7 +527,7 @@ cudaError_t launch_any(bool density, const RunParams& p, const SweepArgs& a, int
 }
 
 template <int D>
-cudaError_t launch_dim(bool density, const RunParams& p, const SweepArgs& a, int when, cudaStream_t st) {
+cudaError_t launch_dim(bool density, const RunParams& p, const SweepArgs& a, RunWhen when, cudaStream_t st) {
   switch (p.metric_kind) {
     case CLUE_METRIC_EUCLIDEAN: return launch_any<D, CLUE_METRIC_EUCLIDEAN>(density, p, a, when, st);
     case CLUE_METRIC_PERIODIC_EUCLIDEAN: return launch_any<D, CLUE_METRIC_PERIODIC_EUCLIDEAN>(density, p, a, when, st);
@@ -535,7 +535,7 @@ cudaError_t launch_dim(bool density, const RunParams& p, const SweepArgs& a, int
   }
 }
 
-cudaError_t launch_sweep_block(bool density, int D, const RunParams& p, const SweepArgs& a, int when,
+cudaError_t launch_sweep_block(bool density, int D, const RunParams& p, const SweepArgs& a, RunWhen when,
                                cudaStream_t st) {
   switch (D) {
     case 1: return launch_dim<1>(density, p, a, when, st);
@@ -589,17 +589,17 @@ AnyForm any_form(int D, const SweepArgs& a) {
   const int64_t event = std::min<int64_t>(a.n / std::max(1, a.n_events), 512);  // points, at most 512
   const bool few = a.n > 256 * event, sparse = a.n < 32 * a.n_tiles;
   if (a.n <= kPointWarps) {
-    (few ? f.thread : f.point) = kAnyAlways;
+    (few ? f.thread : f.point) = kAlways;
     return f;
   }
   f.work_order = true;
   if (a.n <= kBlocks && !few && !sparse) {
-    f.block = kAnyAlways;
+    f.block = kAlways;
   } else if (a.n <= most_blocks && a.max_event_points > kLargeTilePoints) {
-    f.block = kAnyLargeTiles;
-    f.thread = kAnyNoLargeTiles;
+    f.block = kLargeTiles;
+    f.thread = kNoLargeTiles;
   } else {  // (no tile can hold more than 256 points, or the points fill the GPU)
-    f.thread = kAnyAlways;
+    f.thread = kAlways;
   }
   return f;
 }

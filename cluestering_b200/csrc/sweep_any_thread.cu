@@ -16,8 +16,8 @@ namespace clue_impl {
 namespace {
 
 template <int D>
-__global__ void __launch_bounds__(kThreads) k_density_thread(const RunParams p, const SweepArgs a, const int when) {
-  if (!any_form_runs(a, when))
+__global__ void __launch_bounds__(kThreads) k_density_thread(const RunParams p, const SweepArgs a, const RunWhen when) {
+  if (!runs_when(a, when))
     return;
   const int64_t n = a.n;
   const bool mahalanobis = p.metric_kind == CLUE_METRIC_MAHALANOBIS;
@@ -57,8 +57,8 @@ __global__ void __launch_bounds__(kThreads) k_density_thread(const RunParams p, 
 
 template <int D>
 __global__ void __launch_bounds__(kThreads)
-    k_nearest_higher_thread(const RunParams p, const SweepArgs a, const int when) {
-  if (!any_form_runs(a, when))
+    k_nearest_higher_thread(const RunParams p, const SweepArgs a, const RunWhen when) {
+  if (!runs_when(a, when))
     return;
   const int64_t n = a.n;
   const bool mahalanobis = p.metric_kind == CLUE_METRIC_MAHALANOBIS;
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 template <int D>
-cudaError_t launch_dim(bool density, const RunParams& p, const SweepArgs& a, int when, cudaStream_t st) {
+cudaError_t launch_dim(bool density, const RunParams& p, const SweepArgs& a, RunWhen when, cudaStream_t st) {
   const int blocks = (int)std::min<int64_t>((a.n + kThreads - 1) / kThreads, (int64_t)sm_count() * 16);
   if (density)
     k_density_thread<D><<<blocks, kThreads, 0, st>>>(p, a, when);
@@ -136,7 +136,7 @@ cudaError_t launch_dim(bool density, const RunParams& p, const SweepArgs& a, int
 
 }  // namespace
 
-cudaError_t launch_sweep_thread(bool density, int D, const RunParams& p, const SweepArgs& a, int when,
+cudaError_t launch_sweep_thread(bool density, int D, const RunParams& p, const SweepArgs& a, RunWhen when,
                                 cudaStream_t st) {
   switch (D) {
     case 1: return launch_dim<1>(density, p, a, when, st);

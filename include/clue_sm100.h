@@ -197,7 +197,7 @@ clue_status clue_workspace_kernel_launches(const clue_workspace* ws, int64_t* la
  * they decide only how the work is spread over the GPU. ------------------- */
 typedef struct {
   /* Density sweep, 2-D and 3-D Euclidean runs above 65,536 points or of more
-   * than 64 events (and smaller ones with crowded tiles): a warp whose 32 points have
+   * than 64 events (32 above 49,152 points; and smaller ones with crowded tiles): a warp whose 32 points have
    * different search boxes streams the union of their boxes through shared
    * memory when the union holds at most (threshold / 16) times the
    * candidates of the warp's largest own box; otherwise each point reads its
@@ -216,7 +216,7 @@ typedef struct {
    * tile): it decides the search boxes and the order of the density sums. */
   int32_t cell_points;
   /* Block shape of the density sweep of runs above 65,536 points or of more than
-   * 64 events (others have one shape): 0 = 256 threads with 4 blocks per SM, 1 = 128 threads with
+   * 64 events (32 above 49,152 points; others have one shape): 0 = 256 threads with 4 blocks per SM, 1 = 128 threads with
    * 8, 2 = 256 threads with 3. */
   int32_t density_shape;
   /* Block shape of the nearest-higher cell search with one lane per point (2-D

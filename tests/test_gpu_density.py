@@ -112,10 +112,8 @@ def test_cell_boxes_of_one_tile(D, n, cell_points):
 @pytest.mark.parametrize("kernel,params,weights", KERNELS + [("gaussian", (1.0, 1.0), "exponential")])
 @pytest.mark.parametrize("D,n,outlier,r", [(2, 8192, 3e3, 1.2), (2, 8193, 3e5, 1.2), (2, 12288, 3e5, 1.2),
                                            (3, 12289, 3e4, 1.5), (2, 20011, 3e3, 1.2), (3, 20011, 3e5, 1.5),
-                                           (2, 20011, None, 90.0), (3, 9001, None, 25.0), (2, 65536, 3e5, 1.2)])
+                                           (2, 20011, None, 90.0), (3, 9001, None, 25.0)])
 def test_crowded_tiles(D, n, outlier, r, kernel, params, weights):
-    if n == 65536 and kernel != "flat":
-        pytest.skip("the checker's time")
     c, w = event(D, n, weights, 1600 + D)
     if outlier:
         c[:, n // 2] = outlier
@@ -142,16 +140,22 @@ def test_crowded_tiles_in_a_batch(mode, kernel, params, weights):
                                                 exp_mode=O.EXP_CLUE, n_threads=8))
 
 
-# Small events: lanes per point up to 64 events (nearest higher 64 in 2-D, 128 in 3-D,
-# half of that above 65,536 points), one lane per point beyond.
+# Small events: lanes per point up to 64 events (density 32 above 49,152 points; nearest
+# higher 64 in 2-D, 128 in 3-D, half of that above 65,536 points), beyond that one lane per
+# point unless a tile holds more than 256 points.
 @pytest.mark.parametrize("kernel,params,weights", KERNELS[1:3])
 @pytest.mark.parametrize("D,events,m", [(2, 63, 90), (2, 64, 90), (2, 65, 90), (3, 65, 40), (3, 128, 40), (3, 129, 40),
-                                        (2, 32, 2049), (2, 33, 2049), (3, 64, 1025), (3, 65, 1025)])
-def test_batches_of_small_events(D, events, m, kernel, params, weights):
+                                        (2, 32, 2049), (2, 33, 2049), (3, 64, 1025), (3, 65, 1025),
+                                        (2, 32, 1700), (2, 33, 1700)])
+@pytest.mark.parametrize("crowd", [False, True])
+def test_batches_of_small_events(D, events, m, crowd, kernel, params, weights):
     rng = np.random.default_rng(1800 + events)
     sizes = rng.integers(1, 2 * m, events)
     sizes[-1] += max(0, m * events - sizes.sum())
+    sizes[0] = 900
     c = rng.uniform(0.0, 6.0, (D, int(sizes.sum()))).astype(np.float32)
+    if crowd:  # one tile of the first event
+        c[:, 300:900] = 3.0 + 0.01 * c[:, 300:900]
     w = rng.exponential(1.0, c.shape[1]).astype(np.float32)
     tags = rng.integers(0, 9, c.shape[1]).astype(np.uint32) if kernel == "flat" else None
     check(c, w, 0.8, 2.0, 1.1, kernel=kernel, kernel_params=params, sizes=sizes, tags=tags,
