@@ -2080,10 +2080,12 @@ cudaError_t launch_density_fast(const RunParams& p, const SweepArgs& a, cudaStre
 // 136, of 4,096 65 / 136, 500,000 in 3-D events of 4,096 169 / 267. But where a tile
 // holds a blob its points are the longest chains: 24,850 points in 66 events of 256 to 512
 // 125 / 35, 85,884 in 100 of up to 2,048 159 / 77, 127,362 in 64 of up to 8,192 134 / 87.
+// And so in one event above 65,536 points: blobs and even points of 131,072 in 2-D 162 / 90
+// and 56 / 80, of 262,144 193 / 152 and 76 / 143, in 3-D 483 / 328 and 121 / 148.
 NearestForm nearest_form(int D, int64_t n, int32_t n_events, int32_t max_event_points) {
   const int lanes = n <= 4096 ? 32 : n <= 16384 ? 16 : n <= (int64_t)1 << (D == 3 ? 19 : 18) ? 8 : 1;
   const bool small_events = n_events > (D == 2 ? 32 : 64) * (n <= kGroupPoints ? 2 : 1);
-  if (lanes == 1 || !small_events)
+  if (lanes == 1 || (!small_events && n <= kGroupPoints))
     return {lanes, kAlways};
   if (max_event_points <= kLargeTilePoints)  // no tile can hold more
     return {1, kAlways};
