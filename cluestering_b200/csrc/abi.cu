@@ -1442,7 +1442,11 @@ clue_status clue_workspace_autotune(clue_workspace* ws, const clue_params* param
   };
   // Only choices that this run obeys: another's candidates would all be the same run,
   // and the fastest of them, by chance, would stay for the runs that do obey it.
-  const TuningUse use = tuning_use(ws->tables.shape, make_run_params(params, points, best));
+  int32_t large_tiles = 0;
+  if (s == CLUE_OK &&
+      (e = cudaMemcpy(&large_tiles, ws->b.counters + 3, sizeof(int32_t), cudaMemcpyDeviceToHost)) != cudaSuccess)
+    s = fail_cuda(e, "large-tile count");
+  const TuningUse use = tuning_use(ws->tables.shape, make_run_params(params, points, best), large_tiles);
   if (use.density && points->ndim == 2)
     try_field(&clue_tuning::density_union_x16_2d, {0, 12, 16, 20, 24, 32, 48, 1 << 20});
   else if (use.density)

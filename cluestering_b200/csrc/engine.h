@@ -187,10 +187,11 @@ cudaError_t launch_run(const RunShape& shape, const RunParams& prm, const RunIO&
                        cudaEvent_t* marks = nullptr);
 
 // Which choices of clue_tuning a run of this shape obeys; the others change nothing.
+// large_tiles: its tiles of more than kLargeTilePoints points (counters[3] after a run).
 struct TuningUse {
   bool density, cells, nearest, binning, labels;
 };
-TuningUse tuning_use(const RunShape& shape, const RunParams& prm);
+TuningUse tuning_use(const RunShape& shape, const RunParams& prm, int32_t large_tiles);
 
 // The stages of an event_path run before and after the sweeps.
 cudaError_t launch_event_front(const RunShape& shape, const RunParams& prm, const RunIO& io, const GridDesc& grid,

@@ -1525,13 +1525,13 @@ static bool local_labels(const RunShape& sh) {
          local_labels_ready(sh.max_event_points);
 }
 
-TuningUse tuning_use(const RunShape& sh, const RunParams& prm) {
+TuningUse tuning_use(const RunShape& sh, const RunParams& prm, int32_t large_tiles) {
   const bool fast = sweep_fast_path(prm), event = event_path(sh);
   TuningUse u;
   u.density = fast && !sweep_groups(prm, sh.n, sh.n_events);
   u.cells = fast;
   const NearestForm near = nearest_form(sh.D, sh.n, sh.n_events, sh.max_event_points);
-  u.nearest = fast && (near.lanes == 1 || near.when != kAlways);
+  u.nearest = fast && (near.lanes == 1 || (near.when == kLargeTiles && large_tiles == 0));
   u.binning = !event && sh.stable;
   u.labels = !event && !local_labels(sh);
   return u;
