@@ -17,6 +17,8 @@
 // the cell layout, and everything after the sweeps, in one launch each (event.cu).
 #include <atomic>
 #include <cfloat>
+#include <type_traits>
+
 #include <cuda/atomic>
 
 #include "engine.h"
@@ -325,7 +327,8 @@ __global__ void __launch_bounds__(kThreads) k_bin_stable(RunParams p, CoordPtrs 
   int* col = s_col + (threadIdx.x >> 5) * max_tiles;
   const int e = sort_event_of(events, n_events, w);
   const EventDesc ev = events[e];
-  const GridDesc g = grids[ev.grid];
+  // (the general form reads the dimensions it needs: small events are not worth all ten)
+  std::conditional_t<DD == 0, const GridDesc&, const GridDesc> g = grids[ev.grid];
   const int D = DD ? DD : p.D;
   const int c = w - ev.sort_first;
   const int T = g.T;
@@ -349,6 +352,8 @@ __global__ void __launch_bounds__(kThreads) k_bin_stable(RunParams p, CoordPtrs 
     }
 #pragma unroll
     for (int u = 0; u < kStableAhead; ++u) {
+      if (base + u * 32 >= end)
+        break;  // the same for the whole warp
       const int i = base + u * 32 + lane;
       const bool valid = i < end;
       int t = -1;

@@ -125,3 +125,14 @@ def test_large_runs_off_the_fast_path(n, crowd):
     c = _crowded(rng.uniform(0.0, n / 100.0, (1, n)), n, crowd / n, 3)
     w = rng.exponential(1.0, n).astype(np.float32)
     check(c, w, 0.2, 2.0, 0.4, metric="manhattan", path="device")
+
+
+# Stable binning of events that end inside the rounds loaded ahead, any number of
+# dimensions (events of one point, of a round less or more one, of all rounds).
+@pytest.mark.parametrize("D", [1, 2, 3, 4, 10])
+def test_binning_of_tiny_events(D):
+    sizes = [1, 31, 32, 33, 95, 96, 97, 127, 128, 129, 1023, 1024, 1025, 0, 5] * 3
+    rng = np.random.default_rng(38 + D)
+    c = rng.uniform(0.0, 4.0, (D, sum(sizes))).astype(np.float32)
+    w = rng.exponential(1.0, c.shape[1]).astype(np.float32)
+    check(c, w, 0.5, 2.0, 0.7, metric="chebyshev", sizes=sizes, grid_mode=clue.GRID_PER_EVENT, path="device")
