@@ -123,7 +123,8 @@ constexpr int32_t kLocalLabelPoints = 1 << 16;
 bool local_labels_ready(int32_t points);
 
 // Single events of at most kEventPoints points and kEventTiles tiles run their
-// stages before and after the sweeps as one cluster launch each (event.cu).
+// stages before and after the sweeps as one cluster launch each (event.cu). The counters of
+// a tile take 72 bytes of a block's shared memory: 184 of 227 KB.
 constexpr int32_t kEventPoints = 1 << 16;
 constexpr int32_t kEventTiles = 2560;
 // Whether a run of this shape takes that form; the first call on a device
