@@ -577,23 +577,35 @@ cudaError_t launch_forms(bool density, int D, const RunParams& p, const SweepArg
 // Tiles of few points: one grid for a batch, 65,536 points in 32 events of 2,048 (4
 // points a tile) 184 / 592, in 4-D 274 / 606; per event, 65,536 in 4-D events of 256 (16
 // points a tile) 172 / 317, of 512 (32) 289 / 300.
-// Beyond 65,536 points it depends on the points: even ones (no tile of more than 256
-// points) of 131,072 in 4-D 1,665 / 2,232 and 262,144 in 1-D 401 / 580; clustered ones
-// 3,546 / 1,153 and 1,852 / 1,612; 1,048,576 clustered ones in 2-D 8,149 / 6,860, in
-// 3-D 8,784 / 7,120, but in 1-D 4,717 / 6,147. So both kernels are launched there, and
-// in smaller runs of sparse tiles, and one of them returns at once (about 4 us).
+// But one event of sparse tiles in many dimensions has many candidates (a call, thread /
+// block): 16,385 points in 6-D (22 a tile) 425 / 258 and 1,415 / 654, 65,536 in 7-D (30)
+// 778 / 717 and 4,096 / 3,287, in 8-D (10) 675 / 848 (24 a tile asked for, 65,536 in 2-D 466 /
+// 534, 3-D 471 / 633, 4-D 642 / 791); above that many points the threads fill the GPU:
+// 110,000 in 6-D (27 a tile) 1,718 / 2,074.
+// Beyond 65,536 points it depends on the points. Even ones (no tile of more than 256
+// points) in one event, dc of 0.05 and 0.3 tiles, a call, thread / block: 70,000 in 1-D 326 /
+// 253 and 336 / 299, in 3-D 646 / 445 and 714 / 722, in 5-D 1,043 / 677 and 2,475 / 1,671;
+// 100,000 in 1-D 340 / 283 and 349 / 344, in 3-D 696 / 574 and 795 / 953, in 4-D 985 / 618
+// and 1,504 / 1,316; 131,072 in 3-D 696 / 675 and 875 / 1,191, in 4-D 1,329 / 828 and 2,122 /
+// 1,916, in 7-D 1,750 / 1,889 and 10,164 / 9,271; 200,000 in 5-D 1,500 / 1,579 and 4,173 /
+// 4,538. Clustered ones of 131,072 in 4-D 3,546 / 1,153, 262,144 in 1-D 1,852 / 1,612;
+// 1,048,576 in 2-D 8,149 / 6,860, in 3-D 8,784 / 7,120, but in 1-D 4,717 / 6,147. So both
+// kernels are launched there, and in smaller runs of sparse tiles, and one of them returns
+// at once (about 4 us).
 AnyForm any_form(int D, const SweepArgs& a) {
   constexpr int64_t kPointWarps = 1 << 14, kBlocks = 1 << 16;
+  const bool one = a.n_events <= 1;
+  const int64_t even_blocks = !one ? kBlocks : D <= 3 ? 5 << 14 : 1 << 17;
   const int64_t most_blocks = D == 1 ? 1 << 18 : 1 << 20;
   AnyForm f;
   const int64_t event = std::min<int64_t>(a.n / std::max(1, a.n_events), 512);  // points, at most 512
-  const bool few = a.n > 256 * event, sparse = a.n < 32 * a.n_tiles;
+  const bool few = a.n > 256 * event, sparse = a.n < (one && D >= 6 && a.n <= kBlocks ? 16 : 32) * a.n_tiles;
   if (a.n <= kPointWarps) {
     (few ? f.thread : f.point) = kAlways;
     return f;
   }
   f.work_order = true;
-  if (a.n <= kBlocks && !few && !sparse) {
+  if (a.n <= even_blocks && !few && !sparse) {
     f.block = kAlways;
   } else if (a.n <= most_blocks && a.max_event_points > kLargeTilePoints) {
     f.block = kLargeTiles;

@@ -136,3 +136,15 @@ def test_binning_of_tiny_events(D):
     c = rng.uniform(0.0, 4.0, (D, sum(sizes))).astype(np.float32)
     w = rng.exponential(1.0, c.shape[1]).astype(np.float32)
     check(c, w, 0.5, 2.0, 0.7, metric="chebyshev", sizes=sizes, grid_mode=clue.GRID_PER_EVENT, path="device")
+
+
+# One event of even points at the sizes where the block of 8 warps gives way to the thread
+# per point, and of sparse tiles in many dimensions, with and without a crowded tile.
+@pytest.mark.parametrize("D,n,side", [(1, 81920, 4000.0), (3, 81921, 40.0), (4, 131072, 30.0), (4, 131073, 30.0),
+                                      (6, 16385, 20.0), (6, 65537, 60.0), (7, 16385, 20.0)])
+@pytest.mark.parametrize("crowd", [0, 400])
+def test_single_event_lines(D, n, side, crowd):
+    rng = np.random.default_rng(n + D)
+    c = _crowded(rng.uniform(0.0, side, (D, n)), n, crowd / n, 5)
+    w = rng.exponential(1.0, n).astype(np.float32)
+    check(c, w, 0.5, 2.0, 0.9, metric="chebyshev", path="device")
