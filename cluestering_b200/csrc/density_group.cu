@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(NT, MINB) k_density_group(const RunParams p, c
   const float4* __restrict__ rec_cell = a.rec_cell;
   const float R = reach(p.dc2);
   const float R2 = __fmul_ru(R, R);
-  if (G < 32 && density_streams(a))
+  if (G < 32 && density_streams<D>(a))
     return;
   for (;;) {
     int64_t w0 = 0;

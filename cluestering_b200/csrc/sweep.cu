@@ -544,7 +544,7 @@ template <int D, int KIND, bool NORMAL, int NT, int MINB, bool BY_LOAD = false>
 __global__ void __launch_bounds__(NT, MINB) k_density_fast(const RunParams p, const SweepArgs a) {
   if (BY_LOAD) {
     cudaGridDependencySynchronize();  // (launch_density_by_load)
-    if (!density_streams(a))
+    if (!density_streams<D>(a))
       return;
   }
   __shared__ __align__(16) float4 s_ring[NT / 32][kRing][kChunk];
@@ -922,7 +922,7 @@ __device__ __forceinline__ int strip_position(int c, int s) {
 // for each window of 4,096 points that their tile meets (6 ps of the whole GPU a test;
 // exact sums 3 ps). With 32 points per warp the longest item bounds the kernel: 30 ns for
 // each record of its box, with the smooth kernels 90 ns and 160 ns for each that is a
-// candidate, with exact sums 60 ns.
+// candidate, with exact sums 60 ns. (In 3-D the points bound it too: density_streams.)
 template <int D>
 __device__ __forceinline__ void add_load(const RunParams& p, const SweepArgs& a, const GridDesc& g,
                                          const int4& bounds, int event_n, int m, const float* inv, float squares) {

@@ -120,8 +120,12 @@ cudaError_t launch_density_group(int D, const RunParams& p, const SweepArgs& a, 
 // Whether such a run may take 32 points per warp all the same (density_streams), and
 // both kernels are launched.
 bool density_by_load(const RunParams& p, int64_t n, int32_t n_events);
+// In 3-D 32 points per warp take at least 3.4 ns a point, for the boxes of many tiles: a
+// call of 65,536 points in 160 blobs 413 us with them and 292 with lanes, in 80 428 / 372,
+// in 40 511 / 538, in 20 553 / 848 (loads 132 / 66, 229 / 143, 414 / 171, 775 / 405).
+template <int D>
 __device__ __forceinline__ bool density_streams(const SweepArgs& a) {
-  return a.load && a.load[0] > a.load[1] + 50.0f;
+  return a.load && a.load[0] > fmaxf(a.load[1], D == 3 ? 3.4e-3f * (float)a.n : 0.0f) + 50.0f;
 }
 // Runs whose sweeps give every point a group of lanes (sweep_groups) take the
 // points in layout order, and k_cells_tile lays the cells out with a block per tile;
