@@ -2075,17 +2075,24 @@ cudaError_t launch_density_fast(const RunParams& p, const SweepArgs& a, cudaStre
 // evenly spread points of 524,288: 762 / 617 and 215 / 283, of 1,048,576: 1,259 /
 // 1,197 and 403 / 549, of 2,097,152: 2,278 / 2,377 and 777 / 1,519.
 // Small events of even points have few cells to look at: 65,536 points in 2-D events of 16
-// 18 / 43, of 512 35 / 45, of 1,024 39 / 46, 16,384 in events of 128 24 / 28, of 256 32 / 30;
-// 65,536 in 3-D events of 128 32 / 47, of 512 49 / 49; 250,000 in 2-D events of 1,024 54 /
-// 136, of 4,096 65 / 136, 500,000 in 3-D events of 4,096 169 / 267. But where a tile
-// holds a blob its points are the longest chains: 24,850 points in 66 events of 256 to 512
-// 125 / 35, 85,884 in 100 of up to 2,048 159 / 77, 127,362 in 64 of up to 8,192 134 / 87.
-// And so in one event above 65,536 points: blobs and even points of 131,072 in 2-D 162 / 90
-// and 56 / 80, of 262,144 193 / 152 and 76 / 143, in 3-D 483 / 328 and 121 / 148.
+// 18 / 43, of 512 35 / 45, of 1,024 39 / 46; in 3-D events of 128 32 / 47, of 512 49 / 49;
+// 250,000 in 2-D events of 1,024 54 / 136, of 4,096 65 / 136, 500,000 in 3-D events of 4,096
+// 169 / 267. But where a tile holds a blob its points are the longest chains: 24,850 points
+// in 66 events of 256 to 512 125 / 35, 85,884 in 100 of up to 2,048 159 / 77, 127,362 in 64
+// of up to 8,192 134 / 87. Up to 32,768 points, where a tile need not be large for that,
+// lanes cost even points little: a call of 16,384 points in 2-D events of 64 157 / 158 us,
+// a blob in each 179 / 166, in events of 250 161 / 157 and 264 / 193; of 32,768 in events of
+// 16 211 / 211 and 223 / 222, of 250 167 / 167 and 280 / 207.
+// And so in one event above 98,304 points, in 3-D 262,144: blobs and even points of 131,072
+// in 2-D 162 / 90 and 56 / 80, of 262,144 193 / 152 and 76 / 143. The lines are where even
+// points (three densities, dm of 1.5 and 5) take about as long both ways, a call, one
+// lane / 8: 65,537 in 2-D 241 / 234, 226 / 225, 203 / 213; 98,304 285 / 274,
+// 239 / 250, 251 / 251; 131,072 315 / 317, 252 / 273, 227 / 249; in 3-D 65,537 396 / 368,
+// 352 / 341; 200,000 637 / 613, 554 / 543, 489 / 490; 400,000 1,061 / 1,037, 752 / 765.
 NearestForm nearest_form(int D, int64_t n, int32_t n_events, int32_t max_event_points) {
   const int lanes = n <= 4096 ? 32 : n <= 16384 ? 16 : n <= (int64_t)1 << (D == 3 ? 19 : 18) ? 8 : 1;
-  const bool small_events = n_events > (D == 2 ? 32 : 64) * (n <= kGroupPoints ? 2 : 1);
-  if (lanes == 1 || (!small_events && n <= kGroupPoints))
+  const bool small_events = n > 1 << 15 && n_events > (D == 2 ? 32 : 64) * (n <= kGroupPoints ? 2 : 1);
+  if (lanes == 1 || (!small_events && n <= (D == 2 ? 3 << 15 : 1 << 18)))
     return {lanes, kAlways};
   if (max_event_points <= kLargeTilePoints)  // no tile can hold more
     return {1, kAlways};

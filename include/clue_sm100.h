@@ -221,8 +221,9 @@ typedef struct {
   int32_t density_shape;
   /* Block shape of the nearest-higher cell search with one lane per point (2-D
    * runs above 262,144 points, 3-D runs above 524,288 and, where no tile holds more
-   * than 256 points, runs above 65,536 and batches of more than 64 events in 2-D
-   * and 128 in 3-D; other runs have one shape): 0 = 256 threads with 8 blocks per SM in
+   * than 256 points, 2-D runs above 98,304, 3-D runs above 262,144 and batches of more
+   * than 64 events in 2-D and 128 in 3-D (half above 65,536 points) of more than 32,768
+   * points; other runs have one shape): 0 = 256 threads with 8 blocks per SM in
    * 2-D (4 in 3-D), 1 = 256 threads with 6, 2 = 128 threads with 16 in 2-D (8 in 3-D). */
   int32_t nh_shape;
   /* Tile binning: 0 = counting sort by atomics, then each tile's points put

@@ -60,3 +60,28 @@ def test_large_runs_in_three_dimensions(n, shape, tags):
     algo.set_tuning(nh_shape=shape)
     check(c, w, 1.0, 2.0, 1.5, path="device", clusterer=algo,
           tags=rng.integers(0, 3, n).astype(np.uint32) if tags else None)
+
+
+# The lines above which even points have one lane per point and others eight: one event,
+# and batches of events of at most 250 points, none of whose tiles can be large.
+@pytest.mark.parametrize("D,n", [(2, 98304), (2, 98305), (3, 262144), (3, 262145)])
+@pytest.mark.parametrize("crowd", [0, 400])
+def test_even_points_of_one_event(D, n, crowd):
+    rng = np.random.default_rng(n + crowd)
+    c = rng.uniform(0.0, 200.0 if D == 2 else 60.0, (D, n))
+    c[:, n - crowd:] = 10.0 + 0.05 * rng.normal(0.0, 1.0, (D, crowd))
+    w = rng.exponential(1.0, n).astype(np.float32)
+    check(c.astype(np.float32), w, 0.9, 2.0, 1.3, path="device")
+
+
+@pytest.mark.parametrize("D,n,m", [(2, 16384, 16), (2, 32768, 250), (2, 32769, 250), (3, 32768, 100), (3, 32769, 100)])
+def test_batches_of_small_events(D, n, m):
+    import cluestering_b200 as clue
+    rng = np.random.default_rng(n + m)
+    c = rng.uniform(0.0, 20.0, (D, n))
+    blob = rng.random(n) < 0.5
+    c[:, blob] = 10.0 + 0.5 * rng.normal(0.0, 1.0, (D, int(blob.sum())))
+    sizes = [m] * (n // m) + ([n % m] if n % m else [])
+    w = rng.exponential(1.0, n).astype(np.float32)
+    check(c.astype(np.float32), w, 0.9, 2.0, 1.3, path="device", sizes=sizes, grid_mode=clue.GRID_PER_EVENT,
+          tags=rng.integers(0, 3, n).astype(np.uint32))
