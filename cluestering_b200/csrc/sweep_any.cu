@@ -581,7 +581,8 @@ cudaError_t launch_forms(bool density, int D, const RunParams& p, const SweepArg
 // block): 16,385 points in 6-D (22 a tile) 425 / 258 and 1,415 / 654, 65,536 in 7-D (30)
 // 778 / 717 and 4,096 / 3,287, in 8-D (10) 675 / 848 (24 a tile asked for, 65,536 in 2-D 466 /
 // 534, 3-D 471 / 633, 4-D 642 / 791); above that many points the threads fill the GPU:
-// 110,000 in 6-D (27 a tile) 1,718 / 2,074.
+// 110,000 in 6-D (27 a tile) 1,718 / 2,074, 131,072 in 6-D (32) 972 / 1,120 and 2,934 / 4,237,
+// but 90,000 in 6-D (123) 4,846 / 2,656.
 // Beyond 65,536 points it depends on the points. Even ones (no tile of more than 256
 // points) in one event, dc of 0.05 and 0.3 tiles, a call, thread / block: 70,000 in 1-D 326 /
 // 253 and 336 / 299, in 3-D 646 / 445 and 714 / 722, in 5-D 1,043 / 677 and 2,475 / 1,671;
@@ -599,7 +600,8 @@ AnyForm any_form(int D, const SweepArgs& a) {
   const int64_t most_blocks = D == 1 ? 1 << 18 : 1 << 20;
   AnyForm f;
   const int64_t event = std::min<int64_t>(a.n / std::max(1, a.n_events), 512);  // points, at most 512
-  const bool few = a.n > 256 * event, sparse = a.n < (one && D >= 6 && a.n <= kBlocks ? 16 : 32) * a.n_tiles;
+  const int tile = a.n > kBlocks ? 48 : one && D >= 6 ? 16 : 32;  // points
+  const bool few = a.n > 256 * event, sparse = a.n < tile * a.n_tiles;
   if (a.n <= kPointWarps) {
     (few ? f.thread : f.point) = kAlways;
     return f;
